@@ -454,12 +454,13 @@ static int build_resid_tables(ss_ctx* c, const std::vector<int>& shell_start, Re
     TRY(upload_v(c, "rs_tmax", tmax, &dtm));
     c->have_resid = true;
   }
-  void* p;
+  // the resident tables, looked up and not asked for by a size: a request larger than a table of
+  // two or three shells would replace its buffer and lose its content
   ResidDev R;
-  TRY(pool_get(c, "rs_node", 0, &p)); R.node = (const float2*)p;
-  TRY(pool_get(c, "rs_off", 0, &p)); R.off = (const int*)p;
-  TRY(pool_get(c, "rs_invh", 0, &p)); R.inv_h = (const float*)p;
-  TRY(pool_get(c, "rs_tmax", 0, &p)); R.tmax = (const float*)p;
+  R.node = (const float2*)c->pool["rs_node"].ptr;
+  R.off = (const int*)c->pool["rs_off"].ptr;
+  R.inv_h = (const float*)c->pool["rs_invh"].ptr;
+  R.tmax = (const float*)c->pool["rs_tmax"].ptr;
   *out = R;
   return SS_OK;
 }

@@ -93,3 +93,29 @@ def test_two_e_job_matches_staged_calls(estimator, precision):
     assert np.array_equal(g_after, g)
     assert np.array_equal(e_job, e)
     assert np.array_equal(s_job, s)
+
+
+def test_concurrent_mc_jobs_of_the_smallest_systems():
+    """MC-only jobs of one-atom hydrogen systems (two shells: the smallest resident tables), all at
+    once on fresh contexts: each equals, bit for bit, the same correction computed alone."""
+    def atom(zeta, x):
+        mol = basis.molecule_bohr(["H"], [[x, 0.3, -0.2]])
+        return basis.build_basis(mol, {1: [("1S", zeta), ("2P", zeta + 0.1)]}, basis.FitParams(ng0=6))
+
+    systems = [atom(0.9 + 0.05 * t, 0.4 * t) for t in range(8)]
+    q = basis.build_mapping(4)
+    alone = []
+    for s, b in enumerate(systems):
+        with api.Context(0) as ctx:
+            ctx.set_basis(b)
+            ctx.set_quartets(*q)
+            alone.append(ctx.zvmc(1.8, 5 + s, 8192, 2, "shared", "split_bf16"))
+    for _ in range(4):
+        with api.Context(0) as ctx:
+            ctx.job_limits(0, 8)
+            ids = [ctx.job_submit_inputs(b, q, 1.8, 5 + s, 8192, 2, "shared", "split_bf16", 0.0, mc_only=True)
+                   for s, b in enumerate(systems)]
+            for (mean, sigma), jid in zip(alone, ids):
+                m, e = ctx.job_result(jid)
+                np.testing.assert_array_equal(m, mean)
+                np.testing.assert_array_equal(e, sigma)
