@@ -340,7 +340,7 @@ template <class T>
 static int upload_v(ss_ctx* c, const char* name, const std::vector<T>& v, T** out) {
   void* p;
   TRY(pool_get(c, name, sizeof(T) * std::max<size_t>(v.size(), 1), &p));
-  if (!v.empty()) SS_CUDA_TRY(cudaMemcpyAsync(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, c->stream));
+  TRY(h2d_copy(c, p, v.data(), sizeof(T) * v.size()));
   *out = (T*)p;
   return SS_OK;
 }

@@ -97,11 +97,40 @@ void dev_free(ss_ctx* c, DevBuf& b) {
   b.bytes = 0;
 }
 
+// Copies up to STAGE_MAX go through a pinned ring (a wrap waits for the copies still in it);
+// larger ones are rare and wait for the stream instead.
+int h2d_copy(ss_ctx* c, void* dst, const void* src, size_t bytes) {
+  constexpr size_t STAGE_CAP = (size_t)4 << 20, STAGE_MAX = (size_t)1 << 20;
+  if (bytes == 0) return SS_OK;
+  if (bytes > STAGE_MAX) {
+    SS_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
+    SS_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    return SS_OK;
+  }
+  if (!c->stage) SS_CUDA_TRY(cudaHostAlloc((void**)&c->stage, STAGE_CAP, cudaHostAllocDefault));
+  if (c->stage_off + bytes > STAGE_CAP) {
+    for (auto& e : c->stage_evt) SS_CUDA_TRY(cudaEventSynchronize(e.second));
+    c->stage_off = 0;
+  }
+  char* at = c->stage + c->stage_off;
+  memcpy(at, src, bytes);
+  SS_CUDA_TRY(cudaMemcpyAsync(dst, at, bytes, cudaMemcpyHostToDevice, c->stream));
+  c->stage_off += (bytes + 255) / 256 * 256;
+  cudaEvent_t evt = nullptr;
+  for (auto& e : c->stage_evt)
+    if (e.first == c->stream) evt = e.second;
+  if (!evt) {
+    SS_CUDA_TRY(cudaEventCreateWithFlags(&evt, cudaEventDisableTiming));
+    c->stage_evt.emplace_back(c->stream, evt);
+  }
+  SS_CUDA_TRY(cudaEventRecord(evt, c->stream));
+  return SS_OK;
+}
+
 int h2d(ss_ctx* c, DevBuf& b, const void* src, size_t bytes) {
   int rc = dev_alloc(c, b, bytes);
   if (rc) return rc;
-  SS_CUDA_TRY(cudaMemcpyAsync(b.ptr, src, bytes, cudaMemcpyHostToDevice, c->stream));
-  return SS_OK;
+  return h2d_copy(c, b.ptr, src, bytes);
 }
 
 int h2d_async(ss_ctx* c, DevBuf& b, const void* src, size_t bytes) {
@@ -499,6 +528,11 @@ void ss_destroy(ss_ctx* c) {
     cudaEventDestroy(c->pin_evt);
   }
   if (c->pin) cudaFreeHost(c->pin);
+  for (auto& e : c->stage_evt) {
+    cudaEventSynchronize(e.second);
+    cudaEventDestroy(e.second);
+  }
+  if (c->stage) cudaFreeHost(c->stage);
   cudaStreamDestroy(c->stream);
   delete c;
 }

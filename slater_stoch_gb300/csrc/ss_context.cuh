@@ -5,6 +5,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "admission.h"
@@ -62,6 +63,10 @@ struct ss_ctx {
   void* pin = nullptr;
   size_t pin_cap = 0;
   cudaEvent_t pin_evt = nullptr;
+  // pinned staging ring of h2d_copy, and the last copy out of it on each stream
+  char* stage = nullptr;
+  size_t stage_off = 0;
+  std::vector<std::pair<cudaStream_t, cudaEvent_t>> stage_evt;
   int64_t launches = 0;
   int num_sms = 0;
 
@@ -124,6 +129,10 @@ struct ss_ctx {
 namespace ss {
 int dev_alloc(ss_ctx* c, DevBuf& b, size_t bytes);   // (re)allocates only when growing
 void dev_free(ss_ctx* c, DevBuf& b);
+// Copy host memory to the device in stream order; the source is free for reuse when the call
+// returns.  (A plain cudaMemcpyAsync from pageable memory need not have read it by then: where the
+// GPU reaches pageable memory through the host's page tables, it is not staged.)
+int h2d_copy(ss_ctx* c, void* dst, const void* src, size_t bytes);
 int h2d(ss_ctx* c, DevBuf& b, const void* src, size_t bytes);
 // as h2d, through the context's pinned staging buffer, so that the call returns without waiting
 // for the stream (a pageable copy waits for the stream's earlier work)
