@@ -16,7 +16,13 @@ exponential, computed with mpmath at 40 significant digits and rounded once to d
   below 1e-10 relative) and recurs downwards; beyond T = 30 the asymptotic form is exact to
   e^-30.
 
-Run: python slater_stoch_gb300/csrc/gen_boys_tables.py  (rewrites boys_tables.cuh beside it).
+* BOYS_GRID (boys_grid.cuh, for the shell-quartet kernel): grid T_k = k/8 (k = 0..288, T in
+  [0, 36]); row k holds F_n(T_k), n = 0..16; the kernel sums F_L(T_k + d) =
+  sum_{j<9} F_{L+j}(T_k) (-d)^j / j! (|d| <= 1/16, first omitted term below 4e-17 relative) and
+  recurs downwards.
+
+Run: python slater_stoch_gb300/csrc/gen_boys_tables.py  (rewrites boys_tables.cuh and
+boys_grid.cuh beside it).
 """
 from __future__ import annotations
 
@@ -29,6 +35,7 @@ mp.mp.dps = 40
 HI_K, HI_H, HI_T0, HI_J = 281, mp.mpf(1) / 8, mp.mpf(1), 9
 LO_K, LO_H, LO_N = 17, mp.mpf(1) / 16, 25
 B32_K, B32_H, B32_N = 241, mp.mpf(1) / 8, 22
+GRID_K, GRID_H, GRID_N = 289, mp.mpf(1) / 8, 17
 
 
 def boys(n: int, T) -> mp.mpf:
@@ -106,6 +113,24 @@ def main() -> None:
         "",
     ]
     Path(__file__).with_name("boys_tables.cuh").write_text("\n".join(out))
+    grid = [boys(n, k * GRID_H) for k in range(GRID_K) for n in range(GRID_N)]
+    out = [
+        "// boys_grid.cuh -- generated by gen_boys_tables.py (mpmath, 40 digits, rounded once to",
+        "// double); do not edit by hand.",
+        "#pragma once",
+        "",
+        '#include "boys_tables.cuh"',
+        "",
+        "namespace ss {",
+        "",
+        f"constexpr int BOYS_GRID_K = {GRID_K};  // T_k = k/8, T in [0, 36]",
+        f"constexpr int BOYS_GRID_N = {GRID_N};   // F_n(T_k), n = 0..16",
+        "",
+        table("boys_grid_tab", grid, GRID_N),
+        "}  // namespace ss",
+        "",
+    ]
+    Path(__file__).with_name("boys_grid.cuh").write_text("\n".join(out))
 
 
 if __name__ == "__main__":

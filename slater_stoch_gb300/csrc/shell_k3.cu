@@ -1,0 +1,8 @@
+// shell_k3.cu -- shell_eri_kernel of total degree 3 (own translation unit).
+#include "shell_eri.cuh"
+
+namespace ss {
+cudaError_t launch_shell_3(int ncta, int max_no, int max_ni, cudaStream_t st, const ShArgs& A) {
+  return launch_shell_L<3>(ncta, max_no, max_ni, st, A);
+}
+}  // namespace ss

@@ -1,0 +1,8 @@
+// shell_k4.cu -- shell_eri_kernel of total degree 4 (own translation unit).
+#include "shell_eri.cuh"
+
+namespace ss {
+cudaError_t launch_shell_4(int ncta, int max_no, int max_ni, cudaStream_t st, const ShArgs& A) {
+  return launch_shell_L<4>(ncta, max_no, max_ni, st, A);
+}
+}  // namespace ss

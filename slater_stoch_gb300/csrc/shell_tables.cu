@@ -1,0 +1,671 @@
+// shell_tables.cu -- shells and shell pairs of the basis, their primitive tables, and the analytic
+// ERIs of shell quartets (shell_eri.cuh).
+#include <math.h>
+#include <string.h>
+
+#include <algorithm>
+#include <unordered_map>
+#include <vector>
+
+#include "shell_host.h"
+#include "ss_context.cuh"
+
+namespace ss {
+
+#define TRY(x)           \
+  do {                   \
+    int rc_ = (x);       \
+    if (rc_) return rc_; \
+  } while (0)
+
+// ---- pair types ------------------------------------------------------------------------------
+
+static const int SH_DEG[4] = {0, 1, 2, 2};    // S P R D
+static const int SH_NC[4] = {1, 3, 1, 6};
+static const int SH_POW[4][6][3] = {{{0, 0, 0}},
+                                    {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}},
+                                    {{0, 0, 0}},
+                                    {{2, 0, 0}, {1, 1, 0}, {1, 0, 1}, {0, 2, 0}, {0, 1, 1}, {0, 0, 2}}};
+
+// pair type of canonical shell types ta >= tb; same: one shell with itself (components ca >= cb)
+static int struct_index(int ta, int tb, bool same, bool onec) {
+  int base = ta * (ta + 1) / 2 + tb;
+  if (same && ta == SH_P) base = SH_NBASE;
+  if (same && ta == SH_D) base = SH_NBASE + 1;
+  return 2 * base + (onec ? 1 : 0);
+}
+
+static void build_struct(ShStruct& S, int ta, int tb, bool same, bool onec) {
+  memset(&S, 0, sizeof S);
+  S.d = SH_DEG[ta] + SH_DEG[tb];
+  int nterm = 0;
+  for (int ca = 0; ca < SH_NC[ta]; ca++)
+    for (int cb = 0; cb < SH_NC[tb]; cb++) {
+      if (same && cb > ca) continue;
+      const int f = S.ncomp++;
+      const int na = ta == SH_R ? 3 : 1, nb = tb == SH_R ? 3 : 1;
+      int pa[9][3], pb[9][3];
+      for (int x = 0; x < na; x++)
+        for (int y = 0; y < nb; y++) {
+          const int k = S.ncombo[f]++;
+          uint32_t code = 0;
+          for (int ax = 0; ax < 3; ax++) {
+            pa[k][ax] = ta == SH_R ? (ax == x ? 2 : 0) : SH_POW[ta][ca][ax];
+            pb[k][ax] = tb == SH_R ? (ax == y ? 2 : 0) : SH_POW[tb][cb][ax];
+            code |= (uint32_t)pa[k][ax] << (4 * ax) | (uint32_t)pb[k][ax] << (4 * (3 + ax));
+          }
+          S.combo[f][k] = code;
+        }
+      S.fs[f] = nterm;
+      for (int t = 0; t <= S.d; t++)
+        for (int u = 0; t + u <= S.d; u++)
+          for (int v = 0; t + u + v <= S.d; v++) {
+            const int h[3] = {t, u, v};
+            bool any = false;
+            for (int k = 0; k < S.ncombo[f]; k++) {
+              bool ok = true;
+              for (int ax = 0; ax < 3; ax++) {
+                const int e = pa[k][ax] + pb[k][ax];
+                ok = ok && h[ax] <= e && !(onec && ((e - h[ax]) & 1));  // on one centre only equal parities
+              }
+              any = any || ok;
+            }
+            if (any) S.term[nterm++] = (uint32_t)(t | (u << 8) | (v << 16));
+          }
+    }
+  S.fs[S.ncomp] = nterm;
+  S.nterm = nterm;
+}
+
+struct StructTable {
+  std::vector<ShStruct> s;
+  StructTable() : s(SH_NSTRUCT) {
+    for (int ta = 0; ta < 4; ta++)
+      for (int tb = 0; tb <= ta; tb++)
+        for (int oc = 0; oc < 2; oc++) build_struct(s[struct_index(ta, tb, false, oc)], ta, tb, false, oc);
+    for (int oc = 0; oc < 2; oc++) {
+      build_struct(s[struct_index(SH_P, SH_P, true, oc)], SH_P, SH_P, true, oc);
+      build_struct(s[struct_index(SH_D, SH_D, true, oc)], SH_D, SH_D, true, oc);
+    }
+  }
+};
+static const StructTable& structs() {
+  static const StructTable t;
+  return t;
+}
+
+// ---- device tables ---------------------------------------------------------------------------
+
+struct ShFill {
+  ShPrim* prim;
+  double* E;
+  int* cnt;
+};
+
+// Primitive records of one shell pair per CTA, in (m1, m2) order, the primitives with K_AB below
+// the reference's cuts dropped (src/gaussian_product.F90:25-28,
+// src/give_explicit_poly_and_gaussian.F90:46-49), and the Hermite coefficients of every component.
+// fold: both shells have the same fit on one centre, so (m1, m2) and (m2, m1) are the same
+// distribution: m1 <= m2 only, the coefficient doubled for m1 < m2 (exact).
+__global__ void __launch_bounds__(256) shell_fill(BasisDev B, const ShPair* __restrict__ pairs,
+                                                  const ShStruct* __restrict__ st, ShFill out) {
+  const ShPair P = pairs[blockIdx.x];
+  const ShStruct& S = st[P.st];
+  __shared__ int s_wcnt[8], s_total;
+  if (threadIdx.x == 0) s_total = 0;
+  const int na = B.n_gauss[P.fa], nb = B.n_gauss[P.fb];
+  const int64_t ta = B.i_type[P.fa] == 2 ? 1 : 0, tb = B.i_type[P.fb] == 2 ? 1 : 0;
+  const double* A = B.center + 3 * P.fa;
+  const double* C = B.center + 3 * P.fb;
+  const double x0 = A[0] - C[0], x1 = A[1] - C[1], x2 = A[2] - C[2];
+  const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int n = P.same_system ? na * nb : 0;
+  for (int t0 = 0; t0 < n; t0 += 256) {
+    const int t = t0 + threadIdx.x;
+    const int m1 = t / nb, m2 = t - m1 * nb;
+    bool keep = t < n && !(P.fold && m2 < m1);
+    double a = 0, b = 0, K = 0;
+    if (keep) {
+      a = B.g_gauss[m1 + (int64_t)B.ld * P.fa];
+      b = B.g_gauss[m2 + (int64_t)B.ld * P.fb];
+      const double kk = (a * b) * (1.0 / (a + b)) * r2;
+      K = kk > 40.0 ? 0.0 : exp(-kk);
+      keep = !(kk > 40.0) && !(K < 1.e-15);
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    __syncthreads();
+    if (lane == 0) s_wcnt[wid] = __popc(bal);
+    __syncthreads();
+    int pos = s_total + __popc(bal & ((1u << lane) - 1));
+    for (int w = 0; w < wid; w++) pos += s_wcnt[w];
+    if (keep) {
+      ShPrim r;
+      r.p = a + b;
+      const double p_inv = 1.0 / r.p;
+      for (int ax = 0; ax < 3; ax++) r.P[ax] = P.onec ? A[ax] : (a * A[ax] + b * C[ax]) * p_inv;
+      double coef = B.c_gauss[m1 + (int64_t)B.ld * (P.fa + (int64_t)B.n * ta)] *
+                    B.c_gauss[m2 + (int64_t)B.ld * (P.fb + (int64_t)B.n * tb)];
+      if (P.fold && m1 != m2) coef = 2.0 * coef;
+      r.w = (K * coef) * p_inv;
+      r.S = 0.0;
+      out.prim[P.prim_off + pos] = r;
+      // E^{ij}_t of the three axes (McMurchie and Davidson): E^{i+1,j}_t = E^{ij}_{t-1} / 2p +
+      // PA E^{ij}_t + (t+1) E^{ij}_{t+1}, and the same in j with PB
+      const double h = 0.5 * p_inv;
+      double e[3][3][3][5];
+      for (int ax = 0; ax < 3; ax++) {
+        const double pa = P.onec ? 0.0 : r.P[ax] - A[ax], pb = P.onec ? 0.0 : r.P[ax] - C[ax];
+        for (int i = 0; i < 3; i++)
+          for (int j = 0; j < 3; j++) {
+            for (int u = 0; u < 5; u++) {
+              double v = 0.0;
+              if (i == 0 && j == 0) {
+                v = u == 0 ? 1.0 : 0.0;
+              } else {
+                const double* s = j > 0 ? e[ax][i][j - 1] : e[ax][i - 1][0];
+                const double x = j > 0 ? pb : pa;
+                v = x * s[u];
+                if (u > 0) v = fma(h, s[u - 1], v);
+                if (u < 4) v = fma((double)(u + 1), s[u + 1], v);
+              }
+              e[ax][i][j][u] = v;
+            }
+          }
+      }
+      double* E = out.E + P.e_off + (size_t)pos * P.nterm;
+      for (int f = 0; f < S.ncomp; f++)
+        for (int x = S.fs[f]; x < S.fs[f + 1]; x++) {
+          const uint32_t tm = S.term[x];
+          double v = 0.0;
+          for (int k = 0; k < S.ncombo[f]; k++) {
+            const uint32_t c = S.combo[f][k];
+            const double ex = e[0][c & 15][(c >> 12) & 15][tm & 255];
+            const double ey = e[1][(c >> 4) & 15][(c >> 16) & 15][(tm >> 8) & 255];
+            const double ez = e[2][(c >> 8) & 15][(c >> 20) & 15][tm >> 16];
+            v += ex * ey * ez;
+          }
+          E[x] = v;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int w = 0; w < 8; w++) s_total += s_wcnt[w];
+    __syncthreads();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) out.cnt[blockIdx.x] = s_total;
+}
+
+// sum of the slices of every element: elem[e] = sum_s part[e * split + s]
+__global__ void shell_reduce(int nwork, const ShWork* __restrict__ work, const ShPair* __restrict__ pairs, int diag,
+                             const double* __restrict__ part, double* __restrict__ elem) {
+  const ShWork W = work[blockIdx.x];
+  const int ni = diag ? pairs[W.bra].ncomp : pairs[W.bra].ncomp * pairs[W.ket].ncomp;
+  for (int e = threadIdx.x; e < ni; e += blockDim.x) {
+    const double* p = part + W.part + (int64_t)e * W.split;
+    double v = 0.0;
+    for (int s = 0; s < W.split; s++) v = v + p[s];
+    elem[W.elem + e] = v;
+  }
+}
+
+// work entry of every CTA
+__global__ void shell_expand(const ShWork* __restrict__ work, int* __restrict__ cta) {
+  const ShWork W = work[blockIdx.x];
+  for (int s = threadIdx.x; s < W.split; s += blockDim.x) cta[W.cta0 + s] = blockIdx.x;
+}
+
+// Schwarz factors of a pair's primitives and their sorted tables.  A primitive's factor is the
+// largest over the components of sqrt((P_f|P_f) / (f|f)), (f|f) the contracted diagonal: then
+// |(P_f|Q_g)| <= S_P S_Q sqrt((f|f)(g|g)) for every pair of components.  A component without a
+// positive diagonal keeps all its primitives (factor 1e30).  Sorted by decreasing factor (ties:
+// the (m1, m2) order), with an FP32 copy of the records and coefficients.
+__global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pairs, const ShStruct* __restrict__ st,
+                                                  const int* __restrict__ cnt, const double* __restrict__ diag,
+                                                  const ShPrim* __restrict__ prim, const double* __restrict__ E,
+                                                  ShPrim* __restrict__ oprim, ShPrimF* __restrict__ oprimf,
+                                                  double* __restrict__ oE, float* __restrict__ oEf) {
+  __shared__ double s_key[1024];
+  __shared__ int s_idx[1024];
+  const ShPair P = pairs[blockIdx.x];
+  const ShStruct& S = st[P.st];
+  const int m = cnt[blockIdx.x];
+  for (int t = threadIdx.x; t < 1024; t += blockDim.x) {
+    double key = -1.0;
+    if (t < m) {
+      const ShPrim a = prim[P.prim_off + t];
+      const double* e = E + P.e_off + (size_t)t * P.nterm;
+      // (P|P): both on one centre at exponent p/2, so R_{2a 2b 2c} = (2a-1)!!(2b-1)!!(2c-1)!! (-p)^n / (2n+1)
+      const double pre = 34.9868366552 * a.w * a.w * rsqrt(a.p + a.p);
+      key = 0.0;
+      for (int f = 0; f < S.ncomp; f++) {
+        double v = 0.0;
+        for (int x = S.fs[f]; x < S.fs[f + 1]; x++) {
+          double row = 0.0;
+          for (int y = S.fs[f]; y < S.fs[f + 1]; y++) {
+            const uint32_t h = S.term[x] + S.term[y];
+            if (h & 0x010101u) continue;
+            const int hx = h & 255, hy = (h >> 8) & 255, hz = h >> 16;
+            double r = 1.0;
+            for (int i = hx - 1; i > 1; i -= 2) r *= i;
+            for (int i = hy - 1; i > 1; i -= 2) r *= i;
+            for (int i = hz - 1; i > 1; i -= 2) r *= i;
+            const int n = (hx + hy + hz) / 2;
+            for (int i = 0; i < n; i++) r *= -a.p;
+            r /= 2 * n + 1;
+            const int dy = (S.term[y] & 255) + ((S.term[y] >> 8) & 255) + (S.term[y] >> 16);
+            row = fma((dy & 1) ? -r : r, e[y], row);
+          }
+          v = fma(row, e[x], v);
+        }
+        const double d = diag[(size_t)blockIdx.x * SH_MAXCOMP + f];
+        const double s = d > 0.0 ? sqrt(fmax(pre * v, 0.0) / d) : 1e30;
+        key = fmax(key, s < 1e30 ? s : 1e30);  // also where the quotient overflowed or is not a number
+      }
+    }
+    s_key[t] = key;
+    s_idx[t] = t;
+  }
+  __syncthreads();
+  for (int k = 2; k <= 1024; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int t = threadIdx.x; t < 1024; t += blockDim.x) {
+        const int u = t ^ j;
+        if (u > t) {
+          const bool up = (t & k) == 0;
+          const bool first = s_key[t] > s_key[u] || (s_key[t] == s_key[u] && s_idx[t] < s_idx[u]);
+          if (up != first) {
+            const double kk = s_key[t];
+            const int ii = s_idx[t];
+            s_key[t] = s_key[u]; s_idx[t] = s_idx[u];
+            s_key[u] = kk; s_idx[u] = ii;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  for (int t = threadIdx.x; t < m; t += blockDim.x) {
+    ShPrim a = prim[P.prim_off + s_idx[t]];
+    a.S = s_key[t];
+    oprim[P.prim_off + t] = a;
+    ShPrimF g;
+    g.p = (float)a.p;
+    g.w = (float)a.w;
+    for (int ax = 0; ax < 3; ax++) {
+      g.ph[ax] = (float)a.P[ax];
+      g.pl[ax] = (float)(a.P[ax] - (double)g.ph[ax]);
+      g.pad[ax] = 0.f;
+    }
+    g.kx = exp2f(rintf(0.5f * log2f(2.f * g.p)));
+    oprimf[P.prim_off + t] = g;
+  }
+  for (int t = threadIdx.x; t < m * P.nterm; t += blockDim.x) {
+    const int r = t / P.nterm, x = t - r * P.nterm;
+    const double v = E[P.e_off + (size_t)s_idx[r] * P.nterm + x];
+    oE[P.e_off + t] = v;
+    oEf[P.e_off + t] = (float)v;
+  }
+}
+
+#define SH_DECL(L) cudaError_t launch_shell_##L(int, int, int, cudaStream_t, const ShArgs&);
+SH_DECL(0) SH_DECL(1) SH_DECL(2) SH_DECL(3) SH_DECL(4) SH_DECL(5) SH_DECL(6) SH_DECL(7) SH_DECL(8)
+#undef SH_DECL
+
+cudaError_t launch_shell_eri(int L, int ncta, int max_no, int max_ni, cudaStream_t st, const ShArgs& A) {
+  switch (L) {
+#define SH_CASE(l) case l: return launch_shell_##l(ncta, max_no, max_ni, st, A);
+    SH_CASE(0) SH_CASE(1) SH_CASE(2) SH_CASE(3) SH_CASE(4) SH_CASE(5) SH_CASE(6) SH_CASE(7) SH_CASE(8)
+#undef SH_CASE
+  }
+  return cudaErrorInvalidValue;
+}
+
+// ---- host ------------------------------------------------------------------------------------
+
+// Shells of the basis and their pairs (host only; rebuilt by ss_basis_set / ss_basis_systems).
+// A function beyond d, or an r^2-type fit with angular factors, belongs to no shell: its quartets
+// take the per-function kernel (eri_kernel.cuh).
+void build_shells(ss_ctx* c) {
+  ShellBasis& T = c->shells;
+  T = ShellBasis();
+  const int n = c->n, ld = c->ld;
+  T.fsh.assign(n, -1);
+  T.fcomp.assign(n, 0);
+  std::vector<int> first, type, deg_nsys;
+  auto same_fit = [&](int a, int b) {
+    if (c->h_ng[a] != c->h_ng[b] || c->h_itype[a] != c->h_itype[b]) return false;
+    const size_t t = c->h_itype[a] == 2 ? 1 : 0;
+    for (int m = 0; m < c->h_ng[a]; m++)
+      if (c->h_gg[m + (size_t)ld * a] != c->h_gg[m + (size_t)ld * b] ||
+          c->h_cg[m + (size_t)ld * (a + n * t)] != c->h_cg[m + (size_t)ld * (b + n * t)])
+        return false;
+    return true;
+  };
+  auto same_centre = [&](int a, int b) {
+    for (int ax = 0; ax < 3; ax++)
+      if (c->h_center[3 * a + ax] != c->h_center[3 * b + ax]) return false;
+    return true;
+  };
+  auto sys = [&](int f) { return c->h_sys.empty() ? 0 : c->h_sys[f]; };
+  for (int f = 0; f < n; f++) {
+    const int* np = &c->h_npower[3 * f];
+    const int l = np[0] + np[1] + np[2];
+    if (c->h_itype[f] == 2 ? l > 0 : l > 2) {
+      T.all = false;
+      continue;
+    }
+    const int ty = c->h_itype[f] == 2 ? SH_R : (l == 0 ? SH_S : l == 1 ? SH_P : SH_D);
+    int comp = 0;
+    for (int x = 0; x < SH_NC[ty]; x++)
+      if (ty != SH_R && SH_POW[ty][x][0] == np[0] && SH_POW[ty][x][1] == np[1] && SH_POW[ty][x][2] == np[2]) comp = x;
+    T.fcomp[f] = comp;
+    // a shell with this fit whose component is still free (components are mostly consecutive: the
+    // latest shells first)
+    for (int s = (int)first.size() - 1; s >= 0 && T.fsh[f] < 0; s--)
+      if (type[s] == ty && sys(first[s]) == sys(f) && same_centre(first[s], f) && same_fit(first[s], f)) T.fsh[f] = s;
+    if (T.fsh[f] < 0) {
+      T.fsh[f] = (int)first.size();
+      first.push_back(f);
+      type.push_back(ty);
+    }
+  }
+  const int nsh = (int)first.size();
+  T.nsh = nsh;
+  T.pair.clear();
+  T.spair.assign((size_t)nsh * nsh, -1);
+  T.flip.assign((size_t)nsh * nsh, 0);
+  int64_t po = 0, eo = 0;
+  for (int x = 0; x < nsh; x++)
+    for (int y = 0; y <= x; y++) {
+      int a = x, b = y;
+      if (type[a] < type[b]) std::swap(a, b);
+      ShPair P{};
+      P.fa = first[a];
+      P.fb = first[b];
+      P.onec = same_centre(P.fa, P.fb);
+      P.fold = P.onec && same_fit(P.fa, P.fb);
+      P.same_system = sys(P.fa) == sys(P.fb);
+      P.st = struct_index(type[a], type[b], a == b, P.onec);
+      const ShStruct& S = structs().s[P.st];
+      P.d = S.d;
+      P.ncomp = S.ncomp;
+      P.nterm = S.nterm;
+      const int na = c->h_ng[P.fa], nb = c->h_ng[P.fb];
+      P.cap = P.fold ? na * (na + 1) / 2 : na * nb;
+      P.prim_off = po;
+      P.e_off = eo;
+      po += P.cap;
+      eo += (int64_t)P.cap * P.nterm;
+      T.spair[(size_t)x * nsh + y] = T.spair[(size_t)y * nsh + x] = (int)T.pair.size();
+      // (x, y) as given is (b, a) of the pair
+      T.flip[(size_t)a * nsh + b] = 0;
+      T.flip[(size_t)b * nsh + a] = a != b;
+      T.pair.push_back(P);
+    }
+  T.nb.resize(nsh);
+  for (int s = 0; s < nsh; s++) T.nb[s] = SH_NC[type[s]];
+  T.nprim = po;
+  T.nE = eo;
+}
+
+// shell pair and component of functions i and k; false if one of them is in no shell
+static bool shell_component(const ShellBasis& T, int i, int k, int* pair, int* comp) {
+  int a = T.fsh[i], b = T.fsh[k];
+  if (a < 0 || b < 0) return false;
+  int ca = T.fcomp[i], cb = T.fcomp[k];
+  if (T.flip[(size_t)a * T.nsh + b]) {
+    std::swap(a, b);
+    std::swap(ca, cb);
+  }
+  *pair = T.spair[(size_t)a * T.nsh + b];
+  if (a == b) {
+    if (ca < cb) std::swap(ca, cb);
+    *comp = ca * (ca + 1) / 2 + cb;
+  } else {
+    *comp = ca * T.nb[b] + cb;
+  }
+  return true;
+}
+
+// multiply-adds per primitive quartet beyond the Hermite integrals; an s-type bra needs no
+// contraction per bra primitive
+static double side_cost(const ShPair& b, const ShPair& k) {
+  const double h = sh_nherm(b.d);
+  return h * k.nterm + (b.d > 0 ? 6.0 : 0.0);
+}
+
+// bra slices of a shell quartet: a CTA's bra primitives so that it has about 1e6 multiply-adds at
+// a hundred kept kets each, at most SH_MAXSLICE of them; never from what else is in the list, so
+// that the order of summation is the quartet's own
+static int slices(const ShPair& b, const ShPair& k) {
+  const int L = b.d + k.d;
+  static const double rec[SH_MAXL + 1] = {2, 8, 24, 60, 120, 200, 330, 520, 790};
+  const double cost = 30.0 + 4.0 * L + rec[L] + side_cost(b, k);
+  int per = (int)std::min(16.0, std::max(2.0, 1e4 / cost));
+  per = std::max(per, (b.cap + 126) / 127);
+  return std::max(1, (b.cap + per - 1) / per);
+}
+
+
+// Launch the work entries (grouped by total degree), in chunks whose partial sums fit the buffer,
+// and reduce each chunk's partial sums to elements.
+static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF* primf, const double* E, const float* Ef,
+                    bool diag, double eps, double eps32, double* elem) {
+  const ShellBasis& T = c->shells;
+  // partial sums in flight: enough for a whole mid-size system, and bounded
+  size_t cap = (size_t)64 << 20;
+  if (c->budget) cap = std::min(cap, std::max<size_t>((c->budget - std::min(c->budget, c->used)) / 4, 1 << 20));
+  const int64_t cap_d = (int64_t)(cap / sizeof(double));
+  // heaviest degrees first: their CTAs are the longest
+  std::vector<ShWork> chunk;
+  struct Seg { int L, first, n, ncta, no, ni; };
+  std::vector<Seg> segs;
+  int64_t part = 0, most = 0;
+  int ncta = 0;
+  auto flush = [&]() -> int {
+    if (chunk.empty()) return SS_OK;
+    void *dw, *dc, *dp;
+    TRY(pool_get(c, "shell_part", sizeof(double) * (size_t)std::max(part, std::min(most, cap_d)), &dp));
+    DevBuf& wb = c->pool["shell_work"];
+    TRY(h2d_async(c, wb, chunk.data(), sizeof(ShWork) * chunk.size()));
+    dw = wb.ptr;
+    TRY(pool_get(c, "shell_cta", sizeof(int) * (size_t)ncta, &dc));
+    shell_expand<<<(unsigned)chunk.size(), 32, 0, c->stream>>>((const ShWork*)dw, (int*)dc);
+    SS_CUDA_TRY(cudaGetLastError());
+    c->launches++;
+    TRY(fork_eri_streams(c));
+    ShArgs A{};
+    A.pair = (const ShPair*)c->pool["shell_pair"].ptr;
+    A.cnt = (const int*)c->pool["shell_cnt"].ptr;
+    A.st = (const ShStruct*)c->pool["shell_struct"].ptr;
+    A.prim = prim;
+    A.primf = primf;
+    A.E = E;
+    A.Ef = Ef;
+    A.partial = (double*)dp;
+    A.eps = eps;
+    A.eps32 = eps32;
+    A.diag = diag;
+    int rc = SS_OK;
+    for (size_t s = 0; s < segs.size() && !rc; s++) {
+      const Seg& g = segs[s];
+      A.work = (const ShWork*)dw;
+      A.cta = (const int*)dc;
+      A.cta0 = chunk[g.first].cta0;
+      const cudaError_t e = launch_shell_eri(g.L, g.ncta, g.no, g.ni, c->eri_stream[s % ss_ctx::ERI_STREAMS], A);
+      if (e != cudaSuccess) {
+        ss_set_cuda_error(e, "shell_eri_kernel launch", __FILE__, __LINE__);
+        rc = SS_ERR_CUDA;
+      }
+      c->launches++;
+    }
+    const int jrc = join_eri_streams(c);
+    if (rc || jrc) return rc ? rc : jrc;
+    shell_reduce<<<(unsigned)chunk.size(), 64, 0, c->stream>>>((int)chunk.size(), (const ShWork*)dw, A.pair, diag,
+                                                               (const double*)dp, elem);
+    SS_CUDA_TRY(cudaGetLastError());
+    c->launches++;
+    chunk.clear();
+    segs.clear();
+    part = 0;
+    ncta = 0;
+    return SS_OK;
+  };
+  for (int L = 0; L <= SH_MAXL; L++)
+    for (const ShWork& w : Lw.work[L]) most += (int64_t)w.split * (diag ? T.pair[w.bra].ncomp : T.pair[w.bra].ncomp * T.pair[w.ket].ncomp);
+  for (int L = SH_MAXL; L >= 0; L--) {
+    std::vector<ShWork>& v = Lw.work[L];
+    auto cost = [&](const ShWork& w) { return side_cost(T.pair[w.bra], T.pair[w.ket]); };
+    std::stable_sort(v.begin(), v.end(), [&](const ShWork& a, const ShWork& b) { return cost(a) > cost(b); });
+    bool open = false;
+    for (ShWork& w : v) {
+      const ShPair &b = T.pair[w.bra], &k = T.pair[w.ket];
+      const int ni = b.ncomp * k.ncomp;
+      const int64_t need = (int64_t)w.split * (diag ? b.ncomp : ni);
+      if (!chunk.empty() && (part + need > cap_d || ncta > (1 << 28))) {
+        TRY(flush());
+        open = false;
+      }
+      if (!open) {
+        segs.push_back(Seg{L, (int)chunk.size(), 0, 0, 0, 0});
+        open = true;
+      }
+      Seg& g = segs.back();
+      w.cta0 = ncta;
+      w.part = part;
+      chunk.push_back(w);
+      g.n++;
+      g.ncta += w.split;
+      g.no = std::max(g.no, sh_nherm(b.d) * k.ncomp);
+      g.ni = std::max(g.ni, ni);
+      ncta += w.split;
+      part += need;
+    }
+  }
+  return flush();
+}
+
+// Primitive tables of the shell pairs and the Schwarz diagonal (ik|ik) of every function pair in
+// shells, into the host matrix pre (n x n); other pairs' entries are left as they are.
+int shell_precond(ss_ctx* c, std::vector<double>& pre) {
+  const ShellBasis& T = c->shells;
+  const int np = (int)T.pair.size();
+  if (!np) return SS_OK;
+  void* p;
+  TRY(pool_get(c, "shell_struct", sizeof(ShStruct) * SH_NSTRUCT, &p));
+  TRY(h2d_copy(c, p, structs().s.data(), sizeof(ShStruct) * SH_NSTRUCT));
+  const ShStruct* st = (const ShStruct*)p;
+  TRY(h2d_async(c, c->pool["shell_pair"], T.pair.data(), sizeof(ShPair) * np));
+  const ShPair* dpair = (const ShPair*)c->pool["shell_pair"].ptr;
+  ShFill F;
+  int* cnt;
+  double *E2, *diag;
+  ShPrim* prim2;
+  ShPrimF* primf;
+  float* Ef;
+  TRY(pool_get(c, "shell_prim0", sizeof(ShPrim) * T.nprim, &p)); F.prim = (ShPrim*)p;
+  TRY(pool_get(c, "shell_E0", sizeof(double) * T.nE, &p)); F.E = (double*)p;
+  TRY(pool_get(c, "shell_cnt", sizeof(int) * np, &p)); F.cnt = cnt = (int*)p;
+  TRY(pool_get(c, "shell_prim", sizeof(ShPrim) * T.nprim, &p)); prim2 = (ShPrim*)p;
+  TRY(pool_get(c, "shell_primf", sizeof(ShPrimF) * T.nprim, &p)); primf = (ShPrimF*)p;
+  TRY(pool_get(c, "shell_E", sizeof(double) * T.nE, &p)); E2 = (double*)p;
+  TRY(pool_get(c, "shell_Ef", sizeof(float) * T.nE, &p)); Ef = (float*)p;
+  TRY(pool_get(c, "shell_diag", sizeof(double) * np * SH_MAXCOMP, &p)); diag = (double*)p;
+  SS_CUDA_TRY(cudaMemsetAsync(diag, 0, sizeof(double) * np * SH_MAXCOMP, c->stream));
+  shell_fill<<<np, 256, 0, c->stream>>>(c->basis, dpair, st, F);
+  SS_CUDA_TRY(cudaGetLastError());
+  c->launches++;
+  ShellPlan Lw;
+  for (int x = 0; x < np; x++) {
+    const ShPair& P = T.pair[x];
+    if (!P.same_system) continue;
+    ShWork w{};
+    w.bra = w.ket = x;
+    w.split = slices(P, P);
+    w.elem = (int64_t)x * SH_MAXCOMP;
+    w.mask = ~0ull;
+    Lw.work[2 * P.d].push_back(w);
+  }
+  TRY(run_work(c, Lw, F.prim, nullptr, F.E, nullptr, true, 0.0, 0.0, diag));
+  shell_sort<<<np, 512, 0, c->stream>>>(dpair, st, cnt, diag, F.prim, F.E, prim2, primf, E2, Ef);
+  SS_CUDA_TRY(cudaGetLastError());
+  c->launches++;
+  std::vector<double> h((size_t)np * SH_MAXCOMP);
+  SS_CUDA_TRY(cudaMemcpyAsync(h.data(), diag, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
+  SS_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  const int n = c->n;
+  for (int i = 0; i < n; i++)
+    for (int k = 0; k <= i; k++) {
+      int pr, f;
+      if (!shell_component(T, i, k, &pr, &f)) continue;
+      pre[i + (size_t)n * k] = pre[k + (size_t)n * i] = h[(size_t)pr * SH_MAXCOMP + f];
+    }
+  return SS_OK;
+}
+
+// Shell quartets of the selected function quartets.  Quartets with a function in no shell go to
+// `rest`; of the others, slot[q] receives the place of the result (one element, offset from
+// `first`), and *nelem the number of elements.
+int shell_plan(ss_ctx* c, const std::vector<int64_t>& sel, std::vector<int64_t>& slot, std::vector<int64_t>& rest,
+               ShellPlan& plan, int64_t* nelem) {
+  const ShellBasis& T = c->shells;
+  const int n = c->n;
+  std::vector<int32_t> fpair((size_t)n * n, -1);
+  std::vector<int16_t> fcomp((size_t)n * n, 0);
+  for (int i = 0; i < n; i++)
+    for (int k = 0; k <= i; k++) {
+      int pr, f;
+      if (!shell_component(T, i, k, &pr, &f)) continue;
+      fpair[i + (size_t)n * k] = pr;
+      fcomp[i + (size_t)n * k] = (int16_t)f;
+    }
+  const int64_t np = (int64_t)T.pair.size(), nkey = np * (np + 1) / 2;
+  const bool dense = nkey <= (int64_t)64 << 20;
+  std::vector<int32_t> where(dense ? nkey : 0, -1);
+  std::unordered_map<int64_t, int32_t> sparse;
+  struct Quartet { int bra, ket; uint64_t mask; int64_t elem; };
+  std::vector<Quartet> Q;
+  int64_t elem = 0;
+  for (int64_t t : sel) {
+    const int i = c->h_is[t] - 1, k = c->h_ks[t] - 1, j = c->h_js[t] - 1, l = c->h_ls[t] - 1;
+    const size_t a = i + (size_t)n * k, b = j + (size_t)n * l;
+    const int pa = fpair[a], pb = fpair[b];
+    if (pa < 0 || pb < 0) {
+      rest.push_back(t);
+      continue;
+    }
+    const int64_t hi = std::max(pa, pb), lo = std::min(pa, pb), key = hi * (hi + 1) / 2 + lo;
+    int32_t* w = dense ? &where[key] : &sparse.emplace(key, -1).first->second;
+    if (*w < 0) {
+      *w = (int32_t)Q.size();
+      const ShPair &x = T.pair[hi], &y = T.pair[lo];
+      const bool fwd = side_cost(x, y) <= side_cost(y, x);  // the cheaper side as the bra
+      Q.push_back(Quartet{(int)(fwd ? hi : lo), (int)(fwd ? lo : hi), 0, elem});
+      elem += (int64_t)x.ncomp * y.ncomp;
+    }
+    Quartet& s = Q[*w];
+    const int nf = T.pair[s.ket].ncomp;
+    const int fb = pa == s.bra ? fcomp[a] : fcomp[b], fk = pa == s.bra ? fcomp[b] : fcomp[a];
+    s.mask |= 1ull << fk;
+    slot[t] = (s.elem + (int64_t)fb * nf + fk) << SLOT_SPLIT_BITS | 1;
+  }
+  for (const Quartet& s : Q) {
+    ShWork w{};
+    w.bra = s.bra;
+    w.ket = s.ket;
+    w.split = slices(T.pair[s.bra], T.pair[s.ket]);
+    w.elem = s.elem;
+    w.mask = s.mask;
+    plan.work[T.pair[s.bra].d + T.pair[s.ket].d].push_back(w);
+  }
+  *nelem = elem;
+  return SS_OK;
+}
+
+int shell_run(ss_ctx* c, ShellPlan& plan, double eps, double eps32, double* elem) {
+  return run_work(c, plan, (const ShPrim*)c->pool["shell_prim"].ptr, (const ShPrimF*)c->pool["shell_primf"].ptr,
+                  (const double*)c->pool["shell_E"].ptr, (const float*)c->pool["shell_Ef"].ptr, false, eps, eps32, elem);
+}
+
+}  // namespace ss

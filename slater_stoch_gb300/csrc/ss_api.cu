@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "ss_common.cuh"
+#include "shell_host.h"
 #include "ss_context.cuh"
 
 namespace ss {
@@ -162,13 +163,45 @@ static int pair_L(const ss_ctx* c, int f1, int f2) {
   return L;
 }
 
-// Run the ERI kernels for the quartets listed in (qis..qls) restricted to `sel` (indices into
-// them); partial sums are written to d_scratch_b and slot[q] gives the partial row of q.
+int fork_eri_streams(ss_ctx* c) {
+  if (!c->eri_fork) {
+    int lo = 0, hi = 0;  // lowest priority: the MC of a job runs beside the analytic stage
+    SS_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    for (int s = 0; s < ss_ctx::ERI_STREAMS; s++) {
+      SS_CUDA_TRY(cudaStreamCreateWithPriority(&c->eri_stream[s], cudaStreamNonBlocking, lo));
+      SS_CUDA_TRY(cudaEventCreateWithFlags(&c->eri_join[s], cudaEventDisableTiming));
+    }
+    SS_CUDA_TRY(cudaEventCreateWithFlags(&c->eri_fork, cudaEventDisableTiming));
+  }
+  SS_CUDA_TRY(cudaEventRecord(c->eri_fork, c->stream));
+  for (int s = 0; s < ss_ctx::ERI_STREAMS; s++) SS_CUDA_TRY(cudaStreamWaitEvent(c->eri_stream[s], c->eri_fork, 0));
+  return SS_OK;
+}
+
+int join_eri_streams(ss_ctx* c) {
+  for (int s = 0; s < ss_ctx::ERI_STREAMS; s++) {
+    SS_CUDA_TRY(cudaEventRecord(c->eri_join[s], c->eri_stream[s]));
+    SS_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->eri_join[s], 0));
+  }
+  return SS_OK;
+}
+
+// Run the per-function ERI kernels for the quartets listed in (qis..qls) restricted to `sel`
+// (indices into them); partial sums are written to d_scratch_b from entry `first` on and slot[q]
+// gives the partial row of q.  These kernels serve the quartets that have a function in no shell
+// (shell_tables.cu); the others take the shell-quartet kernel.
+static int reset_tables(ss_ctx* c) {
+  build_shells(c);
+  c->have_precond = c->have_gauss = c->have_mc = false;
+  c->have_resid = c->have_mono = false;
+  return SS_OK;
+}
+
 static int run_eri(ss_ctx* c, const int32_t* d_qis, const int32_t* d_qjs, const int32_t* d_qks,
                    const int32_t* d_qls, const std::vector<int32_t>& qis, const std::vector<int32_t>& qjs,
                    const std::vector<int32_t>& qks, const std::vector<int32_t>& qls,
-                   const std::vector<int64_t>& sel, std::vector<int64_t>& slot_of_sel, int64_t& npartial,
-                   const double* d_pre, double eps, double eps32, double* self_out = nullptr) {
+                   const std::vector<int64_t>& sel, std::vector<int64_t>& slot_of_sel, int64_t first,
+                   int64_t& npartial, const double* d_pre, double eps, double eps32, double* self_out = nullptr) {
   // bucket by class (L = max(bra L, ket L), tc = number of r^2-type fits among the four
   // functions) and the ket bound of the light-ket rule (ss_light_ket): v = LK + 1, or 0 for the
   // full-L instance.  A light-ket quartet is evaluated as (jl|ik) when (j,l) is the lighter pair
@@ -192,7 +225,7 @@ static int run_eri(ss_ctx* c, const int32_t* d_qis, const int32_t* d_qjs, const 
   work.reserve(sel.size());
   std::vector<int64_t> begin(NB), count(NB), pbase(NB + 1, 0);
   std::vector<int> maxk(NB, 0), bsplit(NB, 1);
-  slot_of_sel.assign(qis.size(), -1);
+  pbase[0] = first;
   for (int bk = 0; bk < NB; bk++) {
     begin[bk] = (int64_t)work.size();
     const int64_t cnt = (int64_t)bucket[bk].size();
@@ -220,24 +253,14 @@ static int run_eri(ss_ctx* c, const int32_t* d_qis, const int32_t* d_qjs, const 
   if (rc) return rc;
   const int64_t* d_work = (const int64_t*)c->d_scratch_a.ptr;
   double* d_partial = (double*)c->d_scratch_b.ptr;
-  // classes launched round-robin over the side streams, largest launch first; the side streams
-  // start after everything queued on the context stream and the context stream waits for all
-  if (!c->eri_fork) {
-    int lo = 0, hi = 0;  // lowest priority: the MC of a job runs beside the analytic stage
-    SS_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-    for (int s = 0; s < ss_ctx::ERI_STREAMS; s++) {
-      SS_CUDA_TRY(cudaStreamCreateWithPriority(&c->eri_stream[s], cudaStreamNonBlocking, lo));
-      SS_CUDA_TRY(cudaEventCreateWithFlags(&c->eri_join[s], cudaEventDisableTiming));
-    }
-    SS_CUDA_TRY(cudaEventCreateWithFlags(&c->eri_fork, cudaEventDisableTiming));
-  }
+  // classes launched round-robin over the side streams, largest launch first
   std::vector<int> order;
   for (int bk = 0; bk < NB; bk++)
     if (count[bk]) order.push_back(bk);
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return count[a] * bsplit[a] > count[b] * bsplit[b]; });
-  SS_CUDA_TRY(cudaEventRecord(c->eri_fork, c->stream));
-  for (int s = 0; s < ss_ctx::ERI_STREAMS; s++) SS_CUDA_TRY(cudaStreamWaitEvent(c->eri_stream[s], c->eri_fork, 0));
+  rc = fork_eri_streams(c);
+  if (rc) return rc;
   int launch_rc = SS_OK;
   for (size_t oi = 0; oi < order.size() && !launch_rc; oi++) {
     const int bk = order[oi];
@@ -268,11 +291,8 @@ static int run_eri(ss_ctx* c, const int32_t* d_qis, const int32_t* d_qjs, const 
       c->launches++;
     }
   }
-  for (int s = 0; s < ss_ctx::ERI_STREAMS; s++) {
-    SS_CUDA_TRY(cudaEventRecord(c->eri_join[s], c->eri_stream[s]));
-    SS_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->eri_join[s], 0));
-  }
-  return launch_rc;
+  rc = join_eri_streams(c);
+  return launch_rc ? launch_rc : rc;
 }
 
 int build_pair_tables(ss_ctx* c);
@@ -313,71 +333,76 @@ static int sort_prim_pairs(ss_ctx* c) {
   return SS_OK;
 }
 
+// Schwarz diagonal of the function pairs that have a function in no shell, by the per-function
+// kernels, into pre; also the Schwarz factors and the order of all primitive pairs, which their
+// quartets with shell functions need.
+static int function_precond(ss_ctx* c, std::vector<double>& pre) {
+  TRY(build_pair_tables(c));
+  // diagonal quartets (ik|ik), i >= k, in pair-index order (src/two_e_slater.F90:230-236)
+  int n = c->n;
+  int64_t np = (int64_t)n * (n + 1) / 2;
+  std::vector<int32_t> qi(np), qk(np);
+  // a pair without primitive pairs (all screened, or functions of two systems) has (ik|ik) = 0
+  std::vector<int64_t> sel, own, slot(np, -1);
+  for (int i = 0; i < n; i++)
+    for (int k = 0; k <= i; k++) {
+      int64_t p = ss_pair_index(i, k);
+      qi[p] = i + 1;
+      qk[p] = k + 1;
+      if (c->h_pp_cnt[p] == 0) continue;
+      sel.push_back(p);
+      if (c->shells.fsh[i] < 0 || c->shells.fsh[k] < 0) own.push_back(p);
+    }
+  DevBuf di, dk;
+  int rc = h2d(c, di, qi.data(), sizeof(int32_t) * np);
+  if (!rc) rc = h2d(c, dk, qk.data(), sizeof(int32_t) * np);
+  int64_t npartial = 0;
+  // 1. primitive-pair Schwarz factors (items (P,P) of the diagonal quartets) into pad[0],
+  // 2. per-pair sort by decreasing factor, 3. the diagonal quartets themselves
+  if (!rc)
+    rc = run_eri(c, (const int32_t*)di.ptr, (const int32_t*)di.ptr, (const int32_t*)dk.ptr,
+                 (const int32_t*)dk.ptr, qi, qi, qk, qk, sel, slot, 0, npartial, nullptr, 0.0, 0.0,
+                 (double*)((char*)c->d_pp.ptr + offsetof(PrimPair, pad)));
+  if (!rc) rc = sort_prim_pairs(c);
+  slot.assign(np, -1);
+  if (!rc)
+    rc = run_eri(c, (const int32_t*)di.ptr, (const int32_t*)di.ptr, (const int32_t*)dk.ptr,
+                 (const int32_t*)dk.ptr, qi, qi, qk, qk, own, slot, 0, npartial, nullptr, 0.0, 0.0);
+  std::vector<double> part((size_t)std::max<int64_t>(npartial, 1));
+  cudaError_t e = cudaSuccess;
+  if (!rc) {
+    e = cudaMemcpyAsync(part.data(), c->d_scratch_b.ptr, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  }
+  dev_free(c, di);
+  dev_free(c, dk);
+  if (rc) return rc;
+  if (e != cudaSuccess) {
+    ss_set_cuda_error(e, "precond copy", __FILE__, __LINE__);
+    return SS_ERR_CUDA;
+  }
+  for (int64_t p : own) {
+    double v = 0.0;
+    for (int t = 0; t < slot_split(slot[p]); t++) v = v + part[slot_offset(slot[p]) + t];
+    const int i = qi[p] - 1, k = qk[p] - 1;
+    pre[i + (size_t)n * k] = v;
+    pre[k + (size_t)n * i] = v;
+  }
+  return SS_OK;
+}
+
 int ensure_precond(ss_ctx* c) {
   if (c->have_precond) return SS_OK;
   if (!c->n) {
     ss_set_error_msg("no basis set");
     return SS_ERR_STATE;
   }
-  // diagonal quartets (ik|ik), i >= k, in pair-index order (src/two_e_slater.F90:230-236)
-  int n = c->n;
-  int64_t np = (int64_t)n * (n + 1) / 2;
-  std::vector<int32_t> qi(np), qk(np);
-  for (int i = 0; i < n; i++)
-    for (int k = 0; k <= i; k++) {
-      int64_t p = ss_pair_index(i, k);
-      qi[p] = i + 1;
-      qk[p] = k + 1;
-    }
-  DevBuf di, dk;
-  int rc = h2d(c, di, qi.data(), sizeof(int32_t) * np);
-  if (!rc) rc = h2d(c, dk, qk.data(), sizeof(int32_t) * np);
-  // a pair without primitive pairs (all screened, or functions of two systems) has (ik|ik) = 0
-  std::vector<int64_t> sel, slot;
-  sel.reserve(np);
-  for (int64_t p = 0; p < np; p++)
-    if (c->h_pp_cnt[p] > 0) sel.push_back(p);
-  int64_t npartial = 0;
-  // 1. primitive-pair Schwarz factors (items (P,P) of the diagonal quartets) into pad[0],
-  // 2. per-pair sort by decreasing factor, 3. the diagonal quartets themselves
-  if (!rc)
-    rc = run_eri(c, (const int32_t*)di.ptr, (const int32_t*)di.ptr, (const int32_t*)dk.ptr,
-                 (const int32_t*)dk.ptr, qi, qi, qk, qk, sel, slot, npartial, nullptr, 0.0, 0.0,
-                 (double*)((char*)c->d_pp.ptr + offsetof(PrimPair, pad)));
-  if (!rc) rc = sort_prim_pairs(c);
-  if (!rc)
-    rc = run_eri(c, (const int32_t*)di.ptr, (const int32_t*)di.ptr, (const int32_t*)dk.ptr,
-                 (const int32_t*)dk.ptr, qi, qi, qk, qk, sel, slot, npartial, nullptr, 0.0, 0.0);
-  if (rc) {
-    dev_free(c, di);
-    dev_free(c, dk);
-    return rc;
-  }
-  // slots are a permutation of pair indices: gather partials back into pair order on the host side
-  // by re-sorting (cheap: np entries)
-  std::vector<double> part((size_t)std::max<int64_t>(npartial, 1));
-  rc = dev_alloc(c, c->d_precond, sizeof(double) * n * n);
-  if (rc) return rc;
-  cudaError_t e = cudaMemcpyAsync(part.data(), c->d_scratch_b.ptr, sizeof(double) * part.size(),
-                                  cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  dev_free(c, di);
-  dev_free(c, dk);
-  if (e != cudaSuccess) {
-    ss_set_cuda_error(e, "precond copy", __FILE__, __LINE__);
-    return SS_ERR_CUDA;
-  }
+  const int n = c->n;
   c->h_precond.assign((size_t)n * n, 0.0);
-  for (int64_t p = 0; p < np; p++) {
-    double v = 0.0;
-    if (slot[p] >= 0)
-      for (int t = 0; t < slot_split(slot[p]); t++) v = v + part[slot_offset(slot[p]) + t];
-    int i = qi[p] - 1, k = qk[p] - 1;
-    c->h_precond[i + (size_t)n * k] = v;
-    c->h_precond[k + (size_t)n * i] = v;
-  }
-  SS_CUDA_TRY(cudaMemcpyAsync(c->d_precond.ptr, c->h_precond.data(), sizeof(double) * n * n,
-                              cudaMemcpyHostToDevice, c->stream));
+  TRY(shell_precond(c, c->h_precond));
+  if (!c->shells.all) TRY(function_precond(c, c->h_precond));
+  TRY(dev_alloc(c, c->d_precond, sizeof(double) * n * n));
+  TRY(h2d_copy(c, c->d_precond.ptr, c->h_precond.data(), sizeof(double) * n * n));
   c->have_precond = true;
   return SS_OK;
 }
@@ -404,12 +429,19 @@ int ensure_gauss(ss_ctx* c) {
     if (!small) sel.push_back(q);
   }
   c->n_removed = nzero;
-  std::vector<int64_t> slot;
-  int64_t npartial = 0;
-  rc = run_eri(c, (const int32_t*)c->d_is.ptr, (const int32_t*)c->d_js.ptr, (const int32_t*)c->d_ks.ptr,
-               (const int32_t*)c->d_ls.ptr, c->h_is, c->h_js, c->h_ks, c->h_ls, sel, slot, npartial,
-               (const double*)c->d_precond.ptr, c->eri_eps_screen, c->eri_eps32);
-  if (rc) return rc;
+  std::vector<int64_t> slot(c->nint, -1), rest;
+  ShellPlan plan;
+  int64_t nelem = 0, npartial = 0;
+  TRY(shell_plan(c, sel, slot, rest, plan, &nelem));
+  // results: one element per component of the shell quartets, then the per-function partial sums
+  if (rest.empty()) {
+    TRY(dev_alloc(c, c->d_scratch_b, sizeof(double) * std::max<int64_t>(nelem, 1)));
+  } else {
+    TRY(run_eri(c, (const int32_t*)c->d_is.ptr, (const int32_t*)c->d_js.ptr, (const int32_t*)c->d_ks.ptr,
+                (const int32_t*)c->d_ls.ptr, c->h_is, c->h_js, c->h_ks, c->h_ls, rest, slot, nelem, npartial,
+                (const double*)c->d_precond.ptr, c->eri_eps_screen, c->eri_eps32));
+  }
+  TRY(shell_run(c, plan, c->eri_eps_screen, c->eri_eps32, (double*)c->d_scratch_b.ptr));
   rc = h2d_async(c, c->d_scratch_c, slot.data(), sizeof(int64_t) * c->nint);
   if (rc) return rc;
   rc = dev_alloc(c, c->d_gauss, sizeof(double) * c->nint);
@@ -604,7 +636,7 @@ int ss_basis_set(ss_ctx* c, int nbasis, const double* center, const int* npower,
                       (const double*)c->d_cg.ptr, (const double*)c->d_gg.ptr, (const double*)c->d_gs.ptr,
                       nullptr};
   c->h_sys.clear();
-  return build_pair_tables(c);
+  return reset_tables(c);
 }
 
 int ss_basis_systems(ss_ctx* c, int nsys, const int* first) {
@@ -629,7 +661,7 @@ int ss_basis_systems(ss_ctx* c, int nsys, const int* first) {
   if (rc) return rc;
   c->h_sys = sys;
   c->basis.sys = (const int*)c->d_sys.ptr;
-  return build_pair_tables(c);
+  return reset_tables(c);
 }
 
 }  // extern "C"
@@ -660,8 +692,6 @@ int build_pair_tables(ss_ctx* c) {
                                                (PrimPair*)c->d_pp.ptr);
   SS_CUDA_TRY(cudaGetLastError());
   c->launches++;
-  c->have_precond = c->have_gauss = c->have_mc = false;
-  c->have_resid = c->have_mono = false;
   return SS_OK;
 }
 }  // namespace ss

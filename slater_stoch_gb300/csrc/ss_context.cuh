@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "admission.h"
+#include "shell.cuh"
 #include "ss_common.cuh"
 
 namespace ss {
@@ -19,14 +20,15 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
-struct EriPlan {
-  // one entry per (class L) bucket; work lists hold quartet indices
-  std::vector<int> L;
-  std::vector<int64_t> begin, count;  // into work[]
-  std::vector<int> split;
-  std::vector<int64_t> partial_begin;  // into partial[]
-  std::vector<int> max_ket;            // largest ket primitive-pair count in the bucket
-  int64_t total_partial = 0;
+// Shells of the basis (shell_tables.cu): shell and component of every function (-1: in no shell),
+// the pair of every two shells, and whether a pair holds them in the other order.
+struct ShellBasis {
+  bool all = true;  // every function is in a shell
+  int nsh = 0;
+  std::vector<int> fsh, fcomp, nb, spair;
+  std::vector<char> flip;
+  std::vector<ShPair> pair;
+  int64_t nprim = 0, nE = 0;
 };
 
 // Parameters of the shared-walker proposal: a mixture of ZV-map densities
@@ -82,7 +84,9 @@ struct ss_ctx {
   // nuclei for the one-electron nuclear attraction (ss_nuclei_set)
   std::vector<double> h_nuc_xyz, h_nuc_charge;
 
-  // primitive pairs
+  ss::ShellBasis shells;
+
+  // primitive pairs of the per-function kernels (built when a function is in no shell)
   ss::DevBuf d_pp, d_pp_off, d_pp_cnt;
   ss::DevBuf d_ppf;  // FP32 copies of the sorted primitive pairs (mixed-precision tier)
   std::vector<int> h_pp_cnt;
