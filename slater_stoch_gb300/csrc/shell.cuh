@@ -56,10 +56,10 @@ struct ShPair {
 struct ShPrim {
   double p, P[3], w, S;
 };
-// FP32 view: the centre as two floats; kx = 2^k ~ sqrt(2p) scales the Hermite degrees of the FP32
-// evaluation (shell_eri.cuh)
+// Two-float view (high and low parts); w is divided by the pair's power of two (ShArgs::scale), and
+// kx = 2^k ~ sqrt(2p) scales the Hermite degrees of the FP32 evaluations (shell_eri.cuh)
 struct ShPrimF {
-  float p, ph[3], pl[3], w, kx, pad[3];
+  float p[2], ph[3], pl[3], w[2], kx, pad;
 };
 static_assert(sizeof(ShPrim) == 48 && sizeof(ShPrimF) == 48, "primitive records are 48 bytes");
 
@@ -71,27 +71,37 @@ struct ShWork {
   uint64_t mask;         // ket components that are asked for
 };
 
+// Boys tables of one top degree L, row k around T_k = k/8, a_j = F_{L+j}(T_k) / j!: FP64 a_0..a_8,
+// and for the FP32 evaluations a_0..a_4 and e^-T_k as two floats and a_5..a_8 (rows of 20 floats:
+// 16-byte loads of different rows spread over the banks).
+constexpr int SH_BOYS_K = 289, SH_BOYS_ROW = 20;
+struct alignas(16) ShBoys {
+  float f[SH_BOYS_K][SH_BOYS_ROW];
+  double a[SH_BOYS_K][9];
+};
+static_assert(sizeof(ShBoys) % 16 == 0 && sizeof(float) * SH_BOYS_K * SH_BOYS_ROW % 16 == 0 && SH_BOYS_ROW % 4 == 0,
+              "the FP32 tables are copied and read as float4");
+
 struct ShArgs {
   const ShPair* pair;
   const int* cnt;
   const ShPrim* prim;
   const ShPrimF* primf;
   const double* E;
-  const float* Ef;
+  const float2* E2;      // the same as two floats
+  const double* scale;   // power of two of each pair's w in primf
+  const ShBoys* boys;    // [SH_MAXL + 1]
   const ShStruct* st;
   const ShWork* work;
   const int* cta;        // work entry of each CTA of the chunk
   int cta0;              // first CTA of this launch in it
   double* partial;
-  double eps, eps32;
+  double eps, eps32, eps_df;
   int diag;              // 1: (P|Q) of a pair with itself, Q <= P, diagonal elements only
 };
 
-// dynamic shared memory of a launch: Hermite rows, accumulators, outputs
 constexpr int SH_SMEM_MAX = 200 * 1024;
-constexpr int sh_threads(int L) { return L >= 6 ? 64 : 128; }
-constexpr int sh_row(int L) { return sh_nherm(L) | 1; }  // odd row length: conflict-free columns
 
-cudaError_t launch_shell_eri(int L, int ncta, int max_no, int max_ni, cudaStream_t st, const ShArgs& A);
+cudaError_t launch_shell_eri(int L, int ncta, int max_no, int max_ni, int max_col, cudaStream_t st, const ShArgs& A);
 
 }  // namespace ss

@@ -5,31 +5,29 @@
 // is a sum of Hermite Gaussians with coefficients E, and the repulsion of two Hermite Gaussians is
 // R_{t+tau}, a derivative of the Boys function.
 //
-// What bounds it: the FP64 pipe (2 fused multiply-adds per clock and SM).  A warp's FP64
-// instruction occupies it for 16 clocks, so shared-memory operands and index arithmetic are free
-// and only the number of FP64 operations counts.  Per primitive quartet of four shells it takes
-// one Boys evaluation, the Hermite recursion, and one multiply-add per (bra Hermite function, ket
-// Hermite coefficient); the bra's coefficients are applied once per bra primitive, after the sum
-// over the ket's.
-//
 // One CTA per (shell quartet, bra slice).  The (bra, ket) primitive items of the slice are
-// numbered bra-major and taken in batches of one item per thread:
-//  1. each thread forms the Hermite integrals of its item in registers and puts them in shared
+// numbered bra-major and taken in batches:
+//  1. each thread forms the Hermite integrals of an item in registers and puts them in shared
 //     memory (one row per item);
 //  2. for each bra primitive of the batch, thread <-> (group, bra Hermite function, ket component)
 //     sums R_{t+tau} E_tau over its group's items; when the bra primitive is done, its coefficients
 //     contract the sums into the output block.
-// Tiers as in eri_kernel.cuh: primitives are sorted by their Schwarz factor relative to the
-// function pairs' diagonals (the largest over the components), so the kept kets of a bra
-// primitive are a prefix, and those evaluated in FP64 a shorter one; each member of the shell
-// quartet therefore has at least the tier that it would have alone.
+// Tiers: primitives are sorted by their Schwarz factor relative to the function pairs' diagonals
+// (the largest over the components), so the kept kets of a bra primitive are a prefix, and those of
+// each tier a range of it; each member of the shell quartet has at least the tier that it would
+// have alone.  By the bound S_P S_Q of an item:
+//   >= eps_df   FP64
+//   >= eps32    two floats (df32.cuh, 48 bits): FP64 issues 2 lanes per clock and SM, FP32 128
+//   >= eps      FP32
 // The decomposition (slices, batches, groups) depends on the shell quartet alone, so a value does
 // not depend on which other quartets were asked for.
 #pragma once
 #include <math.h>
 
+#include <utility>
+
 #include "boys.cuh"
-#include "boys_grid.cuh"
+#include "df32.cuh"
 #include "shell.cuh"
 
 namespace ss {
@@ -37,24 +35,24 @@ namespace ss {
 constexpr double SH_PI_5_2 = 34.9868366552;  // src/general_primitive_integral.F90:25
 constexpr int SH_MAXSLICE = 16;              // bra primitives of a slice
 
-// F_0..F_L(T), T >= 0.  T <= 36: F_L from the Taylor series around T_k = k/8 (row k of tab: F_{L+j}(T_k) / j!,
-// j < 9), then F_n = (2T F_{n+1} + e^-T) / (2n+1), stable; above, erf(sqrt T) = 1 and the upward
+// F_0..F_L(T), T >= 0.  T <= 36: F_L from the Taylor series around T_k = k/8 (nine terms, |T - T_k|
+// <= 1/16), then F_n = (2T F_{n+1} + e^-T) / (2n+1), stable; above, erf(sqrt T) = 1 and the upward
 // recursion is stable.
 template <int L>
-__device__ __forceinline__ void boys_shell(double T, double (&F)[L + 1], const double* tab, const double* e2) {
+__device__ __forceinline__ void boys_shell(double T, double (&F)[L + 1], const ShBoys* __restrict__ tab) {
   const int64_t tb = bits_of(T);
   if (tb <= 0x4042000000000000LL) {  // T <= 36
     const double t = fma(T, 8.0, RINT_SHIFT);
     // at most 288 for T <= 36; held there so that no value of T can index past the table
-    const int k = (int)min((uint32_t)bits_of(t), (uint32_t)(BOYS_GRID_K - 1));
+    const int k = (int)min((uint32_t)bits_of(t), (uint32_t)(SH_BOYS_K - 1));
     const double x = fma(t - RINT_SHIFT, 0.125, -T);  // T_k - T, exact
-    const double* a = tab + k * 9;
+    const double* a = tab->a[k];
     double s = a[8];
 #pragma unroll
     for (int j = 7; j >= 0; j--) s = fma(s, x, a[j]);
     F[L] = s;
     if (L > 0) {
-      const double e = exp_neg(-T, e2), T2 = T + T;
+      const double e = exp_neg(-T, exp2_32_tab), T2 = T + T;
 #pragma unroll
       for (int n = L - 1; n >= 0; n--) F[n] = fma(T2, F[n + 1], e) * (1.0 / (2 * n + 1));
     }
@@ -63,14 +61,70 @@ __device__ __forceinline__ void boys_shell(double T, double (&F)[L + 1], const d
     F[0] = 0.88622692545275801365 * u;  // sqrt(pi)/2
     if (L > 0) {
       const double h = 0.5 * u * u;
-      const double e = (tb > 0x4054000000000000LL) ? 0.0 : exp_neg(-T, e2);  // T > 80
+      const double e = (tb > 0x4054000000000000LL) ? 0.0 : exp_neg(-T, exp2_32_tab);  // T > 80
 #pragma unroll
       for (int n = 1; n <= L; n++) F[n] = fma((double)(2 * n - 1), F[n - 1], -e) * h;
     }
   }
 }
 
-// FP32: as boys32 (boys.cuh), table columns F_{L+j}(T_k) / j!, j < 6
+// Two floats: the terms of degree >= 5 of the series in FP32 (they are below 1e-8 of F_L); above
+// T = 36, e^-T is below 3e-16 and taken in FP32.
+template <int L>
+__device__ __forceinline__ void boys_shell(df T, df (&F)[L + 1], const float* tab) {
+  if (T.h <= 36.f) {
+    const int k = min((int)fmaf(T.h, 8.f, 0.5f), SH_BOYS_K - 1);
+    const df x = df_fast_sum(__fsub_rn((float)k * 0.125f, T.h), -T.l);  // T_k - T
+    const float4* row = reinterpret_cast<const float4*>(tab + k * SH_BOYS_ROW);
+    const float4 r0 = row[0], r1 = row[1], r2 = row[2], r3 = row[3];
+    float t = fmaf(r3.w, x.h, r3.z);
+    t = fmaf(t, x.h, r3.y);
+    t = fmaf(t, x.h, r3.x);
+    df s = df_fast_sum(r2.x, __fmul_rn(t, x.h));
+    s.l = __fadd_rn(s.l, r2.y);
+    s = df_fma_fast(s, x, df{r1.z, r1.w});
+    s = df_fma_fast(s, x, df{r1.x, r1.y});
+    s = df_fma_fast(s, x, df{r0.z, r0.w});
+    s = df_fma_fast(s, x, df{r0.x, r0.y});
+    F[L] = s;
+    if (L > 0) {
+      // e^-T = e^-T_k e^x, |x| <= 1/16: degrees 5..9 in FP32
+      float q = fmaf(x.h, 1.f / 362880, 1.f / 40320);
+      q = fmaf(q, x.h, 1.f / 5040);
+      q = fmaf(q, x.h, 1.f / 720);
+      q = fmaf(q, x.h, 1.f / 120);
+      df e = df_fast_sum(1.f / 24, __fmul_rn(q, x.h));
+      e.l = __fadd_rn(e.l, (float)(1.0 / 24 - (double)(1.f / 24)));
+      e = df_fma_fast(e, x, df{1.f / 6, (float)(1.0 / 6 - (double)(1.f / 6))});
+      e = df_fma_fast(e, x, df{0.5f, 0.f});
+      e = df_fma_fast(e, x, df{1.f, 0.f});
+      e = df_fma_fast(e, x, df{1.f, 0.f});
+      e = df_mul(e, df{r2.z, r2.w});
+      const df T2 = df_scale(T, 2.f);
+#pragma unroll
+      for (int n = L - 1; n >= 0; n--) {
+        const df v = df_fma(T2, F[n + 1], e);
+        const float ih = 1.f / (2 * n + 1);
+        F[n] = n == 0 ? v : df_mul(v, df{ih, (float)(1.0 / (2 * n + 1) - (double)ih)});
+      }
+    }
+  } else {
+    const df u = df_rsqrt(T);
+    F[0] = df_mul(u, df{0.886226925f, (float)(0.88622692545275801365 - (double)0.886226925f)});
+    if (L > 0) {
+      const df h = df_scale(df_mul(u, u), 0.5f);
+      const float e = T.h > 80.f ? 0.f : expf(-T.h);
+#pragma unroll
+      for (int n = 1; n <= L; n++) {
+        df v = df_mulf(F[n - 1], (float)(2 * n - 1));
+        v = df_fast_sum(v.h, __fsub_rn(v.l, e));
+        F[n] = df_mul(v, h);
+      }
+    }
+  }
+}
+
+// FP32, the same series to degree 5; above T = 30 the asymptotic F_0
 template <int L>
 __device__ __forceinline__ void boys_shell(float T, float (&F)[L + 1], const float* tab) {
   if (T >= 30.f) {
@@ -83,10 +137,10 @@ __device__ __forceinline__ void boys_shell(float T, float (&F)[L + 1], const flo
   }
   const int k = (int)(T * 8.f + 0.5f);
   const float x = (float)k * 0.125f - T;
-  const float* a = tab + k * 6;
-  float s = a[5];
+  const float* a = tab + k * SH_BOYS_ROW;
+  float s = a[12];
 #pragma unroll
-  for (int j = 4; j >= 0; j--) s = fmaf(s, x, a[j]);
+  for (int j = 4; j >= 0; j--) s = fmaf(s, x, a[2 * j]);
   F[L] = s;
   if (L > 0) {
     const float e = expf(-T);
@@ -95,64 +149,99 @@ __device__ __forceinline__ void boys_shell(float T, float (&F)[L + 1], const flo
   }
 }
 
+// the operations of the recursion in each type
+__device__ __forceinline__ double r_mul(double a, double b) { return a * b; }
+__device__ __forceinline__ float r_mul(float a, float b) { return a * b; }
+__device__ __forceinline__ df r_mul(df a, df b) { return df_mul(a, b); }
+__device__ __forceinline__ double r_fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float r_fma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ df r_fma(df a, df b, df c) { return df_fma(a, b, c); }
+__device__ __forceinline__ double r_times(double a, int n) { return n == 1 ? a : (double)n * a; }
+__device__ __forceinline__ float r_times(float a, int n) { return n == 1 ? a : (float)n * a; }
+__device__ __forceinline__ df r_times(df a, int n) {
+  return n == 1 ? a : ((n & (n - 1)) == 0 ? df_scale(a, (float)n) : df_mulf(a, (float)n));
+}
+
+// (t, u, v) of a Hermite index
+struct ShDeg {
+  int t, u, v;
+};
+__host__ __device__ constexpr ShDeg sh_degs(int i) {
+  int d = 0;
+  while (sh_nherm(d) <= i) d++;
+  const int r = d ? i - sh_nherm(d - 1) : 0;
+  int w = 0;
+  while ((w + 1) * (w + 2) / 2 <= r) w++;
+  const int v = r - w * (w + 1) / 2;
+  return ShDeg{d - w, w - v, v};
+}
+
+// One entry of the recursion below, all indices at compile time.
+template <int I, typename Real, int N>
+__device__ __forceinline__ void hermite_step(Real X, Real Y, Real Z, Real (&R)[N]) {
+  constexpr ShDeg h = sh_degs(I);
+  constexpr int big = 99;
+  constexpr int at = h.t ? h.t : big, au = h.u ? h.u : big, av = h.v ? h.v : big;
+  constexpr int ax = (at <= au && at <= av) ? 0 : (au <= av ? 1 : 2);
+  constexpr int n = ax == 0 ? h.t : (ax == 1 ? h.u : h.v);
+  constexpr int i1 = sh_hidx(h.t - (ax == 0), h.u - (ax == 1), h.v - (ax == 2));
+  const Real x = ax == 0 ? X : (ax == 1 ? Y : Z);
+  if constexpr (n == 1) {
+    R[I] = r_mul(x, R[i1]);
+  } else {
+    constexpr int i2 = sh_hidx(h.t - 2 * (ax == 0), h.u - 2 * (ax == 1), h.v - 2 * (ax == 2));
+    R[I] = r_fma(x, R[i1], r_times(R[i2], n - 1));
+  }
+}
+template <typename Real, int N, int... I>
+__device__ __forceinline__ void hermite_level(Real X, Real Y, Real Z, Real (&R)[N], std::integer_sequence<int, I...>) {
+  (hermite_step<(int)sizeof...(I) - I>(X, Y, Z, R), ...);  // indices sizeof...(I) .. 1
+}
+
 // Hermite integrals of degree <= L in place: level m holds R^(m)_tuv, t + u + v <= L - m, and
 // R^(m)_{t+1} = X R^(m+1)_t + t R^(m+1)_{t-1} (the axis with the smallest degree is lowered: a
-// degree of one needs no second term).  Level m overwrites level m + 1 from the highest degree
+// degree of one needs no second term).  Level m overwrites level m + 1 from the highest index
 // down, so each entry reads values that are still of level m + 1.  base[m] = R^(m)_000.
-template <int L, typename Real>
-__device__ __forceinline__ void hermite_recursion(Real X, Real Y, Real Z, const Real (&base)[L + 1],
-                                                  Real (&R)[sh_nherm(L)]) {
-  R[0] = base[L];
-#pragma unroll
-  for (int mm = 0; mm < L; mm++) {  // level m = L - 1 - mm
-#pragma unroll
-    for (int dd = 0; dd <= mm; dd++) {
-      const int d = mm + 1 - dd;
-#pragma unroll
-      for (int w = 0; w <= d; w++)
-#pragma unroll
-        for (int v = 0; v <= w; v++) {
-          const int t = d - w, u = w - v;
-          const int big = 99;
-          const int at = t ? t : big, au = u ? u : big, av = v ? v : big;
-          const int ax = (at <= au && at <= av) ? 0 : (au <= av ? 1 : 2);
-          const int n = ax == 0 ? t : (ax == 1 ? u : v);
-          const Real x = ax == 0 ? X : (ax == 1 ? Y : Z);
-          const int i1 = sh_hidx(t - (ax == 0), u - (ax == 1), v - (ax == 2));
-          if (n == 1) {
-            R[sh_hidx(t, u, v)] = x * R[i1];
-          } else {
-            const int i2 = sh_hidx(t - 2 * (ax == 0), u - 2 * (ax == 1), v - 2 * (ax == 2));
-            const Real b = n == 2 ? R[i2] : (Real)(n - 1) * R[i2];
-            R[sh_hidx(t, u, v)] = fma(x, R[i1], b);
-          }
-        }
-    }
-    R[0] = base[L - 1 - mm];
+template <int L, int M, typename Real>
+__device__ __forceinline__ void hermite_levels(Real X, Real Y, Real Z, const Real (&base)[L + 1],
+                                               Real (&R)[sh_nherm(L)]) {
+  if constexpr (M >= 0) {
+    hermite_level(X, Y, Z, R, std::make_integer_sequence<int, sh_nherm(L - M) - 1>());
+    R[0] = base[M];
+    hermite_levels<L, M - 1>(X, Y, Z, base, R);
   }
 }
 
 __host__ __device__ constexpr int sh_dfact(int n) { return n <= 1 ? 1 : n * sh_dfact(n - 2); }  // n!!
 
+template <typename Real, int N, int... I>
+__device__ __forceinline__ void put_row(const Real (&R)[N], Real* row, std::integer_sequence<int, I...>) {
+  ((row[I] = R[I]), ...);
+}
 template <int L, typename Real>
 __device__ __forceinline__ void store_row(Real X, Real Y, Real Z, const Real (&base)[L + 1], Real* row) {
   Real R[sh_nherm(L)];
-  hermite_recursion<L, Real>(X, Y, Z, base, R);
-#pragma unroll
-  for (int i = 0; i < sh_nherm(L); i++) row[i] = R[i];
+  R[0] = base[L];
+  hermite_levels<L, L - 1>(X, Y, Z, base, R);
+  put_row(R, row, std::make_integer_sequence<int, sh_nherm(L)>());
 }
 
 // all four shells on one centre: only the even degrees, R_{2a 2b 2c} = (2a-1)!! (2b-1)!! (2c-1)!! base[a+b+c]
+template <int I, typename Real, int N>
+__device__ __forceinline__ void put_1c(const Real (&base)[N], Real* row) {
+  constexpr ShDeg h = sh_degs(I);
+  if constexpr (!((h.t | h.u | h.v) & 1)) {
+    constexpr int c = sh_dfact(h.t - 1) * sh_dfact(h.u - 1) * sh_dfact(h.v - 1);
+    row[I] = r_times(base[(h.t + h.u + h.v) / 2], c);
+  }
+}
+template <typename Real, int N, int... I>
+__device__ __forceinline__ void put_row_1c(const Real (&base)[N], Real* row, std::integer_sequence<int, I...>) {
+  (put_1c<I>(base, row), ...);
+}
 template <int L, typename Real>
 __device__ __forceinline__ void store_row_1c(const Real (&base)[L + 1], Real* row) {
-#pragma unroll
-  for (int a = 0; 2 * a <= L; a++)
-#pragma unroll
-    for (int b = 0; 2 * (a + b) <= L; b++)
-#pragma unroll
-      for (int c = 0; 2 * (a + b + c) <= L; c++)
-        row[sh_hidx(2 * a, 2 * b, 2 * c)] =
-            base[(a + b + c) % (L + 1)] * (Real)(sh_dfact(2 * a - 1) * sh_dfact(2 * b - 1) * sh_dfact(2 * c - 1));
+  put_row_1c(base, row, std::make_integer_sequence<int, sh_nherm(L)>());
 }
 
 __constant__ uint32_t sh_hermite[SH_MAXH] = {
@@ -166,34 +255,35 @@ __constant__ uint32_t sh_hermite[SH_MAXH] = {
 };
 __device__ __forceinline__ int sh_degree(uint32_t h) { return (int)((h & 255) + ((h >> 8) & 255) + (h >> 16)); }
 
+// Threads of a CTA and items of a batch: rows of 8 bytes x Hermite integrals bound the batch from
+// degree 5 on, where the sums of step 2 are most of the work.
 template <int L>
-struct ShSmem {
-  static constexpr int NT = sh_threads(L);
-  static constexpr int ROW = sh_row(L);
-  static size_t bytes(int max_no, int max_ni) {
-    return sizeof(double) * (BOYS_GRID_K * 9 + 32 + (size_t)NT * ROW + (max_no > NT ? max_no : NT) + max_ni) +
-           sizeof(float) * BOYS32_K * 6 + sizeof(int) * NT;
+struct ShDim {
+  static constexpr int NT = 128;
+  static constexpr int NB = L >= 5 ? 64 : 128;
+  static constexpr int MINB = L >= 7 ? 2 : L >= 4 ? 3 : 4;  // CTAs per SM the registers must allow
+  static constexpr int ROW = sh_nherm(L) | 1;  // odd: a column over the items meets no bank twice
+  static size_t bytes(int max_no, int max_ni, int max_col) {
+    return sizeof(float) * SH_BOYS_K * SH_BOYS_ROW +
+           sizeof(double) * ((size_t)NB * ROW + (max_no > NT ? max_no : NT) + max_ni) + ((size_t)max_col + 15) / 16 * 16;
   }
 };
 
 template <int L>
-__global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int max_no, int max_ni) {
-  constexpr int NT = ShSmem<L>::NT;
-  constexpr int ROW = ShSmem<L>::ROW;
-  extern __shared__ double sh_raw[];
-  double* s_boys = sh_raw;                       // [BOYS_GRID_K][9]
-  double* s_e2 = s_boys + BOYS_GRID_K * 9;       // [32]
-  double* s_R = s_e2 + 32;                       // [NT][ROW] (float rows in the FP32 pass)
-  double* s_acc = s_R + (size_t)NT * ROW;        // [groups][bra Hermite][ket component]
+__global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel(ShArgs A, int max_no, int max_ni, int max_col) {
+  constexpr int NT = ShDim<L>::NT, NB = ShDim<L>::NB, ROW = ShDim<L>::ROW;
+  extern __shared__ float4 sh_raw[];
+  float* s_boys = reinterpret_cast<float*>(sh_raw);                          // [SH_BOYS_K][SH_BOYS_ROW]
+  double* s_R = reinterpret_cast<double*>(s_boys + SH_BOYS_K * SH_BOYS_ROW);  // [NB][ROW]: double, df or float
+  double* s_acc = s_R + (size_t)NB * ROW;         // [group][bra Hermite][ket component]: double or df
   double* s_out = s_acc + (max_no > NT ? max_no : NT);
-  float* s_boys32 = reinterpret_cast<float*>(s_out + max_ni);  // [BOYS32_K][6]
-  int* s_q = reinterpret_cast<int*>(s_boys32 + BOYS32_K * 6);  // ket primitive of each item
-  __shared__ int s_scan[2][SH_MAXSLICE + 1], s_c64[SH_MAXSLICE], s_p[SH_MAXSLICE];
+  uint8_t* s_col = reinterpret_cast<uint8_t*>(s_out + max_ni);  // [ket term][bra Hermite]: column of t + tau
+  __shared__ int s_scan[3][SH_MAXSLICE + 1], s_first[3][SH_MAXSLICE], s_p[SH_MAXSLICE];
   const int tid = threadIdx.x;
   {  // the launch's dynamic shared memory must hold this carve-up: checked, not assumed
     uint32_t dyn;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-    if (reinterpret_cast<char*>(s_q + NT) - reinterpret_cast<char*>(sh_raw) > (ptrdiff_t)dyn) return;  // block-uniform
+    if (reinterpret_cast<char*>(s_col + max_col) - reinterpret_cast<char*>(sh_raw) > (ptrdiff_t)dyn) return;
   }
 
   const ShWork W = A.work[A.cta[A.cta0 + blockIdx.x]];
@@ -204,41 +294,32 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
   const ShPrim* ket = A.prim + K.prim_off;
   const ShStruct& SB = A.st[B.st];
   const ShStruct& SK = A.st[K.st];
+  const ShBoys* boys = A.boys + L;
   const bool diag = A.diag != 0;
   const bool onec = B.onec && K.onec && bra[0].P[0] == ket[0].P[0] && bra[0].P[1] == ket[0].P[1] &&
                     bra[0].P[2] == ket[0].P[2];
-  const int H = sh_nherm(B.d), nf = K.ncomp, NO = H * nf, NI = B.ncomp * nf;
+  const int H = sh_nherm(B.d), nf = K.ncomp, NO = H * nf, NI = B.ncomp * nf, nterm = K.nterm;
   const uint64_t mask = W.mask;
-  if (NO > (max_no > NT ? max_no : NT) || NI > max_ni || B.d + K.d != L) return;  // block-uniform
+  if (NO > (max_no > NT ? max_no : NT) || NI > max_ni || H * nterm > max_col || B.d + K.d != L) return;  // uniform
 
-  for (int i = tid; i < BOYS_GRID_K * 9; i += NT) {
-    const int k = i / 9, j = i - 9 * k;
-    double f = boys_grid_tab[k * BOYS_GRID_N + L + j];
-    const double inv[9] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320};
-    double s = 1.0;
-#pragma unroll
-    for (int t = 0; t < 9; t++) s = j == t ? inv[t] : s;
-    s_boys[i] = f * s;
+  if (!diag) {
+    const float4* src = reinterpret_cast<const float4*>(boys->f);
+    for (int i = tid; i < SH_BOYS_K * SH_BOYS_ROW / 4; i += NT) sh_raw[i] = src[i];
   }
-  for (int i = tid; i < 32; i += NT) s_e2[i] = exp2_32_tab[i];
-  for (int i = tid; i < BOYS32_K * 6; i += NT) {
-    const int k = i / 6, j = i - 6 * k;
-    const float inv[6] = {1.f, 1.f, 0.5f, 1.f / 6, 1.f / 24, 1.f / 120};
-    float s = 1.f;
-#pragma unroll
-    for (int t = 0; t < 6; t++) s = j == t ? inv[t] : s;
-    s_boys32[i] = boys32_tab[k * BOYS32_N + L + j] * s;
+  for (int i = tid; i < H * nterm; i += NT) {
+    const int x = i / H;
+    s_col[i] = (uint8_t)sh_pack_idx(SK.term[x] + sh_hermite[i - x * H]);
   }
   for (int i = tid; i < NI; i += NT) s_out[i] = 0.0;
 
-  // the slice's bra primitives (slice, slice + split, ...) and their ket prefixes
+  // the slice's bra primitives (slice, slice + split, ...) and their ket ranges
   int ns = 0;
   if (slice < nb) ns = min(SH_MAXSLICE, (nb - slice + W.split - 1) / W.split);
   if (tid < SH_MAXSLICE) {
     const int p = slice + tid * W.split;
-    int c = 0, c64 = 0;
+    int c = 0, cd = 0, cf = 0;  // ranges [0, cd) FP64, [cd, cf) two floats, [cf, c) FP32
     if (tid < ns) {
-      c = c64 = diag ? p + 1 : nk;
+      c = cd = cf = diag ? p + 1 : nk;
       if (!diag && A.eps > 0.0) {
         const double sb = bra[p].S;
         auto first_below = [&](double thr) {  // first ket with sb * S < thr
@@ -250,68 +331,49 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
           return lo;
         };
         c = first_below(A.eps);
-        c64 = A.eps32 > A.eps ? first_below(A.eps32) : c;
+        cd = cf = c;
+        if (A.eps32 > A.eps) {
+          cf = first_below(A.eps32);
+          cd = first_below(A.eps_df);
+        }
       }
       s_p[tid] = p;
     }
-    s_c64[tid] = c64;
-    s_scan[0][tid + 1] = c64;
-    s_scan[1][tid + 1] = c - c64;
+    s_first[0][tid] = 0;
+    s_first[1][tid] = cd;
+    s_first[2][tid] = cf;
+    s_scan[0][tid + 1] = cd;
+    s_scan[1][tid + 1] = cf - cd;
+    s_scan[2][tid + 1] = c - cf;
   }
   __syncthreads();
-  if (tid < 2) {
+  if (tid < 3) {
     s_scan[tid][0] = 0;
     for (int j = 0; j < SH_MAXSLICE; j++) s_scan[tid][j + 1] += s_scan[tid][j];
   }
-  // this thread's place in step 2 when a segment's outputs fit the CTA
+  // this thread's place in step 2 when a bra primitive's sums fit the CTA
   const int G = NO < NT ? NT / NO : 1;
   const int my_g = NO < NT ? tid / NO : 0;
   const int my_o = NO < NT ? tid - my_g * NO : tid;
   for (int o = tid; o < (NO > NT ? NO : NT); o += NT) s_acc[o] = 0.0;
+  const double scale = diag ? 1.0 : A.scale[W.bra] * A.scale[W.ket];
   __syncthreads();
 
-  // sums of the bra primitive in slot j are complete: contract with its coefficients
-  auto flush = [&](int j, float kx) {
-    __syncthreads();
-    for (int o = tid; o < NO; o += NT) {
-      double v = s_acc[o];
-      for (int g = 1; g < G; g++) {
-        v += s_acc[o + g * NO];
-        s_acc[o + g * NO] = 0.0;
-      }
-      if (kx != 1.f) {  // undo the FP32 pass's degree scaling (powers of two: exact)
-        for (int d = sh_degree(sh_hermite[o / nf]); d > 0; d--) v *= (double)kx;
-      }
-      s_acc[o] = v;
-    }
-    __syncthreads();
-    const double* Eb = A.E + B.e_off + (size_t)s_p[j] * B.nterm;
-    for (int e = tid; e < NI; e += NT) {
-      const int a = e / nf, f = e - a * nf;
-      if (!((mask >> f) & 1)) continue;
-      double s = 0.0;
-      for (int x = SB.fs[a]; x < SB.fs[a + 1]; x++) s = fma(Eb[x], s_acc[sh_pack_idx(SB.term[x]) * nf + f], s);
-      s_out[e] += s;
-    }
-    __syncthreads();
-    for (int o = tid; o < NO; o += NT) s_acc[o] = 0.0;
-  };
-
-  for (int tier = 0; tier < 2; tier++) {
+  for (int tier = 0; tier < 3; tier++) {
     const int* scan = s_scan[tier];
     const int n = scan[SH_MAXSLICE];
-    for (int base = 0; base < n; base += NT) {
+    for (int base = 0; base < n; base += NB) {
+      const int top = min(base + NB, n);
       // ---- 1. one item per thread ----
-      const int item = base + tid;
-      if (item < n) {
+      for (int item = base + tid; item < top; item += NT) {
         int j = 0;
 #pragma unroll
         for (int s = SH_MAXSLICE / 2; s > 0; s >>= 1)
           if (scan[j + s] <= item) j += s;
         const int p = s_p[j];
-        const int q = item - scan[j] + (tier ? s_c64[j] : 0);
-        s_q[tid] = q;
+        const int q = item - scan[j] + s_first[tier][j];
         if (tier == 0) {
+          double* row = s_R + (item - base) * ROW;
           const ShPrim a = bra[p], b = ket[q];
           double pre = a.w * b.w;
           if (diag && q < p) pre = pre + pre;
@@ -320,7 +382,6 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
           const double alpha = a.p * b.p * (rs * rs);
           const double m2a = -2.0 * alpha;
           double bs[L + 1];
-          double* row = s_R + tid * ROW;
           if (onec) {
             bs[0] = pre;
             double pw = pre;
@@ -333,7 +394,7 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
           } else {
             const double X = a.P[0] - b.P[0], Y = a.P[1] - b.P[1], Z = a.P[2] - b.P[2];
             double F[L + 1];
-            boys_shell<L>(alpha * fma(X, X, fma(Y, Y, Z * Z)), F, s_boys, s_e2);
+            boys_shell<L>(alpha * fma(X, X, fma(Y, Y, Z * Z)), F, boys);
             double pw = pre;
 #pragma unroll
             for (int m = 0; m <= L; m++) {
@@ -342,19 +403,52 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
             }
             store_row<L, double>(X, Y, Z, bs, row);
           }
+          continue;
+        }
+        // two floats and FP32: degree n carries a factor kx^-n (kx ~ sqrt(2p) of the bra
+        // primitive), which keeps (2 alpha)^L of tight primitives inside the FP32 range
+        const ShPrimF a = A.primf[B.prim_off + p], b = A.primf[K.prim_off + q];
+        const float kx = a.kx, ik2 = 1.f / (kx * kx);
+        if (tier == 1) {
+          df* row = reinterpret_cast<df*>(s_R) + (item - base) * ROW;
+          const df pa{a.p[0], a.p[1]}, pb{b.p[0], b.p[1]};
+          const df rs = df_rsqrt(df_add(pa, pb));
+          const df pre = df_mul(df_mul(df{a.w[0], a.w[1]}, df{b.w[0], b.w[1]}), rs);
+          const df alpha = df_mul(df_mul(pa, rs), df_mul(pb, rs));
+          const df m2a = df_scale(alpha, -2.f * ik2);
+          df bs[L + 1];
+          if (onec) {
+            bs[0] = pre;
+            df pw = pre;
+#pragma unroll
+            for (int m = 1; m <= L; m++) {
+              const float ih = 1.f / (2 * m + 1);
+              pw = df_mul(pw, m2a);
+              bs[m] = df_mul(pw, df{ih, (float)(1.0 / (2 * m + 1) - (double)ih)});
+            }
+            store_row_1c<L, df>(bs, row);
+          } else {
+            df X = df_sub(df{a.ph[0], a.pl[0]}, df{b.ph[0], b.pl[0]});
+            df Y = df_sub(df{a.ph[1], a.pl[1]}, df{b.ph[1], b.pl[1]});
+            df Z = df_sub(df{a.ph[2], a.pl[2]}, df{b.ph[2], b.pl[2]});
+            df F[L + 1];
+            boys_shell<L>(df_renorm(df_mul(alpha, df_fma(X, X, df_fma(Y, Y, df_mul(Z, Z))))), F, s_boys);
+            df pw = pre;
+#pragma unroll
+            for (int m = 0; m <= L; m++) {
+              bs[m] = df_mul(pw, F[m]);
+              if (m < L) pw = df_mul(pw, m2a);
+            }
+            store_row<L, df>(df_scale(X, kx), df_scale(Y, kx), df_scale(Z, kx), bs, row);
+          }
         } else {
-          // FP32: degree n carries a factor kx^-n (kx ~ sqrt(2p) of the bra primitive), which
-          // keeps (2 alpha)^L of tight primitives inside the FP32 range
-          const ShPrimF a = A.primf[B.prim_off + p], b = A.primf[K.prim_off + q];
-          const float kx = H == 1 ? 1.f : a.kx;
-          const float ik = 1.f / kx;
-          float pre = a.w * b.w;
-          const float rs = rsqrtf(a.p + b.p);
+          float* row = reinterpret_cast<float*>(s_R) + (item - base) * ROW;
+          float pre = a.w[0] * b.w[0];
+          const float rs = rsqrtf(a.p[0] + b.p[0]);
           pre *= rs;
-          const float alpha = (a.p * rs) * (b.p * rs);
-          const float m2a = -2.f * (alpha * ik * ik);
+          const float alpha = (a.p[0] * rs) * (b.p[0] * rs);
+          const float m2a = -2.f * (alpha * ik2);
           float bs[L + 1];
-          float* row = reinterpret_cast<float*>(s_R) + tid * ROW;
           if (onec) {
             bs[0] = pre;
             float pw = pre;
@@ -369,7 +463,7 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
             const float Y = (a.ph[1] - b.ph[1]) + (a.pl[1] - b.pl[1]);
             const float Z = (a.ph[2] - b.ph[2]) + (a.pl[2] - b.pl[2]);
             float F[L + 1];
-            boys_shell<L>(alpha * fmaf(X, X, fmaf(Y, Y, Z * Z)), F, s_boys32);
+            boys_shell<L>(alpha * fmaf(X, X, fmaf(Y, Y, Z * Z)), F, s_boys);
             float pw = pre;
 #pragma unroll
             for (int m = 0; m <= L; m++) {
@@ -381,8 +475,7 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
         }
       }
       __syncthreads();
-      // ---- 2. segments of the batch: runs of one bra primitive (an s-type bra needs none) ----
-      const int top = min(base + NT, n);
+      // ---- 2. segments of the batch: runs of one bra primitive ----
       int j = 0;
 #pragma unroll
       for (int s = SH_MAXSLICE / 2; s > 0; s >>= 1)
@@ -390,53 +483,107 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
       int lo = base;
       while (lo < top) {
         while (scan[j + 1] <= lo) j++;
-        const int hi = H == 1 ? top : min(top, scan[j + 1]);
-        const float kx = (tier && H > 1) ? A.primf[B.prim_off + s_p[j]].kx : 1.f;
-        const int i0 = lo - base, i1 = hi - base;
+        // with an s-type bra the FP64 sums need no contraction and no segments
+        const int hi = (H == 1 && tier == 0) ? top : min(top, scan[j + 1]);
+        const float kx = tier ? A.primf[B.prim_off + s_p[j]].kx : 1.f;
+        const int i0 = lo - base + my_g, i1 = hi - base;
+        const int q0 = lo - scan[j] + s_first[tier][j] + my_g;  // ket of the thread's first item
         for (int o = my_o; o < NO && my_g < G; o += NT) {
           const int t = o / nf, f = o - t * nf;
           if ((mask >> f) & 1) {
             const uint32_t ht = sh_hermite[t];
-            double acc = 0.0;
-            for (int x = SK.fs[f]; x < SK.fs[f + 1]; x++) {
-              const uint32_t tau = SK.term[x];
-              const uint32_t tt = ht + tau;
-              if (onec && (tt & 0x010101u)) continue;  // odd degrees vanish on one centre
-              const int col = sh_pack_idx(tt);
-              const int dt = sh_degree(tau);
-              if (tier == 0) {
-                const double* Ek = A.E + K.e_off + x;
-                const double* Rc = s_R + col;
+            const int x1 = SK.fs[f + 1];
+            if (tier == 0) {
+              double acc = 0.0;
+              for (int x = SK.fs[f]; x < x1; x++) {
+                const uint32_t tau = SK.term[x];
+                if (onec && ((ht + tau) & 0x010101u)) continue;  // odd degrees vanish on one centre
+                const double* Rc = s_R + s_col[x * H + t];
                 double s = 0.0;
+                if (H == 1) {  // items of several bra primitives: the kets are not consecutive
+                  int jj = j;
+                  for (int i = i0; i < i1; i += G) {
+                    while (scan[jj + 1] <= base + i) jj++;
+                    const int q = base + i - scan[jj] + s_first[0][jj];
+                    s = fma(Rc[i * ROW], A.E[K.e_off + (size_t)q * nterm + x], s);
+                  }
+                } else {
+                  const double* Ek = A.E + K.e_off + (size_t)q0 * nterm + x;
 #pragma unroll 4
-                for (int i = i0 + my_g; i < i1; i += G) s = fma(Rc[i * ROW], Ek[(size_t)s_q[i] * K.nterm], s);
-                acc += (dt & 1) ? -s : s;
-              } else {
-                const float* Ek = A.Ef + K.e_off + x;
-                const float* Rc = reinterpret_cast<const float*>(s_R) + col;
-                float s = 0.f;
-#pragma unroll 4
-                for (int i = i0 + my_g; i < i1; i += G) s = fmaf(Rc[i * ROW], Ek[(size_t)s_q[i] * K.nterm], s);
-                double v = (double)s;
-                for (int d = 0; d < dt; d++) v *= (double)kx;
-                acc += (dt & 1) ? -v : v;
+                  for (int i = i0; i < i1; i += G, Ek += (size_t)G * nterm) s = fma(Rc[i * ROW], *Ek, s);
+                }
+                acc += (sh_degree(tau) & 1) ? -s : s;
               }
+              s_acc[o + my_g * NO] += acc;
+            } else {
+              const float k2 = kx * kx;
+              df acc = reinterpret_cast<df*>(s_acc)[o + my_g * NO];
+              for (int x = SK.fs[f]; x < x1; x++) {
+                const uint32_t tau = SK.term[x];
+                if (onec && ((ht + tau) & 0x010101u)) continue;
+                const float2* Ek = A.E2 + K.e_off + (size_t)q0 * nterm + x;
+                const int col = s_col[x * H + t];
+                const int dt = sh_degree(tau);
+                // the ket's share of the degree scaling and its sign: exact
+                const float sc = ((dt & 1) ? -kx : 1.f) * ((dt & 2) ? k2 : 1.f) * ((dt & 4) ? k2 * k2 : 1.f);
+                if (tier == 1) {
+                  const df* Rc = reinterpret_cast<const df*>(s_R) + col;
+                  df s{0.f, 0.f};
+#pragma unroll 4
+                  for (int i = i0; i < i1; i += G, Ek += (size_t)G * nterm) {
+                    const float2 e = *Ek;
+                    s = df_fma(Rc[i * ROW], df{e.x, e.y}, s);
+                  }
+                  acc = df_add(acc, df_scale(s, sc));
+                } else {
+                  const float* Rc = reinterpret_cast<const float*>(s_R) + col;
+                  float s = 0.f;
+#pragma unroll 4
+                  for (int i = i0; i < i1; i += G, Ek += (size_t)G * nterm) s = fmaf(Rc[i * ROW], Ek->x, s);
+                  acc = df_add(acc, df{s * sc, 0.f});
+                }
+              }
+              reinterpret_cast<df*>(s_acc)[o + my_g * NO] = df_renorm(acc);
             }
-            s_acc[o + my_g * NO] += acc;
           }
           if (NO < NT) break;
         }
-        if (H > 1 && hi == scan[j + 1]) flush(j, kx);
+        const bool done = H == 1 ? (base + NB >= n && hi == top) : hi == scan[j + 1];
+        if (done) {  // the sums of this bra primitive (s-type bra: of the tier) are complete
+          __syncthreads();
+          for (int o = tid; o < NO; o += NT) {
+            double v;
+            if (tier == 0) {
+              v = s_acc[o];
+              for (int g = 1; g < G; g++) v += s_acc[o + g * NO];
+            } else {
+              const df* acc = reinterpret_cast<const df*>(s_acc);
+              df sum = acc[o];
+              for (int g = 1; g < G; g++) sum = df_add(sum, acc[o + g * NO]);
+              v = df_to(sum) * scale;
+              // the bra's share of the degree scaling
+              for (int d = sh_degree(sh_hermite[o / nf]); d > 0; d--) v *= (double)kx;
+            }
+            for (int g = 1; g < G; g++) s_acc[o + g * NO] = 0.0;
+            s_acc[o] = v;
+          }
+          __syncthreads();
+          const double* Eb = A.E + B.e_off + (size_t)s_p[H == 1 ? 0 : j] * B.nterm;
+          for (int e = tid; e < NI; e += NT) {
+            const int a = e / nf, f = e - a * nf;
+            if (!((mask >> f) & 1) || (diag && a != f)) continue;
+            double s = 0.0;
+            for (int x = SB.fs[a]; x < SB.fs[a + 1]; x++) s = fma(Eb[x], s_acc[sh_pack_idx(SB.term[x]) * nf + f], s);
+            s_out[e] += s;
+          }
+          __syncthreads();
+          for (int o = tid; o < NO; o += NT) s_acc[o] = 0.0;
+        }
         lo = hi;
       }
       __syncthreads();
     }
   }
-  if (H == 1 && nb > 0) {
-    if (tid == 0) s_p[0] = 0;
-    flush(0, 1.f);
-  }
-  __syncthreads();
   if (diag) {
     for (int a = tid; a < nf; a += NT) A.partial[W.part + (int64_t)a * W.split + slice] = SH_PI_5_2 * s_out[a * nf + a];
   } else {
@@ -445,12 +592,12 @@ __global__ void __launch_bounds__(sh_threads(L)) shell_eri_kernel(ShArgs A, int 
 }
 
 template <int L>
-cudaError_t launch_shell_L(int ncta, int max_no, int max_ni, cudaStream_t st, const ShArgs& A) {
-  const size_t smem = ShSmem<L>::bytes(max_no, max_ni);
+cudaError_t launch_shell_L(int ncta, int max_no, int max_ni, int max_col, cudaStream_t st, const ShArgs& A) {
+  const size_t smem = ShDim<L>::bytes(max_no, max_ni, max_col);
   if (smem > SH_SMEM_MAX) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(shell_eri_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, SH_SMEM_MAX);
   if (e != cudaSuccess) return e;
-  shell_eri_kernel<L><<<ncta, ShSmem<L>::NT, smem, st>>>(A, max_no, max_ni);
+  shell_eri_kernel<L><<<ncta, ShDim<L>::NT, smem, st>>>(A, max_no, max_ni, max_col);
   return cudaGetLastError();
 }
 

@@ -2,7 +2,7 @@
 #include "shell_eri.cuh"
 
 namespace ss {
-cudaError_t launch_shell_2(int ncta, int max_no, int max_ni, cudaStream_t st, const ShArgs& A) {
-  return launch_shell_L<2>(ncta, max_no, max_ni, st, A);
+cudaError_t launch_shell_2(int ncta, int max_no, int max_ni, int max_col, cudaStream_t st, const ShArgs& A) {
+  return launch_shell_L<2>(ncta, max_no, max_ni, max_col, st, A);
 }
 }  // namespace ss

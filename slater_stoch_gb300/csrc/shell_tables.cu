@@ -7,10 +7,20 @@
 #include <unordered_map>
 #include <vector>
 
+#include "boys_grid.cuh"
 #include "shell_host.h"
 #include "ss_context.cuh"
 
 namespace ss {
+
+// A kept primitive quartet whose Schwarz bound is below this part of the shell quartet's (and above
+// the FP32 tier) is evaluated in two floats, the larger ones in FP64.  Measured error against plain
+// 64-bit values, largest over the integrals of a system relative to their Schwarz bounds (water 7
+// functions; O; O-H; H2O of 19 functions): all FP64 1.4e-15, 4.3e-15, 4.5e-15, 2.8e-15 with the
+// per-function kernels; here 1e-5: 1.2e-15, 2.4e-15, 1.9e-15, 2.8e-15; 1e-4: 1.9e-15, 2.2e-15,
+// 9.4e-15, 2.8e-15; 1e-3: 1.4e-14, 9.6e-15, 4.0e-14, 9.9e-15; all two-float: 2.5e-14 to 1.5e-13.
+// About a tenth of the FP64 work is left above 1e-5.
+constexpr double SH_DF_EPS = 1e-5;
 
 #define TRY(x)           \
   do {                   \
@@ -220,12 +230,15 @@ __global__ void shell_expand(const ShWork* __restrict__ work, int* __restrict__ 
 // largest over the components of sqrt((P_f|P_f) / (f|f)), (f|f) the contracted diagonal: then
 // |(P_f|Q_g)| <= S_P S_Q sqrt((f|f)(g|g)) for every pair of components.  A component without a
 // positive diagonal keeps all its primitives (factor 1e30).  Sorted by decreasing factor (ties:
-// the (m1, m2) order), with an FP32 copy of the records and coefficients.
+// the (m1, m2) order), with a two-float copy of the records and coefficients whose w is divided by
+// a power of two near the square root of the pair's largest diagonal, so that the FP32 evaluations
+// of distant (small) pairs stay inside the FP32 range.
 __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pairs, const ShStruct* __restrict__ st,
                                                   const int* __restrict__ cnt, const double* __restrict__ diag,
                                                   const ShPrim* __restrict__ prim, const double* __restrict__ E,
                                                   ShPrim* __restrict__ oprim, ShPrimF* __restrict__ oprimf,
-                                                  double* __restrict__ oE, float* __restrict__ oEf) {
+                                                  double* __restrict__ oE, float2* __restrict__ oE2,
+                                                  double* __restrict__ oscale) {
   __shared__ double s_key[1024];
   __shared__ int s_idx[1024];
   const ShPair P = pairs[blockIdx.x];
@@ -285,36 +298,65 @@ __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pai
       }
       __syncthreads();
     }
+  double dmax = 0.0;
+  for (int f = 0; f < S.ncomp; f++) dmax = fmax(dmax, diag[(size_t)blockIdx.x * SH_MAXCOMP + f]);
+  const int ex = dmax > 0.0 ? ilogb(dmax) / 2 : 0;
+  if (threadIdx.x == 0) oscale[blockIdx.x] = ldexp(1.0, ex);
   for (int t = threadIdx.x; t < m; t += blockDim.x) {
     ShPrim a = prim[P.prim_off + s_idx[t]];
     a.S = s_key[t];
     oprim[P.prim_off + t] = a;
+    auto two = [](double v, float* hi, float* lo) {
+      *hi = (float)v;
+      *lo = (float)(v - (double)*hi);
+    };
     ShPrimF g;
-    g.p = (float)a.p;
-    g.w = (float)a.w;
-    for (int ax = 0; ax < 3; ax++) {
-      g.ph[ax] = (float)a.P[ax];
-      g.pl[ax] = (float)(a.P[ax] - (double)g.ph[ax]);
-      g.pad[ax] = 0.f;
-    }
-    g.kx = exp2f(rintf(0.5f * log2f(2.f * g.p)));
+    two(a.p, &g.p[0], &g.p[1]);
+    two(ldexp(a.w, -ex), &g.w[0], &g.w[1]);
+    for (int ax = 0; ax < 3; ax++) two(a.P[ax], &g.ph[ax], &g.pl[ax]);
+    g.kx = exp2f(rintf(0.5f * log2f(2.f * g.p[0])));
+    g.pad = 0.f;
     oprimf[P.prim_off + t] = g;
   }
   for (int t = threadIdx.x; t < m * P.nterm; t += blockDim.x) {
     const int r = t / P.nterm, x = t - r * P.nterm;
     const double v = E[P.e_off + (size_t)s_idx[r] * P.nterm + x];
     oE[P.e_off + t] = v;
-    oEf[P.e_off + t] = (float)v;
+    const float hi = (float)v;
+    oE2[P.e_off + t] = make_float2(hi, (float)(v - (double)hi));
   }
 }
 
-#define SH_DECL(L) cudaError_t launch_shell_##L(int, int, int, cudaStream_t, const ShArgs&);
+// Boys tables of every top degree (ShBoys), from the grid F_n(T_k)
+__global__ void shell_boys(ShBoys* __restrict__ out) {
+  const int L = blockIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= SH_BOYS_K) return;
+  double fact = 1.0;
+  float* f = out[L].f[k];
+  for (int j = 0; j < 9; j++) {
+    if (j > 1) fact *= j;
+    const double a = boys_grid_tab[k * BOYS_GRID_N + L + j] / fact;
+    out[L].a[k][j] = a;
+    if (j < 5) {
+      f[2 * j] = (float)a;
+      f[2 * j + 1] = (float)(a - (double)(float)a);
+    } else {
+      f[12 + j - 5] = (float)a;
+    }
+  }
+  const double e = exp(-0.125 * k);
+  f[10] = (float)e;
+  f[11] = (float)(e - (double)(float)e);
+  for (int j = 16; j < SH_BOYS_ROW; j++) f[j] = 0.f;
+}
+
+#define SH_DECL(L) cudaError_t launch_shell_##L(int, int, int, int, cudaStream_t, const ShArgs&);
 SH_DECL(0) SH_DECL(1) SH_DECL(2) SH_DECL(3) SH_DECL(4) SH_DECL(5) SH_DECL(6) SH_DECL(7) SH_DECL(8)
 #undef SH_DECL
 
-cudaError_t launch_shell_eri(int L, int ncta, int max_no, int max_ni, cudaStream_t st, const ShArgs& A) {
+cudaError_t launch_shell_eri(int L, int ncta, int max_no, int max_ni, int max_col, cudaStream_t st, const ShArgs& A) {
   switch (L) {
-#define SH_CASE(l) case l: return launch_shell_##l(ncta, max_no, max_ni, st, A);
+#define SH_CASE(l) case l: return launch_shell_##l(ncta, max_no, max_ni, max_col, st, A);
     SH_CASE(0) SH_CASE(1) SH_CASE(2) SH_CASE(3) SH_CASE(4) SH_CASE(5) SH_CASE(6) SH_CASE(7) SH_CASE(8)
 #undef SH_CASE
   }
@@ -450,7 +492,7 @@ static int slices(const ShPair& b, const ShPair& k) {
 
 // Launch the work entries (grouped by total degree), in chunks whose partial sums fit the buffer,
 // and reduce each chunk's partial sums to elements.
-static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF* primf, const double* E, const float* Ef,
+static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF* primf, const double* E, const float2* E2,
                     bool diag, double eps, double eps32, double* elem) {
   const ShellBasis& T = c->shells;
   // partial sums in flight: enough for a whole mid-size system, and bounded
@@ -459,7 +501,7 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
   const int64_t cap_d = (int64_t)(cap / sizeof(double));
   // heaviest degrees first: their CTAs are the longest
   std::vector<ShWork> chunk;
-  struct Seg { int L, first, n, ncta, no, ni; };
+  struct Seg { int L, first, n, ncta, no, ni, col; };
   std::vector<Seg> segs;
   int64_t part = 0, most = 0;
   int ncta = 0;
@@ -482,10 +524,13 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
     A.prim = prim;
     A.primf = primf;
     A.E = E;
-    A.Ef = Ef;
+    A.E2 = E2;
+    A.scale = (const double*)c->pool["shell_scale"].ptr;
+    A.boys = (const ShBoys*)c->pool["shell_boys"].ptr;
     A.partial = (double*)dp;
     A.eps = eps;
     A.eps32 = eps32;
+    A.eps_df = SH_DF_EPS;
     A.diag = diag;
     int rc = SS_OK;
     for (size_t s = 0; s < segs.size() && !rc; s++) {
@@ -493,7 +538,7 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
       A.work = (const ShWork*)dw;
       A.cta = (const int*)dc;
       A.cta0 = chunk[g.first].cta0;
-      const cudaError_t e = launch_shell_eri(g.L, g.ncta, g.no, g.ni, c->eri_stream[s % ss_ctx::ERI_STREAMS], A);
+      const cudaError_t e = launch_shell_eri(g.L, g.ncta, g.no, g.ni, g.col, c->eri_stream[s % ss_ctx::ERI_STREAMS], A);
       if (e != cudaSuccess) {
         ss_set_cuda_error(e, "shell_eri_kernel launch", __FILE__, __LINE__);
         rc = SS_ERR_CUDA;
@@ -528,7 +573,7 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
         open = false;
       }
       if (!open) {
-        segs.push_back(Seg{L, (int)chunk.size(), 0, 0, 0, 0});
+        segs.push_back(Seg{L, (int)chunk.size(), 0, 0, 0, 0, 0});
         open = true;
       }
       Seg& g = segs.back();
@@ -539,6 +584,7 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
       g.ncta += w.split;
       g.no = std::max(g.no, sh_nherm(b.d) * k.ncomp);
       g.ni = std::max(g.ni, ni);
+      g.col = std::max(g.col, sh_nherm(b.d) * k.nterm);
       ncta += w.split;
       part += need;
     }
@@ -563,14 +609,22 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
   double *E2, *diag;
   ShPrim* prim2;
   ShPrimF* primf;
-  float* Ef;
+  float2* E2f;
+  double* scale;
   TRY(pool_get(c, "shell_prim0", sizeof(ShPrim) * T.nprim, &p)); F.prim = (ShPrim*)p;
   TRY(pool_get(c, "shell_E0", sizeof(double) * T.nE, &p)); F.E = (double*)p;
   TRY(pool_get(c, "shell_cnt", sizeof(int) * np, &p)); F.cnt = cnt = (int*)p;
   TRY(pool_get(c, "shell_prim", sizeof(ShPrim) * T.nprim, &p)); prim2 = (ShPrim*)p;
   TRY(pool_get(c, "shell_primf", sizeof(ShPrimF) * T.nprim, &p)); primf = (ShPrimF*)p;
   TRY(pool_get(c, "shell_E", sizeof(double) * T.nE, &p)); E2 = (double*)p;
-  TRY(pool_get(c, "shell_Ef", sizeof(float) * T.nE, &p)); Ef = (float*)p;
+  TRY(pool_get(c, "shell_E2", sizeof(float2) * T.nE, &p)); E2f = (float2*)p;
+  TRY(pool_get(c, "shell_scale", sizeof(double) * np, &p)); scale = (double*)p;
+  if (!c->pool["shell_boys"].ptr) {  // constants, once per context
+    TRY(pool_get(c, "shell_boys", sizeof(ShBoys) * (SH_MAXL + 1), &p));
+    shell_boys<<<dim3((SH_BOYS_K + 63) / 64, SH_MAXL + 1), 64, 0, c->stream>>>((ShBoys*)p);
+    SS_CUDA_TRY(cudaGetLastError());
+    c->launches++;
+  }
   TRY(pool_get(c, "shell_diag", sizeof(double) * np * SH_MAXCOMP, &p)); diag = (double*)p;
   SS_CUDA_TRY(cudaMemsetAsync(diag, 0, sizeof(double) * np * SH_MAXCOMP, c->stream));
   shell_fill<<<np, 256, 0, c->stream>>>(c->basis, dpair, st, F);
@@ -588,7 +642,7 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
     Lw.work[2 * P.d].push_back(w);
   }
   TRY(run_work(c, Lw, F.prim, nullptr, F.E, nullptr, true, 0.0, 0.0, diag));
-  shell_sort<<<np, 512, 0, c->stream>>>(dpair, st, cnt, diag, F.prim, F.E, prim2, primf, E2, Ef);
+  shell_sort<<<np, 512, 0, c->stream>>>(dpair, st, cnt, diag, F.prim, F.E, prim2, primf, E2, E2f, scale);
   SS_CUDA_TRY(cudaGetLastError());
   c->launches++;
   std::vector<double> h((size_t)np * SH_MAXCOMP);
@@ -665,7 +719,7 @@ int shell_plan(ss_ctx* c, const std::vector<int64_t>& sel, std::vector<int64_t>&
 
 int shell_run(ss_ctx* c, ShellPlan& plan, double eps, double eps32, double* elem) {
   return run_work(c, plan, (const ShPrim*)c->pool["shell_prim"].ptr, (const ShPrimF*)c->pool["shell_primf"].ptr,
-                  (const double*)c->pool["shell_E"].ptr, (const float*)c->pool["shell_Ef"].ptr, false, eps, eps32, elem);
+                  (const double*)c->pool["shell_E"].ptr, (const float2*)c->pool["shell_E2"].ptr, false, eps, eps32, elem);
 }
 
 }  // namespace ss
