@@ -8,13 +8,30 @@
 // parts, and the error stays about 2^-47 of the operands' magnitude.
 #pragma once
 
+// The arithmetic is plain IEEE FP32 with explicit fma, so it also compiles as host C++ (the host
+// build of the tests, contraction off).
+#ifdef __CUDACC__
+#define SS_DF __device__ __forceinline__
+#else
+#include <cmath>
+#define SS_DF inline
+inline float __fmul_rn(float a, float b) { return a * b; }
+inline float __fadd_rn(float a, float b) { return a + b; }
+inline float __fsub_rn(float a, float b) { return a - b; }
+inline float __fmaf_rn(float a, float b, float c) { return std::fma(a, b, c); }
+#endif
+
 namespace ss {
+
+#ifdef __CUDACC__
+SS_DF float df_rsqrt_seed(float x) { return rsqrtf(x); }
+#else
+SS_DF float df_rsqrt_seed(float x) { return 1.0f / std::sqrt(x); }
+#endif
 
 struct alignas(8) df {
   float h, l;
 };
-
-#define SS_DF __device__ __forceinline__
 
 SS_DF df df_from(double x) {
   const float h = (float)x;
@@ -57,7 +74,7 @@ SS_DF df df_fma_fast(df a, df b, df c) {
 SS_DF df df_renorm(df a) { return df_fast_sum(a.h, a.l); }
 // 1/sqrt(a): a float estimate corrected to the nearest float, then its residual 1 - a y^2
 SS_DF df df_rsqrt(df a) {
-  float y = rsqrtf(a.h);
+  float y = df_rsqrt_seed(a.h);
   float r = 0.f;
 #pragma unroll
   for (int it = 0; it < 2; it++) {

@@ -49,6 +49,7 @@ struct ShPair {
   int fa, fb;                        // one function of each shell (exponents, coefficients, centre)
   int onec, fold, same_system;
   int64_t prim_off, e_off;           // first primitive; first Hermite coefficient
+  double pmax;                       // largest exponent sum of its primitives
 };
 
 // A primitive pair: exponent sum, centre, w = K_AB c_a c_b / p, and (sorted tables) the largest
@@ -56,10 +57,9 @@ struct ShPair {
 struct ShPrim {
   double p, P[3], w, S;
 };
-// Two-float view (high and low parts); w is divided by the pair's power of two (ShArgs::scale), and
-// kx = 2^k ~ sqrt(2p) scales the Hermite degrees of the FP32 evaluations (shell_eri.cuh)
+// Two-float view (high and low parts); w is divided by the pair's power of two (ShArgs::scale)
 struct ShPrimF {
-  float p[2], ph[3], pl[3], w[2], kx, pad;
+  float p[2], ph[3], pl[3], w[2], pad[2];
 };
 static_assert(sizeof(ShPrim) == 48 && sizeof(ShPrimF) == 48, "primitive records are 48 bytes");
 

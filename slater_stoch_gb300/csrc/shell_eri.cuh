@@ -24,11 +24,17 @@
 #pragma once
 #include <math.h>
 
+#include <algorithm>
 #include <utility>
 
 #include "boys.cuh"
 #include "df32.cuh"
 #include "shell.cuh"
+
+#ifndef __CUDACC__
+using std::fma;
+using std::min;
+#endif
 
 namespace ss {
 
@@ -39,7 +45,7 @@ constexpr int SH_MAXSLICE = 16;              // bra primitives of a slice
 // <= 1/16), then F_n = (2T F_{n+1} + e^-T) / (2n+1), stable; above, erf(sqrt T) = 1 and the upward
 // recursion is stable.
 template <int L>
-__device__ __forceinline__ void boys_shell(double T, double (&F)[L + 1], const ShBoys* __restrict__ tab) {
+SS_DF void boys_shell(double T, double (&F)[L + 1], const ShBoys* __restrict__ tab) {
   const int64_t tb = bits_of(T);
   if (tb <= 0x4042000000000000LL) {  // T <= 36
     const double t = fma(T, 8.0, RINT_SHIFT);
@@ -71,7 +77,7 @@ __device__ __forceinline__ void boys_shell(double T, double (&F)[L + 1], const S
 // Two floats: the terms of degree >= 5 of the series in FP32 (they are below 1e-8 of F_L); above
 // T = 36, e^-T is below 3e-16 and taken in FP32.
 template <int L>
-__device__ __forceinline__ void boys_shell(df T, df (&F)[L + 1], const float* tab) {
+SS_DF void boys_shell(df T, df (&F)[L + 1], const float* tab) {
   if (T.h <= 36.f) {
     const int k = min((int)fmaf(T.h, 8.f, 0.5f), SH_BOYS_K - 1);
     const df x = df_fast_sum(__fsub_rn((float)k * 0.125f, T.h), -T.l);  // T_k - T
@@ -126,7 +132,7 @@ __device__ __forceinline__ void boys_shell(df T, df (&F)[L + 1], const float* ta
 
 // FP32, the same series to degree 5; above T = 30 the asymptotic F_0
 template <int L>
-__device__ __forceinline__ void boys_shell(float T, float (&F)[L + 1], const float* tab) {
+SS_DF void boys_shell(float T, float (&F)[L + 1], const float* tab) {
   if (T >= 30.f) {
     const float h = 0.5f / T;
     const float e = expf(-T);
@@ -150,15 +156,15 @@ __device__ __forceinline__ void boys_shell(float T, float (&F)[L + 1], const flo
 }
 
 // the operations of the recursion in each type
-__device__ __forceinline__ double r_mul(double a, double b) { return a * b; }
-__device__ __forceinline__ float r_mul(float a, float b) { return a * b; }
-__device__ __forceinline__ df r_mul(df a, df b) { return df_mul(a, b); }
-__device__ __forceinline__ double r_fma(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float r_fma(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ df r_fma(df a, df b, df c) { return df_fma(a, b, c); }
-__device__ __forceinline__ double r_times(double a, int n) { return n == 1 ? a : (double)n * a; }
-__device__ __forceinline__ float r_times(float a, int n) { return n == 1 ? a : (float)n * a; }
-__device__ __forceinline__ df r_times(df a, int n) {
+SS_DF double r_mul(double a, double b) { return a * b; }
+SS_DF float r_mul(float a, float b) { return a * b; }
+SS_DF df r_mul(df a, df b) { return df_mul(a, b); }
+SS_DF double r_fma(double a, double b, double c) { return fma(a, b, c); }
+SS_DF float r_fma(float a, float b, float c) { return fmaf(a, b, c); }
+SS_DF df r_fma(df a, df b, df c) { return df_fma(a, b, c); }
+SS_DF double r_times(double a, int n) { return n == 1 ? a : (double)n * a; }
+SS_DF float r_times(float a, int n) { return n == 1 ? a : (float)n * a; }
+SS_DF df r_times(df a, int n) {
   return n == 1 ? a : ((n & (n - 1)) == 0 ? df_scale(a, (float)n) : df_mulf(a, (float)n));
 }
 
@@ -178,7 +184,7 @@ __host__ __device__ constexpr ShDeg sh_degs(int i) {
 
 // One entry of the recursion below, all indices at compile time.
 template <int I, typename Real, int N>
-__device__ __forceinline__ void hermite_step(Real X, Real Y, Real Z, Real (&R)[N]) {
+SS_DF void hermite_step(Real X, Real Y, Real Z, Real (&R)[N]) {
   constexpr ShDeg h = sh_degs(I);
   constexpr int big = 99;
   constexpr int at = h.t ? h.t : big, au = h.u ? h.u : big, av = h.v ? h.v : big;
@@ -194,7 +200,7 @@ __device__ __forceinline__ void hermite_step(Real X, Real Y, Real Z, Real (&R)[N
   }
 }
 template <typename Real, int N, int... I>
-__device__ __forceinline__ void hermite_level(Real X, Real Y, Real Z, Real (&R)[N], std::integer_sequence<int, I...>) {
+SS_DF void hermite_level(Real X, Real Y, Real Z, Real (&R)[N], std::integer_sequence<int, I...>) {
   (hermite_step<(int)sizeof...(I) - I>(X, Y, Z, R), ...);  // indices sizeof...(I) .. 1
 }
 
@@ -203,7 +209,7 @@ __device__ __forceinline__ void hermite_level(Real X, Real Y, Real Z, Real (&R)[
 // degree of one needs no second term).  Level m overwrites level m + 1 from the highest index
 // down, so each entry reads values that are still of level m + 1.  base[m] = R^(m)_000.
 template <int L, int M, typename Real>
-__device__ __forceinline__ void hermite_levels(Real X, Real Y, Real Z, const Real (&base)[L + 1],
+SS_DF void hermite_levels(Real X, Real Y, Real Z, const Real (&base)[L + 1],
                                                Real (&R)[sh_nherm(L)]) {
   if constexpr (M >= 0) {
     hermite_level(X, Y, Z, R, std::make_integer_sequence<int, sh_nherm(L - M) - 1>());
@@ -215,11 +221,11 @@ __device__ __forceinline__ void hermite_levels(Real X, Real Y, Real Z, const Rea
 __host__ __device__ constexpr int sh_dfact(int n) { return n <= 1 ? 1 : n * sh_dfact(n - 2); }  // n!!
 
 template <typename Real, int N, int... I>
-__device__ __forceinline__ void put_row(const Real (&R)[N], Real* row, std::integer_sequence<int, I...>) {
+SS_DF void put_row(const Real (&R)[N], Real* row, std::integer_sequence<int, I...>) {
   ((row[I] = R[I]), ...);
 }
 template <int L, typename Real>
-__device__ __forceinline__ void store_row(Real X, Real Y, Real Z, const Real (&base)[L + 1], Real* row) {
+SS_DF void store_row(Real X, Real Y, Real Z, const Real (&base)[L + 1], Real* row) {
   Real R[sh_nherm(L)];
   R[0] = base[L];
   hermite_levels<L, L - 1>(X, Y, Z, base, R);
@@ -228,7 +234,7 @@ __device__ __forceinline__ void store_row(Real X, Real Y, Real Z, const Real (&b
 
 // all four shells on one centre: only the even degrees, R_{2a 2b 2c} = (2a-1)!! (2b-1)!! (2c-1)!! base[a+b+c]
 template <int I, typename Real, int N>
-__device__ __forceinline__ void put_1c(const Real (&base)[N], Real* row) {
+SS_DF void put_1c(const Real (&base)[N], Real* row) {
   constexpr ShDeg h = sh_degs(I);
   if constexpr (!((h.t | h.u | h.v) & 1)) {
     constexpr int c = sh_dfact(h.t - 1) * sh_dfact(h.u - 1) * sh_dfact(h.v - 1);
@@ -236,14 +242,15 @@ __device__ __forceinline__ void put_1c(const Real (&base)[N], Real* row) {
   }
 }
 template <typename Real, int N, int... I>
-__device__ __forceinline__ void put_row_1c(const Real (&base)[N], Real* row, std::integer_sequence<int, I...>) {
+SS_DF void put_row_1c(const Real (&base)[N], Real* row, std::integer_sequence<int, I...>) {
   (put_1c<I>(base, row), ...);
 }
 template <int L, typename Real>
-__device__ __forceinline__ void store_row_1c(const Real (&base)[L + 1], Real* row) {
+SS_DF void store_row_1c(const Real (&base)[L + 1], Real* row) {
   put_row_1c(base, row, std::make_integer_sequence<int, sh_nherm(L)>());
 }
 
+#ifdef __CUDACC__
 __constant__ uint32_t sh_hermite[SH_MAXH] = {
 #define H_(t, u, v) ((t) | ((u) << 8) | ((v) << 16))
     H_(0, 0, 0), H_(1, 0, 0), H_(0, 1, 0), H_(0, 0, 1), H_(2, 0, 0), H_(1, 1, 0), H_(1, 0, 1), H_(0, 2, 0),
@@ -357,6 +364,11 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
   const int my_o = NO < NT ? tid - my_g * NO : tid;
   for (int o = tid; o < (NO > NT ? NO : NT); o += NT) s_acc[o] = 0.0;
   const double scale = diag ? 1.0 : A.scale[W.bra] * A.scale[W.ket];
+  // FP32 evaluations: degree n carries a factor kx^-n, a power of two that holds (2 alpha / kx^2)^L
+  // below 2^100 for the tightest primitives (1 unless 2 alpha exceeds 2^(100/L))
+  float kx = 1.f;
+  if (L > 0) kx = exp2f(fmaxf(0.f, ceilf(0.5f * (log2f((float)(2.0 * fmin(B.pmax, K.pmax))) - 100.f / (L > 0 ? L : 1)))));
+  const float k2 = kx * kx, ik2 = 1.f / k2;
   __syncthreads();
 
   for (int tier = 0; tier < 3; tier++) {
@@ -405,10 +417,7 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
           }
           continue;
         }
-        // two floats and FP32: degree n carries a factor kx^-n (kx ~ sqrt(2p) of the bra
-        // primitive), which keeps (2 alpha)^L of tight primitives inside the FP32 range
         const ShPrimF a = A.primf[B.prim_off + p], b = A.primf[K.prim_off + q];
-        const float kx = a.kx, ik2 = 1.f / (kx * kx);
         if (tier == 1) {
           df* row = reinterpret_cast<df*>(s_R) + (item - base) * ROW;
           const df pa{a.p[0], a.p[1]}, pb{b.p[0], b.p[1]};
@@ -485,7 +494,6 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
         while (scan[j + 1] <= lo) j++;
         // with an s-type bra the FP64 sums need no contraction and no segments
         const int hi = (H == 1 && tier == 0) ? top : min(top, scan[j + 1]);
-        const float kx = tier ? A.primf[B.prim_off + s_p[j]].kx : 1.f;
         const int i0 = lo - base + my_g, i1 = hi - base;
         const int q0 = lo - scan[j] + s_first[tier][j] + my_g;  // ket of the thread's first item
         for (int o = my_o; o < NO && my_g < G; o += NT) {
@@ -516,7 +524,6 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
               }
               s_acc[o + my_g * NO] += acc;
             } else {
-              const float k2 = kx * kx;
               df acc = reinterpret_cast<df*>(s_acc)[o + my_g * NO];
               for (int x = SK.fs[f]; x < x1; x++) {
                 const uint32_t tau = SK.term[x];
@@ -600,5 +607,7 @@ cudaError_t launch_shell_L(int ncta, int max_no, int max_ni, int max_col, cudaSt
   shell_eri_kernel<L><<<ncta, ShDim<L>::NT, smem, st>>>(A, max_no, max_ni, max_col);
   return cudaGetLastError();
 }
+
+#endif  // __CUDACC__
 
 }  // namespace ss

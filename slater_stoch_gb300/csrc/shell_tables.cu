@@ -314,8 +314,7 @@ __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pai
     two(a.p, &g.p[0], &g.p[1]);
     two(ldexp(a.w, -ex), &g.w[0], &g.w[1]);
     for (int ax = 0; ax < 3; ax++) two(a.P[ax], &g.ph[ax], &g.pl[ax]);
-    g.kx = exp2f(rintf(0.5f * log2f(2.f * g.p[0])));
-    g.pad = 0.f;
+    g.pad[0] = g.pad[1] = 0.f;
     oprimf[P.prim_off + t] = g;
   }
   for (int t = threadIdx.x; t < m * P.nterm; t += blockDim.x) {
@@ -435,6 +434,8 @@ void build_shells(ss_ctx* c) {
       P.nterm = S.nterm;
       const int na = c->h_ng[P.fa], nb = c->h_ng[P.fb];
       P.cap = P.fold ? na * (na + 1) / 2 : na * nb;
+      P.pmax = *std::max_element(&c->h_gg[(size_t)ld * P.fa], &c->h_gg[(size_t)ld * P.fa] + na) +
+               *std::max_element(&c->h_gg[(size_t)ld * P.fb], &c->h_gg[(size_t)ld * P.fb] + nb);
       P.prim_off = po;
       P.e_off = eo;
       po += P.cap;
