@@ -42,6 +42,58 @@ struct ShStruct {
   uint32_t combo[SH_MAXCOMP][9];     // packed powers of the two functions: 4 bits each ax ay az bx by bz
 };
 
+constexpr int SH_DEG[4] = {0, 1, 2, 2};  // S P R D
+constexpr int SH_NC[4] = {1, 3, 1, 6};
+constexpr int SH_POW[4][6][3] = {{{0, 0, 0}},
+                                 {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}},
+                                 {{0, 0, 0}},
+                                 {{2, 0, 0}, {1, 1, 0}, {1, 0, 1}, {0, 2, 0}, {0, 1, 1}, {0, 0, 2}}};
+
+// Pair type of canonical shell types ta >= tb; same: one shell with itself (components ca >= cb);
+// onec: both shells on one centre.  Components ca-major; a component's terms in (t, u, v) order.
+constexpr ShStruct sh_struct(int ta, int tb, bool same, bool onec) {
+  ShStruct S{};
+  S.d = SH_DEG[ta] + SH_DEG[tb];
+  int nterm = 0;
+  for (int ca = 0; ca < SH_NC[ta]; ca++)
+    for (int cb = 0; cb < SH_NC[tb]; cb++) {
+      if (same && cb > ca) continue;
+      const int f = S.ncomp++;
+      const int na = ta == SH_R ? 3 : 1, nb = tb == SH_R ? 3 : 1;
+      int pa[9][3] = {}, pb[9][3] = {};
+      for (int x = 0; x < na; x++)
+        for (int y = 0; y < nb; y++) {
+          const int k = S.ncombo[f]++;
+          uint32_t code = 0;
+          for (int ax = 0; ax < 3; ax++) {
+            pa[k][ax] = ta == SH_R ? (ax == x ? 2 : 0) : SH_POW[ta][ca][ax];
+            pb[k][ax] = tb == SH_R ? (ax == y ? 2 : 0) : SH_POW[tb][cb][ax];
+            code |= (uint32_t)pa[k][ax] << (4 * ax) | (uint32_t)pb[k][ax] << (4 * (3 + ax));
+          }
+          S.combo[f][k] = code;
+        }
+      S.fs[f] = nterm;
+      for (int t = 0; t <= S.d; t++)
+        for (int u = 0; t + u <= S.d; u++)
+          for (int v = 0; t + u + v <= S.d; v++) {
+            const int h[3] = {t, u, v};
+            bool any = false;
+            for (int k = 0; k < S.ncombo[f]; k++) {
+              bool ok = true;
+              for (int ax = 0; ax < 3; ax++) {
+                const int e = pa[k][ax] + pb[k][ax];
+                ok = ok && h[ax] <= e && !(onec && ((e - h[ax]) & 1));  // on one centre only equal parities
+              }
+              any = any || ok;
+            }
+            if (any) S.term[nterm++] = (uint32_t)(t | (u << 8) | (v << 16));
+          }
+    }
+  S.fs[S.ncomp] = nterm;
+  S.nterm = nterm;
+  return S;
+}
+
 // One shell pair.  Its primitives occupy prim[prim_off .. prim_off + cap), cnt[pair] of them used.
 struct ShPair {
   int st, d, ncomp, nterm;
@@ -67,7 +119,9 @@ static_assert(sizeof(ShPrim) == 48 && sizeof(ShPrimF) == 48, "primitive records 
 struct ShWork {
   int bra, ket;          // shell pairs
   int cta0, split;       // first CTA, number of bra slices
-  int64_t part, elem;    // first partial sum [element][slice]; first element of the result
+  int lane, lcta0, nlane;  // lane kernel: instance (-1: none), first CTA, CTAs
+  int lsplit, nkc;       // its partial sums per element (bra blocks x ket chunks), ket chunks
+  int64_t part, elem;    // first partial sum [element][split + lsplit]; first element of the result
   uint64_t mask;         // ket components that are asked for
 };
 
@@ -96,12 +150,34 @@ struct ShArgs {
   const int* cta;        // work entry of each CTA of the chunk
   int cta0;              // first CTA of this launch in it
   double* partial;
+  const int* lcta;       // the same for the lane kernels
   double eps, eps32, eps_df;
   int diag;              // 1: (P|Q) of a pair with itself, Q <= P, diagonal elements only
 };
 
 constexpr int SH_SMEM_MAX = 200 * 1024;
+constexpr int SH_MAXSLICE = 16;  // bra primitives of a slice
 
 cudaError_t launch_shell_eri(int L, int ncta, int max_no, int max_ni, int max_col, cudaStream_t st, const ShArgs& A);
+
+// Lane kernels (shell_lane.cuh): bra degree DB, ket type; a CTA takes SH_LANE_BRA bra primitives (one
+// per thread), SH_LANE_KET ket primitives and one chunk of the ket's components.
+constexpr int SH_LANE_BRA = 128, SH_LANE_KET = 64;
+// ket components per chunk for a bra of degree db and a ket type (ta, tb), 0: no such kernel
+constexpr int sh_lane_chunk(int db, int ta, int tb) {
+  const int k = ta * (ta + 1) / 2 + tb;  // SS PS PP RS RP RR DS DP DR DD
+  if (k == 0) return db <= 4 ? 1 : 0;                                        // SS
+  if (k == 1) return db == 1 || db == 2 ? 3 : (db == 3 || db == 4 ? 1 : 0);  // PS
+  if (k == 2) return db == 2 ? 3 : 0;                                        // PP
+  if (k == 3) return db >= 1 && db <= 3 ? 1 : 0;                             // RS
+  if (k == 4) return db == 1 || db == 2 ? 3 : (db == 3 ? 1 : 0);             // RP
+  if (k == 5) return db == 1 || db == 2 ? 1 : 0;                             // RR
+  if (k == 6) return db == 2 ? 3 : 0;                                        // DS
+  if (k == 8) return db == 1 ? 3 : 0;                                        // DR
+  return 0;
+}
+// instance = 8 * (pair type index) + bra degree, + SH_LANE_ONEC where all four shells are on one centre
+constexpr int SH_LANE_ONEC = 1024;
+cudaError_t launch_shell_lane(int instance, int ncta, cudaStream_t st, const ShArgs& A);
 
 }  // namespace ss

@@ -39,7 +39,6 @@ using std::min;
 namespace ss {
 
 constexpr double SH_PI_5_2 = 34.9868366552;  // src/general_primitive_integral.F90:25
-constexpr int SH_MAXSLICE = 16;              // bra primitives of a slice
 
 // F_0..F_L(T), T >= 0.  T <= 36: F_L from the Taylor series around T_k = k/8 (nine terms, |T - T_k|
 // <= 1/16), then F_n = (2T F_{n+1} + e^-T) / (2n+1), stable; above, erf(sqrt T) = 1 and the upward
@@ -266,9 +265,9 @@ __device__ __forceinline__ int sh_degree(uint32_t h) { return (int)((h & 255) + 
 // degree 5 on, where the sums of step 2 are most of the work.
 template <int L>
 struct ShDim {
-  static constexpr int NT = 128;
+  static constexpr int NT = L >= 6 ? 256 : 128;
   static constexpr int NB = L >= 5 ? 64 : 128;
-  static constexpr int MINB = L >= 7 ? 2 : L >= 4 ? 3 : 4;  // CTAs per SM the registers must allow
+  static constexpr int MINB = L >= 6 ? 2 : 4;  // CTAs per SM the registers must allow
   static constexpr int ROW = sh_nherm(L) | 1;  // odd: a column over the items meets no bank twice
   static size_t bytes(int max_no, int max_ni, int max_col) {
     return sizeof(float) * SH_BOYS_K * SH_BOYS_ROW +
@@ -309,7 +308,10 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
   const uint64_t mask = W.mask;
   if (NO > (max_no > NT ? max_no : NT) || NI > max_ni || H * nterm > max_col || B.d + K.d != L) return;  // uniform
 
-  if (!diag) {
+  // the tiers below FP64 of a quartet with a lane kernel are that kernel's
+  const int tiers = diag || W.lane >= 0 ? 1 : 3;
+  const int64_t stride = W.split + W.lsplit;
+  if (tiers > 1) {
     const float4* src = reinterpret_cast<const float4*>(boys->f);
     for (int i = tid; i < SH_BOYS_K * SH_BOYS_ROW / 4; i += NT) sh_raw[i] = src[i];
   }
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
   const float k2 = kx * kx, ik2 = 1.f / k2;
   __syncthreads();
 
-  for (int tier = 0; tier < 3; tier++) {
+  for (int tier = 0; tier < tiers; tier++) {
     const int* scan = s_scan[tier];
     const int n = scan[SH_MAXSLICE];
     for (int base = 0; base < n; base += NB) {
@@ -592,9 +594,9 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
     }
   }
   if (diag) {
-    for (int a = tid; a < nf; a += NT) A.partial[W.part + (int64_t)a * W.split + slice] = SH_PI_5_2 * s_out[a * nf + a];
+    for (int a = tid; a < nf; a += NT) A.partial[W.part + a * stride + slice] = SH_PI_5_2 * s_out[a * nf + a];
   } else {
-    for (int e = tid; e < NI; e += NT) A.partial[W.part + (int64_t)e * W.split + slice] = SH_PI_5_2 * s_out[e];
+    for (int e = tid; e < NI; e += NT) A.partial[W.part + e * stride + slice] = SH_PI_5_2 * s_out[e];
   }
 }
 

@@ -14,7 +14,7 @@ struct ShellPlan {
 
 void build_shells(ss_ctx* c);
 int shell_precond(ss_ctx* c, std::vector<double>& pre);
-int shell_plan(ss_ctx* c, const std::vector<int64_t>& sel, std::vector<int64_t>& slot, std::vector<int64_t>& rest,
+int shell_plan(ss_ctx* c, bool tiers, const std::vector<int64_t>& sel, std::vector<int64_t>& slot, std::vector<int64_t>& rest,
                ShellPlan& plan, int64_t* nelem);
 int shell_run(ss_ctx* c, ShellPlan& plan, double eps, double eps32, double* elem);
 

@@ -1,0 +1,8 @@
+// shell_lane_dr1.cu -- shell_lane_kernel of the ket type DR, on one centre (own translation unit).
+#include "shell_lane.cuh"
+
+namespace ss {
+cudaError_t launch_lane_dr1(int db, int ncta, cudaStream_t st, const ShArgs& A) {
+  return launch_lane_bra<SH_D, SH_R, false, true, false>(db, ncta, st, A);
+}
+}  // namespace ss

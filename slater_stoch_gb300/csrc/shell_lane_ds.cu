@@ -1,0 +1,8 @@
+// shell_lane_ds.cu -- shell_lane_kernel of the ket type DS (own translation unit).
+#include "shell_lane.cuh"
+
+namespace ss {
+cudaError_t launch_lane_ds(int db, int ncta, cudaStream_t st, const ShArgs& A) {
+  return launch_lane_bra<SH_D, SH_S, false, false, false>(db, ncta, st, A);
+}
+}  // namespace ss

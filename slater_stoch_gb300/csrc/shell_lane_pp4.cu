@@ -1,0 +1,8 @@
+// shell_lane_pp4.cu -- shell_lane_kernel of the ket type PP, all four shells on one centre (own translation unit).
+#include "shell_lane.cuh"
+
+namespace ss {
+cudaError_t launch_lane_pp4(int db, int ncta, cudaStream_t st, const ShArgs& A) {
+  return launch_lane_bra<SH_P, SH_P, false, true, true>(db, ncta, st, A);
+}
+}  // namespace ss

@@ -30,13 +30,6 @@ constexpr double SH_DF_EPS = 1e-5;
 
 // ---- pair types ------------------------------------------------------------------------------
 
-static const int SH_DEG[4] = {0, 1, 2, 2};    // S P R D
-static const int SH_NC[4] = {1, 3, 1, 6};
-static const int SH_POW[4][6][3] = {{{0, 0, 0}},
-                                    {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}},
-                                    {{0, 0, 0}},
-                                    {{2, 0, 0}, {1, 1, 0}, {1, 0, 1}, {0, 2, 0}, {0, 1, 1}, {0, 0, 2}}};
-
 // pair type of canonical shell types ta >= tb; same: one shell with itself (components ca >= cb)
 static int struct_index(int ta, int tb, bool same, bool onec) {
   int base = ta * (ta + 1) / 2 + tb;
@@ -45,57 +38,15 @@ static int struct_index(int ta, int tb, bool same, bool onec) {
   return 2 * base + (onec ? 1 : 0);
 }
 
-static void build_struct(ShStruct& S, int ta, int tb, bool same, bool onec) {
-  memset(&S, 0, sizeof S);
-  S.d = SH_DEG[ta] + SH_DEG[tb];
-  int nterm = 0;
-  for (int ca = 0; ca < SH_NC[ta]; ca++)
-    for (int cb = 0; cb < SH_NC[tb]; cb++) {
-      if (same && cb > ca) continue;
-      const int f = S.ncomp++;
-      const int na = ta == SH_R ? 3 : 1, nb = tb == SH_R ? 3 : 1;
-      int pa[9][3], pb[9][3];
-      for (int x = 0; x < na; x++)
-        for (int y = 0; y < nb; y++) {
-          const int k = S.ncombo[f]++;
-          uint32_t code = 0;
-          for (int ax = 0; ax < 3; ax++) {
-            pa[k][ax] = ta == SH_R ? (ax == x ? 2 : 0) : SH_POW[ta][ca][ax];
-            pb[k][ax] = tb == SH_R ? (ax == y ? 2 : 0) : SH_POW[tb][cb][ax];
-            code |= (uint32_t)pa[k][ax] << (4 * ax) | (uint32_t)pb[k][ax] << (4 * (3 + ax));
-          }
-          S.combo[f][k] = code;
-        }
-      S.fs[f] = nterm;
-      for (int t = 0; t <= S.d; t++)
-        for (int u = 0; t + u <= S.d; u++)
-          for (int v = 0; t + u + v <= S.d; v++) {
-            const int h[3] = {t, u, v};
-            bool any = false;
-            for (int k = 0; k < S.ncombo[f]; k++) {
-              bool ok = true;
-              for (int ax = 0; ax < 3; ax++) {
-                const int e = pa[k][ax] + pb[k][ax];
-                ok = ok && h[ax] <= e && !(onec && ((e - h[ax]) & 1));  // on one centre only equal parities
-              }
-              any = any || ok;
-            }
-            if (any) S.term[nterm++] = (uint32_t)(t | (u << 8) | (v << 16));
-          }
-    }
-  S.fs[S.ncomp] = nterm;
-  S.nterm = nterm;
-}
-
 struct StructTable {
   std::vector<ShStruct> s;
   StructTable() : s(SH_NSTRUCT) {
     for (int ta = 0; ta < 4; ta++)
       for (int tb = 0; tb <= ta; tb++)
-        for (int oc = 0; oc < 2; oc++) build_struct(s[struct_index(ta, tb, false, oc)], ta, tb, false, oc);
+        for (int oc = 0; oc < 2; oc++) s[struct_index(ta, tb, false, oc)] = sh_struct(ta, tb, false, oc);
     for (int oc = 0; oc < 2; oc++) {
-      build_struct(s[struct_index(SH_P, SH_P, true, oc)], SH_P, SH_P, true, oc);
-      build_struct(s[struct_index(SH_D, SH_D, true, oc)], SH_D, SH_D, true, oc);
+      s[struct_index(SH_P, SH_P, true, oc)] = sh_struct(SH_P, SH_P, true, oc);
+      s[struct_index(SH_D, SH_D, true, oc)] = sh_struct(SH_D, SH_D, true, oc);
     }
   }
 };
@@ -207,23 +158,25 @@ __global__ void __launch_bounds__(256) shell_fill(BasisDev B, const ShPair* __re
   if (threadIdx.x == 0) out.cnt[blockIdx.x] = s_total;
 }
 
-// sum of the slices of every element: elem[e] = sum_s part[e * split + s]
+// sum of the partial sums of every element, in their order
 __global__ void shell_reduce(int nwork, const ShWork* __restrict__ work, const ShPair* __restrict__ pairs, int diag,
                              const double* __restrict__ part, double* __restrict__ elem) {
   const ShWork W = work[blockIdx.x];
   const int ni = diag ? pairs[W.bra].ncomp : pairs[W.bra].ncomp * pairs[W.ket].ncomp;
   for (int e = threadIdx.x; e < ni; e += blockDim.x) {
-    const double* p = part + W.part + (int64_t)e * W.split;
+    const int n = W.split + W.lsplit;
+    const double* p = part + W.part + (int64_t)e * n;
     double v = 0.0;
-    for (int s = 0; s < W.split; s++) v = v + p[s];
+    for (int s = 0; s < n; s++) v = v + p[s];
     elem[W.elem + e] = v;
   }
 }
 
 // work entry of every CTA
-__global__ void shell_expand(const ShWork* __restrict__ work, int* __restrict__ cta) {
+__global__ void shell_expand(const ShWork* __restrict__ work, int* __restrict__ cta, int* __restrict__ lcta) {
   const ShWork W = work[blockIdx.x];
   for (int s = threadIdx.x; s < W.split; s += blockDim.x) cta[W.cta0 + s] = blockIdx.x;
+  for (int s = threadIdx.x; s < W.nlane; s += blockDim.x) lcta[W.lcta0 + s] = blockIdx.x;
 }
 
 // Schwarz factors of a pair's primitives and their sorted tables.  A primitive's factor is the
@@ -362,6 +315,33 @@ cudaError_t launch_shell_eri(int L, int ncta, int max_no, int max_ni, int max_co
   return cudaErrorInvalidValue;
 }
 
+#define SH_LANE_KETS(X) \
+  X(ss, SH_S, SH_S) X(ps, SH_P, SH_S) X(pp, SH_P, SH_P) X(rs, SH_R, SH_S) X(rp, SH_R, SH_P) X(rr, SH_R, SH_R) \
+  X(ds, SH_D, SH_S) X(dr, SH_D, SH_R)
+#define SH_DECL(n, a, b)                                                     \
+  cudaError_t launch_lane_##n(int, int, cudaStream_t, const ShArgs&);        \
+  cudaError_t launch_lane_##n##1(int, int, cudaStream_t, const ShArgs&);     \
+  cudaError_t launch_lane_##n##4(int, int, cudaStream_t, const ShArgs&);
+SH_LANE_KETS(SH_DECL)
+#undef SH_DECL
+cudaError_t launch_lane_pps(int, int, cudaStream_t, const ShArgs&);
+cudaError_t launch_lane_pps4(int, int, cudaStream_t, const ShArgs&);
+// an s pair has one term on one and on two centres
+cudaError_t launch_lane_ss1(int db, int ncta, cudaStream_t st, const ShArgs& A) { return launch_lane_ss(db, ncta, st, A); }
+
+cudaError_t launch_shell_lane(int instance, int ncta, cudaStream_t st, const ShArgs& A) {
+  const bool all = instance >= SH_LANE_ONEC;
+  const int db = instance & 7, ket = (instance & (SH_LANE_ONEC - 1)) >> 3;
+#define SH_CASE(n, a, b)                                                          \
+  if (ket / 2 == a * (a + 1) / 2 + b)                                             \
+    return all ? launch_lane_##n##4(db, ncta, st, A) : (ket & 1) ? launch_lane_##n##1(db, ncta, st, A) \
+                                                                 : launch_lane_##n(db, ncta, st, A);
+  SH_LANE_KETS(SH_CASE)
+#undef SH_CASE
+  if (ket / 2 == SH_NBASE) return all ? launch_lane_pps4(db, ncta, st, A) : launch_lane_pps(db, ncta, st, A);
+  return cudaErrorInvalidValue;
+}
+
 // ---- host ------------------------------------------------------------------------------------
 
 // Shells of the basis and their pairs (host only; rebuilt by ss_basis_set / ss_basis_systems).
@@ -471,25 +451,41 @@ static bool shell_component(const ShellBasis& T, int i, int k, int* pair, int* c
   return true;
 }
 
-// multiply-adds per primitive quartet beyond the Hermite integrals; an s-type bra needs no
-// contraction per bra primitive
-static double side_cost(const ShPair& b, const ShPair& k) {
-  const double h = sh_nherm(b.d);
-  return h * k.nterm + (b.d > 0 ? 6.0 : 0.0);
+// multiply-adds of the Hermite integrals of total degree L
+static const double SH_REC[SH_MAXL + 1] = {2, 8, 24, 60, 120, 200, 330, 520, 790};
+
+// pair type (without the one-centre bit) of the lane kernels' rule
+static int lane_chunk(const ShPair& b, const ShPair& k) {
+  const int base = k.st / 2;
+  if (base == SH_NBASE + 1) return 0;  // D with itself
+  const int ix = base == SH_NBASE ? SH_P * (SH_P + 1) / 2 + SH_P : base;
+  for (int ta = 0; ta < 4; ta++)
+    for (int tb = 0; tb <= ta; tb++)
+      if (ta * (ta + 1) / 2 + tb == ix) return sh_lane_chunk(b.d, ta, tb);
+  return 0;
 }
 
-// bra slices of a shell quartet: a CTA's bra primitives so that it has about 1e6 multiply-adds at
-// a hundred kept kets each, at most SH_MAXSLICE of them; never from what else is in the list, so
-// that the order of summation is the quartet's own
-static int slices(const ShPair& b, const ShPair& k) {
+// FP32-pipe instructions of one primitive quartet in two floats with this bra and ket: the Hermite
+// integrals (once per chunk of the ket's components in the lane kernels), a two-float
+// multiply-add per bra Hermite function and ket term, and the shared kernel's own overhead
+// (loads and indices per term, barriers and segments).  The cheaper orientation is taken.
+static double side_cost(const ShPair& b, const ShPair& k) {
   const int L = b.d + k.d;
-  static const double rec[SH_MAXL + 1] = {2, 8, 24, 60, 120, 200, 330, 520, 790};
-  const double cost = 30.0 + 4.0 * L + rec[L] + side_cost(b, k);
-  int per = (int)std::min(16.0, std::max(2.0, 1e4 / cost));
-  per = std::max(per, (b.cap + 126) / 127);
+  const double herm = 290.0 + 36.0 * L + 8.0 * SH_REC[L], terms = (double)sh_nherm(b.d) * k.nterm;
+  const int c = lane_chunk(b, k);
+  return c ? herm * ((k.ncomp + c - 1) / c) + 12.2 * terms : herm + 18.0 * terms + 1500.0;
+}
+
+// bra slices of a shell quartet in the shared kernel: a CTA's bra primitives so that it has about
+// 1e6 multiply-adds at a hundred kept kets each (16 where it only has the FP64 tier), at most
+// SH_MAXSLICE of them; never from what else is in the list, so that the order of summation is the
+// quartet's own
+static int slices(const ShPair& b, const ShPair& k, bool lane) {
+  const int L = b.d + k.d;
+  const double cost = 30.0 + 4.0 * L + SH_REC[L] + (double)sh_nherm(b.d) * k.nterm;
+  const int per = lane ? SH_MAXSLICE : (int)std::min((double)SH_MAXSLICE, std::max(2.0, 1e4 / cost));
   return std::max(1, (b.cap + per - 1) / per);
 }
-
 
 // Launch the work entries (grouped by total degree), in chunks whose partial sums fit the buffer,
 // and reduce each chunk's partial sums to elements.
@@ -504,17 +500,33 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
   std::vector<ShWork> chunk;
   struct Seg { int L, first, n, ncta, no, ni, col; };
   std::vector<Seg> segs;
+  struct LaneSeg { int instance, cta0, ncta; };
+  std::vector<LaneSeg> lanes;
   int64_t part = 0, most = 0;
-  int ncta = 0;
+  int ncta = 0, nlane = 0;
   auto flush = [&]() -> int {
     if (chunk.empty()) return SS_OK;
+    // the lane kernels' CTAs, an instance's together
+    std::vector<int> order;
+    for (size_t t = 0; t < chunk.size(); t++)
+      if (chunk[t].lane >= 0) order.push_back((int)t);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return chunk[x].lane > chunk[y].lane; });
+    lanes.clear();
+    nlane = 0;
+    for (int t : order) {
+      if (lanes.empty() || lanes.back().instance != chunk[t].lane) lanes.push_back(LaneSeg{chunk[t].lane, nlane, 0});
+      chunk[t].lcta0 = nlane;
+      lanes.back().ncta += chunk[t].nlane;
+      nlane += chunk[t].nlane;
+    }
     void *dw, *dc, *dp;
     TRY(pool_get(c, "shell_part", sizeof(double) * (size_t)std::max(part, std::min(most, cap_d)), &dp));
     DevBuf& wb = c->pool["shell_work"];
     TRY(h2d_async(c, wb, chunk.data(), sizeof(ShWork) * chunk.size()));
     dw = wb.ptr;
-    TRY(pool_get(c, "shell_cta", sizeof(int) * (size_t)ncta, &dc));
-    shell_expand<<<(unsigned)chunk.size(), 32, 0, c->stream>>>((const ShWork*)dw, (int*)dc);
+    TRY(pool_get(c, "shell_cta", sizeof(int) * ((size_t)ncta + nlane), &dc));
+    int* lcta = (int*)dc + ncta;
+    shell_expand<<<(unsigned)chunk.size(), 32, 0, c->stream>>>((const ShWork*)dw, (int*)dc, lcta);
     SS_CUDA_TRY(cudaGetLastError());
     c->launches++;
     TRY(fork_eri_streams(c));
@@ -533,13 +545,24 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
     A.eps32 = eps32;
     A.eps_df = SH_DF_EPS;
     A.diag = diag;
+    A.work = (const ShWork*)dw;
+    A.cta = (const int*)dc;
+    A.lcta = lcta;
     int rc = SS_OK;
+    size_t launch = 0;
+    for (size_t s = 0; s < lanes.size() && !rc; s++) {
+      A.cta0 = lanes[s].cta0;
+      const cudaError_t e = launch_shell_lane(lanes[s].instance, lanes[s].ncta, c->eri_stream[launch++ % ss_ctx::ERI_STREAMS], A);
+      if (e != cudaSuccess) {
+        ss_set_cuda_error(e, "shell_lane_kernel launch", __FILE__, __LINE__);
+        rc = SS_ERR_CUDA;
+      }
+      c->launches++;
+    }
     for (size_t s = 0; s < segs.size() && !rc; s++) {
       const Seg& g = segs[s];
-      A.work = (const ShWork*)dw;
-      A.cta = (const int*)dc;
       A.cta0 = chunk[g.first].cta0;
-      const cudaError_t e = launch_shell_eri(g.L, g.ncta, g.no, g.ni, g.col, c->eri_stream[s % ss_ctx::ERI_STREAMS], A);
+      const cudaError_t e = launch_shell_eri(g.L, g.ncta, g.no, g.ni, g.col, c->eri_stream[launch++ % ss_ctx::ERI_STREAMS], A);
       if (e != cudaSuccess) {
         ss_set_cuda_error(e, "shell_eri_kernel launch", __FILE__, __LINE__);
         rc = SS_ERR_CUDA;
@@ -555,11 +578,11 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
     chunk.clear();
     segs.clear();
     part = 0;
-    ncta = 0;
+    ncta = nlane = 0;
     return SS_OK;
   };
   for (int L = 0; L <= SH_MAXL; L++)
-    for (const ShWork& w : Lw.work[L]) most += (int64_t)w.split * (diag ? T.pair[w.bra].ncomp : T.pair[w.bra].ncomp * T.pair[w.ket].ncomp);
+    for (const ShWork& w : Lw.work[L]) most += (int64_t)(w.split + w.lsplit) * (diag ? T.pair[w.bra].ncomp : T.pair[w.bra].ncomp * T.pair[w.ket].ncomp);
   for (int L = SH_MAXL; L >= 0; L--) {
     std::vector<ShWork>& v = Lw.work[L];
     auto cost = [&](const ShWork& w) { return side_cost(T.pair[w.bra], T.pair[w.ket]); };
@@ -568,8 +591,8 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
     for (ShWork& w : v) {
       const ShPair &b = T.pair[w.bra], &k = T.pair[w.ket];
       const int ni = b.ncomp * k.ncomp;
-      const int64_t need = (int64_t)w.split * (diag ? b.ncomp : ni);
-      if (!chunk.empty() && (part + need > cap_d || ncta > (1 << 28))) {
+      const int64_t need = (int64_t)(w.split + w.lsplit) * (diag ? b.ncomp : ni);
+      if (!chunk.empty() && (part + need > cap_d || ncta + nlane > (1 << 28))) {
         TRY(flush());
         open = false;
       }
@@ -587,6 +610,7 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
       g.ni = std::max(g.ni, ni);
       g.col = std::max(g.col, sh_nherm(b.d) * k.nterm);
       ncta += w.split;
+      nlane += w.nlane;
       part += need;
     }
   }
@@ -637,7 +661,8 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
     if (!P.same_system) continue;
     ShWork w{};
     w.bra = w.ket = x;
-    w.split = slices(P, P);
+    w.split = slices(P, P, false);
+    w.lane = -1;
     w.elem = (int64_t)x * SH_MAXCOMP;
     w.mask = ~0ull;
     Lw.work[2 * P.d].push_back(w);
@@ -661,8 +686,8 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
 
 // Shell quartets of the selected function quartets.  Quartets with a function in no shell go to
 // `rest`; of the others, slot[q] receives the place of the result (one element, offset from
-// `first`), and *nelem the number of elements.
-int shell_plan(ss_ctx* c, const std::vector<int64_t>& sel, std::vector<int64_t>& slot, std::vector<int64_t>& rest,
+// `first`), and *nelem the number of elements.  tiers: the FP32 tiers are on.
+int shell_plan(ss_ctx* c, bool tiers, const std::vector<int64_t>& sel, std::vector<int64_t>& slot, std::vector<int64_t>& rest,
                ShellPlan& plan, int64_t* nelem) {
   const ShellBasis& T = c->shells;
   const int n = c->n;
@@ -709,7 +734,18 @@ int shell_plan(ss_ctx* c, const std::vector<int64_t>& sel, std::vector<int64_t>&
     ShWork w{};
     w.bra = s.bra;
     w.ket = s.ket;
-    w.split = slices(T.pair[s.bra], T.pair[s.ket]);
+    const ShPair &b = T.pair[s.bra], &k = T.pair[s.ket];
+    const int chunk = tiers ? lane_chunk(b, k) : 0;
+    w.lane = -1;
+    if (chunk) {
+      bool all = b.onec && k.onec;
+      for (int ax = 0; ax < 3; ax++) all = all && c->h_center[3 * b.fa + ax] == c->h_center[3 * k.fa + ax];
+      w.lane = 8 * k.st + b.d + (all ? SH_LANE_ONEC : 0);
+      w.nkc = (k.cap + SH_LANE_KET - 1) / SH_LANE_KET;
+      w.lsplit = w.nkc * ((b.cap + SH_LANE_BRA - 1) / SH_LANE_BRA);
+      w.nlane = w.lsplit * ((k.ncomp + chunk - 1) / chunk);
+    }
+    w.split = slices(b, k, chunk > 0);
     w.elem = s.elem;
     w.mask = s.mask;
     plan.work[T.pair[s.bra].d + T.pair[s.ket].d].push_back(w);
