@@ -592,42 +592,35 @@ __global__ void __launch_bounds__(256) sym_eig_smem_kernel(int n, const double* 
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t GRID_SPIN_LIMIT = 1u << 22;  // bounded grid barrier (seconds of L2 polling; a round takes microseconds)
 constexpr int JACOBI_MAX_SWEEPS = 40;
+constexpr int JACOBI_THREADS = 512;
 
 struct JacobiCtl {
-  unsigned int count, gen;  // grid barrier
+  unsigned int count;       // grid barrier: arrivals since the start
   int rot[2];               // rotations of the current / previous sweep (by sweep parity)
   double amax;
   int sweeps;               // sweeps the last solve took
 };
 
-// Sense-free generation barrier over all CTAs of a cooperative launch (all co-resident).  A
-// wait that runs past its limit sets *err = 2; every later barrier then returns at once.
-__device__ bool grid_barrier(JacobiCtl* ctl, int* err) {
+// Barrier over all CTAs of a cooperative launch (all co-resident); `target` is gridDim.x times the
+// number of barriers so far, this one included.  A wait that runs past its limit sets *err = 2;
+// every later barrier then returns at once.
+__device__ bool grid_barrier(JacobiCtl* ctl, unsigned int target, int* err) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    volatile unsigned int* vgen = &ctl->gen;
-    const unsigned int g = *vgen;
     __threadfence();
-    const unsigned int arrived = atomicAdd(&ctl->count, 1u) + 1u;
-    int ok = 1;
-    if (arrived == gridDim.x) {
-      ctl->count = 0;
-      __threadfence();
-      atomicAdd(&ctl->gen, 1u);
-    } else {
-      uint32_t it = 0;
-      while (*vgen == g) {
-        if (*(volatile int*)err) { ok = 0; break; }
-        if (++it > GRID_SPIN_LIMIT) {
-          atomicExch(err, 2);
-          ok = 0;
-          break;
-        }
+    int ok = atomicAdd(&ctl->count, 1u) + 1u == target;
+    for (uint32_t it = 0; !ok; it++) {
+      ok = (int)(*(volatile unsigned int*)&ctl->count - target) >= 0;
+      if (ok || (it & 63)) continue;
+      if (*(volatile int*)err) break;
+      if (it > GRID_SPIN_LIMIT) {
+        atomicExch(err, 2);
+        break;
       }
     }
     __threadfence();
-    s_ok = ok && *(volatile int*)err == 0;
+    s_ok = ok;
   }
   __syncthreads();
   return s_ok != 0;
@@ -650,49 +643,69 @@ __global__ void jacobi_maxabs(int64_t nn, const double* __restrict__ A, JacobiCt
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) t = fmax(t, sh[w]);
     ctl->amax = t;
     ctl->count = 0;
-    ctl->gen = 0;
     ctl->rot[0] = ctl->rot[1] = 0;
   }
 }
 
-// A0 holds the matrix (it is overwritten), A1 the second buffer, V <- eigenvectors (unsorted),
-// d <- eigenvalues (unsorted, diag of the converged matrix).
-__global__ void __launch_bounds__(256) jacobi_kernel(int n, double* __restrict__ A0, double* __restrict__ A1,
-                                                     double* __restrict__ V, double* __restrict__ d,
-                                                     JacobiCtl* ctl, int* err) {
-  extern __shared__ double s_cs[];  // c[np], s[np]
+// A holds the matrix (overwritten), V <- eigenvectors (unsorted), d <- eigenvalues (unsorted).
+//
+// What bounds it: latency.  A round's rotations act on disjoint index pairs, one grid barrier per
+// round, n - 1 rounds per sweep; the arithmetic of a round is about a microsecond on the whole chip
+// in the first sweeps and next to nothing in the last ones, where few pairs still rotate.  So:
+//  * the 2 x 2 blocks are updated in place.  A thread takes the block (rows of pair R, columns of
+//    pair P) for both orders of P and R, reading and writing only its own four entries (the
+//    matrix is symmetric), lanes along R: coalesced, and no transposed stores.  Both orders
+//    evaluate the same expressions, so the matrix stays exactly symmetric;
+//  * blocks of two pairs that do not rotate, and their columns of V, are left alone;
+//  * what the next round's angles need, the diagonal and the entries of the next pairs, goes to two
+//    small double-buffered arrays: with the circle method next pair i is an entry of the block of
+//    the pairs i - 1 and i + 1 (the first and the last: of their neighbours).
+// With a second matrix written in every round, 64-bit divisions for the indices and a barrier of
+// two words: 351 x 351, 18 sweeps, 69 ms.
+__global__ void __launch_bounds__(JACOBI_THREADS) jacobi_kernel(int n, double* __restrict__ A, double* __restrict__ DO,
+                                                                double* __restrict__ V, double* __restrict__ d,
+                                                                JacobiCtl* ctl, int* err) {
+  extern __shared__ double s_cs[];  // c[np], s[np], then the players of every pair
   __shared__ int s_rot;
   const int np = (n + 1) / 2, np2 = 2 * np;
   double* sc = s_cs;
   double* ss = sc + np;
+  short2* s_pl = reinterpret_cast<short2*>(ss + np);  // (player at position pi, at position np2 - 1 - pi)
   const double eps = 2.2204460492503131e-16;
   const double amax = ctl->amax;
   // entries at or below the rounding level of the matrix (eps max|A|): rounding in the other
   // rotations of their rows regenerates them at that size, so rotating them would never end
   const double tiny = eps * amax;
   const double inv_amax = amax > 0.0 ? 1.0 / amax : 0.0;
-  const int64_t gthreads = (int64_t)gridDim.x * blockDim.x;
-  const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  // V = I
-  for (int64_t e = gtid; e < (int64_t)n * n; e += gthreads) V[e] = (e % n == e / n) ? 1.0 : 0.0;
-  if (!grid_barrier(ctl, err)) return;
-  double* cur = A0;
-  double* nxt = A1;
-  int converged = 0, sweeps_done = 0;
+  const int gthreads = (int)(gridDim.x * blockDim.x), gtid = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int lane = threadIdx.x & 31, gwarp = gtid >> 5, gwarps = gthreads >> 5;
+  double* D[2] = {DO, DO + np2};                    // diagonal
+  double* O[2] = {DO + 2 * np2, DO + 2 * np2 + np};  // entries of the round's pairs
+  for (int e = gtid; e < n * n; e += gthreads) V[e] = (e % n == e / n) ? 1.0 : 0.0;
+  for (int i = gtid; i < np2; i += gthreads) D[0][i] = i < n ? A[i + (size_t)i * n] : 0.0;
+  for (int i = gtid; i < np; i += gthreads) {
+    const int p = rr_player(i, 0, np2), q = rr_player(np2 - 1 - i, 0, np2);
+    O[0][i] = (p < n && q < n) ? A[p + (size_t)q * n] : 0.0;
+  }
+  unsigned int target = gridDim.x;
+  if (!grid_barrier(ctl, target, err)) return;
+  int converged = 0, sweeps_done = 0, b = 0;
+  const int rchunks = (np + 31) / 32, vchunks = (n + 31) / 32;
   for (int sweep = 0; sweep < JACOBI_MAX_SWEEPS && !converged; sweep++) {
     sweeps_done = sweep + 1;
-    for (int round = 0; round < np2 - 1; round++) {
+    for (int round = 0; round < np2 - 1; round++, b ^= 1) {
       if (threadIdx.x == 0) s_rot = 0;
       if (round == 1 && blockIdx.x == 0 && threadIdx.x == 0) ctl->rot[(sweep + 1) & 1] = 0;
       __syncthreads();
-      // rotation of every pair of this round, from the current 2 x 2 diagonal blocks
+      // rotation of every pair of this round, from its 2 x 2 diagonal block
       int myrot = 0;
       for (int pi = threadIdx.x; pi < np; pi += blockDim.x) {
-        int p = rr_player(pi, round, np2), q = rr_player(np2 - 1 - pi, round, np2);
-        if (p > q) { const int t = p; p = q; q = t; }
+        const int p0 = rr_player(pi, round, np2), q0 = rr_player(np2 - 1 - pi, round, np2);
+        s_pl[pi] = make_short2((short)p0, (short)q0);
+        const int p = min(p0, q0), q = max(p0, q0);
         double c = 1.0, s = 0.0;
         if (q < n) {
-          const double apq = cur[p + (size_t)q * n], app = cur[p + (size_t)p * n], aqq = cur[q + (size_t)q * n];
+          const double apq = O[b][pi], app = D[b][p], aqq = D[b][q];
           // skip below the rounding level, or below eps of the diagonal pair (compared squared)
           if (fabs(apq) > tiny && apq * apq > eps * eps * fabs(app) * fabs(aqq)) {
             // the angle in FP32 on entries scaled by 1/max|A| (t = tan(theta) of the rotation that
@@ -720,75 +733,80 @@ __global__ void __launch_bounds__(256) jacobi_kernel(int n, double* __restrict__
       if (blockIdx.x == 0 && myrot) atomicAdd(&s_rot, myrot);
       __syncthreads();
       if (blockIdx.x == 0 && threadIdx.x == 0 && s_rot) atomicAdd(&ctl->rot[sweep & 1], s_rot);
-      // A' = J^T A J by 2 x 2 blocks (pair P rows, pair R columns), P <= R; block (R, P) is
-      // the transpose, written from the same values so the matrix stays exactly symmetric
-      for (int64_t it = gtid; it < (int64_t)np * (np + 1) / 2; it += gthreads) {
-        int R = (int)((sqrtf(8.0f * (float)it + 1.0f) - 1.0f) * 0.5f);  // corrected below
-        while ((int64_t)R * (R + 1) / 2 > it) R--;
-        while ((int64_t)(R + 1) * (R + 2) / 2 <= it) R++;
-        const int P = (int)(it - (int64_t)R * (R + 1) / 2);
-        int p = rr_player(P, round, np2), q = rr_player(np2 - 1 - P, round, np2);
-        int r = rr_player(R, round, np2), s2 = rr_player(np2 - 1 - R, round, np2);
-        if (p > q) { const int t = p; p = q; q = t; }
-        if (r > s2) { const int t = r; r = s2; s2 = t; }
-        const double cP = sc[P], sP = ss[P], cR = sc[R], sR = ss[R];
+      for (int it = gwarp; it < np * rchunks; it += gwarps) {
+        const int P = it / rchunks, R = (it - P * rchunks) * 32 + lane;
+        if (R >= np) continue;
+        const short2 a = s_pl[P], g = s_pl[R];
+        const int p = min((int)a.x, (int)a.y), q = max((int)a.x, (int)a.y);
+        const int r = min((int)g.x, (int)g.y), s2 = max((int)g.x, (int)g.y);
         const bool qv = q < n, sv = s2 < n;
+        const double cP = sc[P], sP = ss[P], cR = sc[R], sR = ss[R];
         if (P == R) {  // diagonal block J^T A_PP J, its off-diagonal entry symmetrised
-          const double app = cur[p + (size_t)p * n];
+          const double app = D[b][p];
           if (!qv) {
-            nxt[p + (size_t)p * n] = app;
+            D[b ^ 1][p] = app;
             continue;
           }
-          const double apq = cur[p + (size_t)q * n], aqq = cur[q + (size_t)q * n];
+          const double apq = O[b][P], aqq = D[b][q];
           const double xpp = cP * app - sP * apq, xpq = cP * apq - sP * aqq;
           const double xqp = sP * app + cP * apq, xqq = sP * apq + cP * aqq;
-          nxt[p + (size_t)p * n] = cP * xpp - sP * xpq;
-          nxt[q + (size_t)q * n] = sP * xqp + cP * xqq;
+          D[b ^ 1][p] = cP * xpp - sP * xpq;
+          D[b ^ 1][q] = sP * xqp + cP * xqq;
           const double bpq = 0.5 * ((sP * xpp + cP * xpq) + (cP * xqp - sP * xqq));
-          nxt[p + (size_t)q * n] = bpq;
-          nxt[q + (size_t)p * n] = bpq;
+          A[p + (size_t)q * n] = bpq;
+          A[q + (size_t)p * n] = bpq;
           continue;
         }
-        const double a_pr = cur[p + (size_t)r * n];
-        const double a_ps = sv ? cur[p + (size_t)s2 * n] : 0.0;
-        const double a_qr = qv ? cur[q + (size_t)r * n] : 0.0;
-        const double a_qs = (qv && sv) ? cur[q + (size_t)s2 * n] : 0.0;
-        // rows: [x_p; x_q] = [[c, -s], [s, c]] [a_p; a_q]
-        const double xpr = cP * a_pr - sP * a_qr, xps = cP * a_ps - sP * a_qs;
-        const double xqr = sP * a_pr + cP * a_qr, xqs = sP * a_ps + cP * a_qs;
-        // columns: [b_r, b_s] = [x_r, x_s] [[c, s], [-s, c]]
-        const double bpr = cR * xpr - sR * xps, bps = sR * xpr + cR * xps;
-        const double bqr = cR * xqr - sR * xqs, bqs = sR * xqr + cR * xqs;
-        nxt[p + (size_t)r * n] = bpr;
-        nxt[r + (size_t)p * n] = bpr;
-        if (sv) {
-          nxt[p + (size_t)s2 * n] = bps;
-          nxt[s2 + (size_t)p * n] = bps;
+        // the block that holds an entry of the next round's pairs (written by one of its two orders)
+        const bool first = P == 0 && R == 1, last = P == np - 2 && R == np - 1;
+        const bool next = R == P + 2 || first || last;
+        if (sP == 0.0 && sR == 0.0 && !next) continue;
+        double* col_p = A + (size_t)p * n;
+        double* col_q = A + (size_t)q * n;
+        // entries (pair P, pair R), whichever of the two is the rows' here
+        double a_pr = col_p[r], a_ps = sv ? col_p[s2] : 0.0;
+        double a_qr = qv ? col_q[r] : 0.0, a_qs = (qv && sv) ? col_q[s2] : 0.0;
+        if (sP != 0.0 || sR != 0.0) {
+          // the pair with the smaller index first, in both orders: x = J_1^T a, b = x J_2
+          const bool sw = P > R;
+          const double c1 = sw ? cR : cP, s1 = sw ? sR : sP, c2 = sw ? cP : cR, s_2 = sw ? sP : sR;
+          const double m01 = sw ? a_qr : a_ps, m10 = sw ? a_ps : a_qr;
+          const double x00 = c1 * a_pr - s1 * m10, x01 = c1 * m01 - s1 * a_qs;
+          const double x10 = s1 * a_pr + c1 * m10, x11 = s1 * m01 + c1 * a_qs;
+          const double b00 = c2 * x00 - s_2 * x01, b01 = s_2 * x00 + c2 * x01;
+          const double b10 = c2 * x10 - s_2 * x11, b11 = s_2 * x10 + c2 * x11;
+          a_pr = b00;
+          a_ps = sw ? b10 : b01;
+          a_qr = sw ? b01 : b10;
+          a_qs = b11;
+          col_p[r] = a_pr;
+          if (sv) col_p[s2] = a_ps;
+          if (qv) col_q[r] = a_qr;
+          if (qv && sv) col_q[s2] = a_qs;
         }
-        if (qv) {
-          nxt[q + (size_t)r * n] = bqr;
-          nxt[r + (size_t)q * n] = bqr;
-        }
-        if (qv && sv) {
-          nxt[q + (size_t)s2 * n] = bqs;
-          nxt[s2 + (size_t)q * n] = bqs;
+        if (next) {
+          // next pair i: of pair i - 1 the player at the high position and of pair i + 1 the one at
+          // the low position; the first: both low, the last: both high
+          const bool lowP = first, lowR = !last;
+          const bool is_q = (lowP ? a.x : a.y) == q, is_s = (lowR ? g.x : g.y) == s2;
+          const int i = first ? 0 : (last ? np - 1 : P + 1);
+          O[b ^ 1][i] = is_q ? (is_s ? a_qs : a_qr) : (is_s ? a_ps : a_pr);
         }
       }
-      // V' = V J, row pairs (each (row, pair) touches its own two entries: in place)
-      for (int64_t it = gtid; it < (int64_t)n * np; it += gthreads) {
-        const int i = (int)(it % n), P = (int)(it / n);
-        if (ss[P] == 0.0) continue;
-        int p = rr_player(P, round, np2), q = rr_player(np2 - 1 - P, round, np2);
-        if (p > q) { const int t = p; p = q; q = t; }
-        if (q >= n) continue;
-        const double vp = V[i + (size_t)p * n], vq = V[i + (size_t)q * n];
-        V[i + (size_t)p * n] = sc[P] * vp - ss[P] * vq;
-        V[i + (size_t)q * n] = ss[P] * vp + sc[P] * vq;
+      // V' = V J, only the columns that rotate
+      for (int it = gwarp; it < np * vchunks; it += gwarps) {
+        const int P = it / vchunks, i = (it - P * vchunks) * 32 + lane;
+        const double s = ss[P];
+        if (s == 0.0 || i >= n) continue;
+        const short2 a = s_pl[P];
+        double* vp = V + i + (size_t)min((int)a.x, (int)a.y) * n;
+        double* vq = V + i + (size_t)max((int)a.x, (int)a.y) * n;
+        const double c = sc[P], x = *vp, y = *vq;
+        *vp = c * x - s * y;
+        *vq = s * x + c * y;
       }
-      if (!grid_barrier(ctl, err)) return;
-      double* t = cur;
-      cur = nxt;
-      nxt = t;
+      target += gridDim.x;
+      if (!grid_barrier(ctl, target, err)) return;
     }
     converged = (*(volatile int*)&ctl->rot[sweep & 1] == 0);
   }
@@ -797,7 +815,7 @@ __global__ void __launch_bounds__(256) jacobi_kernel(int n, double* __restrict__
     if (gtid == 0) atomicExch(err, 1);
     return;
   }
-  for (int64_t i = gtid; i < n; i += gthreads) d[i] = cur[i + (size_t)i * n];
+  for (int i = gtid; i < n; i += gthreads) d[i] = D[b][i];
 }
 
 // w = d ascending (ties by index), V columns permuted the same way (Vu -> V)
@@ -850,19 +868,20 @@ int sym_eig(cudaStream_t st, int n, const double* A, double* V, double* w, doubl
   SS_CUDA_TRY(cudaMemcpyAsync(A0, A, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, st));
   jacobi_maxabs<<<1, 1024, 0, st>>>((int64_t)n * n, A0, ctl);
   SS_CUDA_TRY(cudaGetLastError());
-  // one cooperative grid, all CTAs co-resident
+  // one cooperative grid, all CTAs co-resident: at most one per SM (the barrier gathers them all in
+  // every round), fewer when the blocks of a round do not fill them
   const int np = (n + 1) / 2;
-  const size_t smem = sizeof(double) * 2 * np;
+  const auto smem_of = [](int pairs) { return (sizeof(double) * 2 + sizeof(short2)) * (size_t)pairs; };
+  const size_t smem = smem_of(np);
   SS_CUDA_TRY(cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(double) * 2 * ((4096 + 1) / 2))));  // the largest n
-  int per_sm = 0;
-  SS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, jacobi_kernel, 256, smem));
-  const int64_t items = std::max<int64_t>((int64_t)np * (np + 1) / 2, (int64_t)n * np);  // 2x2 blocks, V rows
-  const int64_t want = std::max<int64_t>(1, (items + 255) / 256);
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sm_count() * std::max(per_sm, 1)));
+                                   (int)smem_of((4096 + 1) / 2)));  // the largest n
+  const int warps = JACOBI_THREADS / 32;
+  const int64_t items = (int64_t)np * ((np + 31) / 32) + (int64_t)np * ((n + 31) / 32);  // of a warp
+  const int64_t want = std::max<int64_t>(1, (items + warps - 1) / warps);
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sm_count()));
   int nn = n;
   void* args[] = {&nn, &A0, &A1, &Vu, &d, &ctl, &d_err};
-  SS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)jacobi_kernel, dim3(grid), dim3(256), args, smem, st));
+  SS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)jacobi_kernel, dim3(grid), dim3(JACOBI_THREADS), args, smem, st));
   eig_sort_kernel<<<n, 128, 0, st>>>(n, d, Vu, w, V);
   SS_CUDA_TRY(cudaGetLastError());
   if (launches) *launches += 3;

@@ -5,7 +5,10 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "mc.cuh"
@@ -371,78 +374,142 @@ static bool same_radial(const ss_ctx* c, int a, int b) {
   return true;
 }
 
+// fn(0), ..., fn(n - 1) over up to eight host threads (the caller's among them); tasks are taken in
+// order from a counter.  Without threads to be had the caller runs them all.
+template <class Fn>
+static void host_parallel(int n, Fn fn) {
+  std::atomic<int> next{0};
+  auto work = [&] {
+    for (int t = next.fetch_add(1); t < n; t = next.fetch_add(1)) fn(t);
+  };
+  std::vector<std::thread> th;
+  const int want = std::min<int>(n, (int)std::min(8u, std::max(1u, std::thread::hardware_concurrency())));
+  try {
+    for (int t = 1; t < want; t++) th.emplace_back(work);
+  } catch (const std::system_error&) {
+  }
+  work();
+  for (std::thread& t : th) t.join();
+}
+
 // Residual tables of the shells (cached per basis): for each shell a cubic Hermite table of
 // delta(t) = u_orb - u_gauss on t = sqrt(r) in [0, t_max], r_max = max(60/zeta, sqrt(60/g_min)),
 // built in FP64.  N starts at 4096 intervals and doubles until the error at every interval
 // midpoint (with the FP32-rounded nodes) is below 1e-6 of the shell's largest |delta|.
-static int build_resid_tables(ss_ctx* c, const std::vector<int>& shell_start, ResidDev* out) {
+//
+// The evaluations (20 exponentials each, about 1.5 ms per shell and 8,193 points on one core) are
+// shared among host threads, and the midpoints of one level are the new nodes of the next, so
+// doubling evaluates the new midpoints only.  A lone atom's job spent 4 of its 6.3 ms here, and the
+// 26-function water's MC began 40 ms late.
+struct ResidLevel {
+  double h, tm;
+  int N = 0;                  // intervals; points k h/2, k = 0..2N: nodes (k even) and midpoints
+  std::vector<double> d, dd;  // delta and d(delta)/dr at the points
+  bool done = false;
+};
+
+static void resid_eval(const ss_ctx* c, int f, double r, double* d, double* dd) {
   const int n = c->n, ld = c->ld;
+  const double zeta = c->h_gs[f];
+  const int k = c->h_nsto[f], ng = c->h_ng[f];
+  const double* c1 = &c->h_cg[(size_t)ld * f];
+  const double* c2 = &c->h_cg[(size_t)ld * (f + n)];
+  const double* g = &c->h_gg[(size_t)ld * f];
+  const double ez = exp(-zeta * r);
+  double rk = 1.0, rk1 = 0.0;  // r^k, k r^(k-1)
+  for (int t = 0; t < k; t++) {
+    rk1 = rk1 * r + rk;
+    rk *= r;
+  }
+  double ug = 0.0, dug = 0.0;
+  for (int m = 0; m < ng; m++) {
+    const double eg = exp(-g[m] * r * r);
+    const double poly = c1[m] + c2[m] * r * r;
+    ug += poly * eg;
+    dug += (2.0 * c2[m] * r - 2.0 * g[m] * r * poly) * eg;
+  }
+  *d = rk * ez - ug;
+  *dd = (rk1 - zeta * rk) * ez - dug;
+}
+
+static int build_resid_tables(ss_ctx* c, const std::vector<int>& shell_start, ResidDev* out) {
+  const int ld = c->ld;
   const int nsh = (int)shell_start.size() - 1;
   if (!c->have_resid) {
     std::vector<float2> node;
     std::vector<int> off(nsh + 1, 0);
     std::vector<float> invh(nsh), tmax(nsh);
+    std::vector<ResidLevel> lev(nsh);
+    std::vector<std::vector<float2>> tab(nsh);
     for (int sh = 0; sh < nsh; sh++) {
       const int f = shell_start[sh];
-      const double zeta = c->h_gs[f];
-      const int k = c->h_nsto[f], ng = c->h_ng[f];
-      const double* c1 = &c->h_cg[(size_t)ld * f];
-      const double* c2 = &c->h_cg[(size_t)ld * (f + n)];
       const double* g = &c->h_gg[(size_t)ld * f];
       double gmin = 1e300;
-      for (int m = 0; m < ng; m++) gmin = std::min(gmin, g[m]);
-      const double rmax = std::max(60.0 / zeta, ng > 0 ? sqrt(60.0 / gmin) : 0.0);
-      const double tm = sqrt(rmax);
-      auto eval = [&](double r, double* d, double* dd) {  // delta and d(delta)/dr
-        const double ez = exp(-zeta * r);
-        double rk = 1.0, rk1 = 0.0;  // r^k, k r^(k-1)
-        for (int t = 0; t < k; t++) {
-          rk1 = rk1 * r + rk;
-          rk *= r;
+      for (int m = 0; m < c->h_ng[f]; m++) gmin = std::min(gmin, g[m]);
+      lev[sh].tm = sqrt(std::max(60.0 / c->h_gs[f], c->h_ng[f] > 0 ? sqrt(60.0 / gmin) : 0.0));
+    }
+    constexpr int CHUNK = 512;  // points of a task
+    for (int N = 4096;; N *= 2) {
+      struct Task { int sh, k0, k1; };
+      std::vector<Task> tasks;
+      for (int sh = 0; sh < nsh; sh++) {
+        ResidLevel& V = lev[sh];
+        if (V.done) continue;
+        // the points known so far are the even ones of this level
+        std::vector<double> d(2 * (size_t)N + 1), dd(2 * (size_t)N + 1);
+        for (size_t k = 0; k < V.d.size(); k++) {
+          d[2 * k] = V.d[k];
+          dd[2 * k] = V.dd[k];
         }
-        double ug = 0.0, dug = 0.0;
-        for (int m = 0; m < ng; m++) {
-          const double eg = exp(-g[m] * r * r);
-          const double poly = c1[m] + c2[m] * r * r;
-          ug += poly * eg;
-          dug += (2.0 * c2[m] * r - 2.0 * g[m] * r * poly) * eg;
+        const bool first = V.d.empty();
+        V.d.swap(d);
+        V.dd.swap(dd);
+        V.N = N;
+        V.h = V.tm / N;
+        for (int k = 0; k <= 2 * N; k += CHUNK) tasks.push_back(Task{first ? sh : sh - nsh, k, std::min(k + CHUNK, 2 * N + 1)});
+      }
+      if (tasks.empty()) break;
+      host_parallel((int)tasks.size(), [&](int x) {
+        const Task& T = tasks[x];
+        const bool odd = T.sh < 0;  // only the new (odd) points
+        ResidLevel& V = lev[odd ? T.sh + nsh : T.sh];
+        const int f = shell_start[odd ? T.sh + nsh : T.sh];
+        for (int k = T.k0; k < T.k1; k++) {
+          if (odd && !(k & 1)) continue;
+          const double t = k * (0.5 * V.h);
+          resid_eval(c, f, t * t, &V.d[k], &V.dd[k]);
         }
-        *d = rk * ez - ug;
-        *dd = (rk1 - zeta * rk) * ez - dug;
-      };
-      std::vector<float2> tab;
-      double h = 0.0;
-      for (int N = 4096;; N *= 2) {
-        h = tm / N;
-        tab.resize(N + 1);
+      });
+      for (int sh = 0; sh < nsh; sh++) {
+        ResidLevel& V = lev[sh];
+        if (V.done) continue;
+        std::vector<float2>& tb = tab[sh];
+        tb.resize(N + 1);
         double dmax = 0.0;
         for (int j = 0; j <= N; j++) {
-          const double t = j * h;
-          double d, dd;
-          eval(t * t, &d, &dd);
-          tab[j] = make_float2((float)d, (float)(h * 2.0 * t * dd));
-          dmax = std::max(dmax, fabs(d));
+          const double t = j * V.h;
+          tb[j] = make_float2((float)V.d[2 * j], (float)(V.h * 2.0 * t * V.dd[2 * j]));
+          dmax = std::max(dmax, fabs(V.d[2 * j]));
         }
         double emax = 0.0;
         for (int j = 0; j < N; j++) {
-          const double t = (j + 0.5) * h;
-          double d, dd;
-          eval(t * t, &d, &dd);
-          const double interp = 0.5 * ((double)tab[j].x + (double)tab[j + 1].x) +
-                                0.125 * ((double)tab[j].y - (double)tab[j + 1].y);
-          emax = std::max(emax, fabs(interp - d));
+          const double interp = 0.5 * ((double)tb[j].x + (double)tb[j + 1].x) +
+                                0.125 * ((double)tb[j].y - (double)tb[j + 1].y);
+          emax = std::max(emax, fabs(interp - V.d[2 * j + 1]));
         }
-        if (emax <= 1e-6 * dmax || dmax == 0.0) break;
-        if (N >= 65536) {
+        V.done = emax <= 1e-6 * dmax || dmax == 0.0;
+        if (!V.done && N >= 65536) {
           ss_set_error_msg("shared estimator: the fit residual of function %d is not resolved by a "
-                           "65536-interval table (error %.3g of its maximum)", f + 1, emax / dmax);
+                           "65536-interval table (error %.3g of its maximum)", shell_start[sh] + 1, emax / dmax);
           return SS_ERR_UNSUPPORTED;
         }
       }
+    }
+    for (int sh = 0; sh < nsh; sh++) {
       off[sh] = (int)node.size();
-      node.insert(node.end(), tab.begin(), tab.end());
-      invh[sh] = (float)(1.0 / h);
-      tmax[sh] = (float)tm;
+      node.insert(node.end(), tab[sh].begin(), tab[sh].end());
+      invh[sh] = (float)(1.0 / lev[sh].h);
+      tmax[sh] = (float)lev[sh].tm;
     }
     off[nsh] = (int)node.size();
     float2* dn;
