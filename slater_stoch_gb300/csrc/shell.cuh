@@ -102,6 +102,7 @@ struct ShPair {
   int onec, fold, same_system;
   int64_t prim_off, e_off;           // first primitive; first Hermite coefficient
   double pmax;                       // largest exponent sum of its primitives
+  int col[5];                        // where ShArgs::col has this pair type's columns as the ket, by bra degree
 };
 
 // A primitive pair: exponent sum, centre, w = K_AB c_a c_b / p, and (sorted tables) the largest
@@ -145,6 +146,7 @@ struct ShArgs {
   const float2* E2;      // the same as two floats
   const double* scale;   // power of two of each pair's w in primf
   const ShBoys* boys;    // [SH_MAXL + 1]
+  const uint8_t* col;    // columns of t + tau of every bra degree and pair type (ShPair::col)
   const ShStruct* st;
   const ShWork* work;
   const int* cta;        // work entry of each CTA of the chunk
@@ -160,9 +162,17 @@ constexpr int SH_MAXSLICE = 16;  // bra primitives of a slice
 
 cudaError_t launch_shell_eri(int L, int ncta, int max_no, int max_ni, int max_col, cudaStream_t st, const ShArgs& A);
 
+// Bytes of the columns [ket term][bra Hermite function] of a bra degree and a pair type: indices of
+// t + tau, in multiples of 16 bytes
+__host__ __device__ constexpr int sh_col_size(int d, int nterm) { return (sh_nherm(d) * nterm + 15) / 16 * 16; }
+
 // Lane kernels (shell_lane.cuh): bra degree DB, ket type; a CTA takes SH_LANE_BRA bra primitives (one
-// per thread), SH_LANE_KET ket primitives and one chunk of the ket's components.
-constexpr int SH_LANE_BRA = 128, SH_LANE_KET = 64;
+// per thread), sh_lane_kets ket primitives and one chunk of the ket's components.  Fewer kets where a
+// ket costs more: on a small system the longest CTA is the stage, and its start-up (the Boys table)
+// is about one ket's work there (7-function water 1.64 ms with 64 kets at every L, 1.40 ms with 32
+// from L = 3; 26-function water 44.3 ms with both).
+constexpr int SH_LANE_BRA = 128;
+constexpr int sh_lane_kets(int L) { return L >= 3 ? 32 : 64; }
 // ket components per chunk for a bra of degree db and a ket type (ta, tb), 0: no such kernel
 constexpr int sh_lane_chunk(int db, int ta, int tb) {
   const int k = ta * (ta + 1) / 2 + tb;  // SS PS PP RS RP RR DS DP DR DD

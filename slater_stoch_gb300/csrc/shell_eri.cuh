@@ -269,9 +269,11 @@ struct ShDim {
   static constexpr int NB = L >= 5 ? 64 : 128;
   static constexpr int MINB = L >= 6 ? 2 : 4;  // CTAs per SM the registers must allow
   static constexpr int ROW = sh_nherm(L) | 1;  // odd: a column over the items meets no bank twice
+  static_assert(NB % 2 == 0, "the columns after the rows begin on 16 bytes");
+  // max_col: a multiple of 16
   static size_t bytes(int max_no, int max_ni, int max_col) {
     return sizeof(float) * SH_BOYS_K * SH_BOYS_ROW +
-           sizeof(double) * ((size_t)NB * ROW + (max_no > NT ? max_no : NT) + max_ni) + ((size_t)max_col + 15) / 16 * 16;
+           sizeof(double) * ((size_t)NB * ROW + (max_no > NT ? max_no : NT) + max_ni) + (size_t)max_col;
   }
 };
 
@@ -281,15 +283,15 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
   extern __shared__ float4 sh_raw[];
   float* s_boys = reinterpret_cast<float*>(sh_raw);                          // [SH_BOYS_K][SH_BOYS_ROW]
   double* s_R = reinterpret_cast<double*>(s_boys + SH_BOYS_K * SH_BOYS_ROW);  // [NB][ROW]: double, df or float
-  double* s_acc = s_R + (size_t)NB * ROW;         // [group][bra Hermite][ket component]: double or df
+  uint8_t* s_col = reinterpret_cast<uint8_t*>(s_R + (size_t)NB * ROW);  // [ket term][bra Hermite]: column of t + tau
+  double* s_acc = reinterpret_cast<double*>(s_col + max_col);  // [group][bra Hermite][ket component]: double or df
   double* s_out = s_acc + (max_no > NT ? max_no : NT);
-  uint8_t* s_col = reinterpret_cast<uint8_t*>(s_out + max_ni);  // [ket term][bra Hermite]: column of t + tau
   __shared__ int s_scan[3][SH_MAXSLICE + 1], s_first[3][SH_MAXSLICE], s_p[SH_MAXSLICE];
   const int tid = threadIdx.x;
   {  // the launch's dynamic shared memory must hold this carve-up: checked, not assumed
     uint32_t dyn;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-    if (reinterpret_cast<char*>(s_col + max_col) - reinterpret_cast<char*>(sh_raw) > (ptrdiff_t)dyn) return;
+    if (reinterpret_cast<char*>(s_out + max_ni) - reinterpret_cast<char*>(sh_raw) > (ptrdiff_t)dyn) return;
   }
 
   const ShWork W = A.work[A.cta[A.cta0 + blockIdx.x]];
@@ -306,7 +308,7 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
                     bra[0].P[2] == ket[0].P[2];
   const int H = sh_nherm(B.d), nf = K.ncomp, NO = H * nf, NI = B.ncomp * nf, nterm = K.nterm;
   const uint64_t mask = W.mask;
-  if (NO > (max_no > NT ? max_no : NT) || NI > max_ni || H * nterm > max_col || B.d + K.d != L) return;  // uniform
+  if (NO > (max_no > NT ? max_no : NT) || NI > max_ni || sh_col_size(B.d, nterm) > max_col || B.d + K.d != L) return;  // uniform
 
   // the tiers below FP64 of a quartet with a lane kernel are that kernel's
   const int tiers = diag || W.lane >= 0 ? 1 : 3;
@@ -315,9 +317,10 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
     const float4* src = reinterpret_cast<const float4*>(boys->f);
     for (int i = tid; i < SH_BOYS_K * SH_BOYS_ROW / 4; i += NT) sh_raw[i] = src[i];
   }
-  for (int i = tid; i < H * nterm; i += NT) {
-    const int x = i / H;
-    s_col[i] = (uint8_t)sh_pack_idx(SK.term[x] + sh_hermite[i - x * H]);
+  {
+    const uint4* src = reinterpret_cast<const uint4*>(A.col + K.col[B.d]);
+    uint4* dst = reinterpret_cast<uint4*>(s_col);
+    for (int i = tid; i < sh_col_size(B.d, nterm) / 16; i += NT) dst[i] = src[i];
   }
   for (int i = tid; i < NI; i += NT) s_out[i] = 0.0;
 

@@ -163,7 +163,8 @@ struct LaneDim {
   static constexpr int MINB = L >= 4 || H >= 10 ? 2 : 3;
   // shared memory: Boys table, ket records and coefficients, then the sums G of the four warps in
   // the place of the ket's
-  static constexpr size_t ket_bytes = SH_LANE_KET * (sizeof(ShPrimF) + sizeof(float2) * KET::S.nterm);
+  static constexpr int KETS = sh_lane_kets(L);
+  static constexpr size_t ket_bytes = KETS * (sizeof(ShPrimF) + sizeof(float2) * KET::S.nterm);
 };
 
 template <class KET, int DB, int F0, int NF, bool ONE4>
@@ -173,10 +174,11 @@ __device__ __forceinline__ void lane_body(const ShArgs& A, const ShWork& W, int 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const ShPair B = A.pair[W.bra], K = A.pair[W.ket];
   const int nb = A.cnt[W.bra], nk = A.cnt[W.ket];
-  const int p0 = blk * SH_LANE_BRA, k0 = kc * SH_LANE_KET, k1 = min(nk, k0 + SH_LANE_KET);
+  constexpr int KETS = LaneDim<KET, DB>::KETS;
+  const int p0 = blk * SH_LANE_BRA, k0 = kc * KETS, k1 = min(nk, k0 + KETS);
   const int p = p0 + tid;
   ShPrimF* s_ket = reinterpret_cast<ShPrimF*>(s_mem);
-  float2* s_E = reinterpret_cast<float2*>(s_ket + SH_LANE_KET);
+  float2* s_E = reinterpret_cast<float2*>(s_ket + KETS);
   df* s_G = reinterpret_cast<df*>(s_mem) + warp * (H * NF * 33);  // [t * NF + f][lane], after the kets
   const ShPrim* bra = A.prim + B.prim_off;
   const ShPrim* ket = A.prim + K.prim_off;

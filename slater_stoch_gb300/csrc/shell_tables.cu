@@ -40,6 +40,8 @@ static int struct_index(int ta, int tb, bool same, bool onec) {
 
 struct StructTable {
   std::vector<ShStruct> s;
+  std::vector<uint8_t> col;         // ShArgs::col
+  int off[SH_NSTRUCT][5] = {};
   StructTable() : s(SH_NSTRUCT) {
     for (int ta = 0; ta < 4; ta++)
       for (int tb = 0; tb <= ta; tb++)
@@ -48,6 +50,20 @@ struct StructTable {
       s[struct_index(SH_P, SH_P, true, oc)] = sh_struct(SH_P, SH_P, true, oc);
       s[struct_index(SH_D, SH_D, true, oc)] = sh_struct(SH_D, SH_D, true, oc);
     }
+    for (int st = 0; st < SH_NSTRUCT; st++)
+      for (int d = 0; d < 5; d++) {
+        const ShStruct& S = s[st];
+        off[st][d] = (int)col.size();
+        col.resize(col.size() + sh_col_size(d, S.nterm));
+        for (int x = 0; x < S.nterm; x++)
+          for (int n = 0, t = 0; n <= d; n++)  // bra Hermite functions in the order of sh_hidx
+            for (int w = 0; w <= n; w++)
+              for (int v = 0; v <= w; v++, t++) {
+                const uint32_t tm = S.term[x];
+                col[off[st][d] + x * sh_nherm(d) + t] = (uint8_t)sh_hidx(
+                    n - w + (int)(tm & 255), w - v + (int)((tm >> 8) & 255), v + (int)(tm >> 16));
+              }
+      }
   }
 };
 static const StructTable& structs() {
@@ -158,17 +174,20 @@ __global__ void __launch_bounds__(256) shell_fill(BasisDev B, const ShPair* __re
   if (threadIdx.x == 0) out.cnt[blockIdx.x] = s_total;
 }
 
-// sum of the partial sums of every element, in their order
-__global__ void shell_reduce(int nwork, const ShWork* __restrict__ work, const ShPair* __restrict__ pairs, int diag,
-                             const double* __restrict__ part, double* __restrict__ elem) {
+// sum of the partial sums of every element: one warp per element, lane sums and a shuffle tree
+__global__ void __launch_bounds__(256) shell_reduce(int nwork, const ShWork* __restrict__ work,
+                                                    const ShPair* __restrict__ pairs, int diag,
+                                                    const double* __restrict__ part, double* __restrict__ elem) {
   const ShWork W = work[blockIdx.x];
   const int ni = diag ? pairs[W.bra].ncomp : pairs[W.bra].ncomp * pairs[W.ket].ncomp;
-  for (int e = threadIdx.x; e < ni; e += blockDim.x) {
-    const int n = W.split + W.lsplit;
+  const int n = W.split + W.lsplit, lane = threadIdx.x & 31;
+  for (int e = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5); e < ni; e += gridDim.y * (blockDim.x >> 5)) {
     const double* p = part + W.part + (int64_t)e * n;
     double v = 0.0;
-    for (int s = 0; s < n; s++) v = v + p[s];
-    elem[W.elem + e] = v;
+    for (int s = lane; s < n; s += 32) v = v + p[s];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) elem[W.elem + e] = v;
   }
 }
 
@@ -204,6 +223,12 @@ __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pai
       const double* e = E + P.e_off + (size_t)t * P.nterm;
       // (P|P): both on one centre at exponent p/2, so R_{2a 2b 2c} = (2a-1)!!(2b-1)!!(2c-1)!! (-p)^n / (2n+1)
       const double pre = 34.9868366552 * a.w * a.w * rsqrt(a.p + a.p);
+      double pw[SH_MAXL / 2 + 1];
+      pw[0] = 1.0;
+#pragma unroll
+      for (int n = 1; n <= SH_MAXL / 2; n++) pw[n] = pw[n - 1] * -a.p;
+#pragma unroll
+      for (int n = 1; n <= SH_MAXL / 2; n++) pw[n] *= 1.0 / (2 * n + 1);
       key = 0.0;
       for (int f = 0; f < S.ncomp; f++) {
         double v = 0.0;
@@ -213,15 +238,15 @@ __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pai
             const uint32_t h = S.term[x] + S.term[y];
             if (h & 0x010101u) continue;
             const int hx = h & 255, hy = (h >> 8) & 255, hz = h >> 16;
-            double r = 1.0;
-            for (int i = hx - 1; i > 1; i -= 2) r *= i;
-            for (int i = hy - 1; i > 1; i -= 2) r *= i;
-            for (int i = hz - 1; i > 1; i -= 2) r *= i;
+            // (2a-1)!! = 1, 1, 3, 15, 105
+            auto dfact = [](int e) { return e <= 2 ? 1.f : e == 4 ? 3.f : e == 6 ? 15.f : 105.f; };
             const int n = (hx + hy + hz) / 2;
-            for (int i = 0; i < n; i++) r *= -a.p;
-            r /= 2 * n + 1;
+            double r = pw[0];
+#pragma unroll
+            for (int t = 1; t <= SH_MAXL / 2; t++) r = t == n ? pw[t] : r;
             const int dy = (S.term[y] & 255) + ((S.term[y] >> 8) & 255) + (S.term[y] >> 16);
-            row = fma((dy & 1) ? -r : r, e[y], row);
+            const float c = dfact(hx) * dfact(hy) * dfact(hz);
+            row = fma(r * (double)((dy & 1) ? -c : c), e[y], row);
           }
           v = fma(row, e[x], v);
         }
@@ -412,6 +437,7 @@ void build_shells(ss_ctx* c) {
       P.d = S.d;
       P.ncomp = S.ncomp;
       P.nterm = S.nterm;
+      for (int d = 0; d < 5; d++) P.col[d] = structs().off[P.st][d];
       const int na = c->h_ng[P.fa], nb = c->h_ng[P.fb];
       P.cap = P.fold ? na * (na + 1) / 2 : na * nb;
       P.pmax = *std::max_element(&c->h_gg[(size_t)ld * P.fa], &c->h_gg[(size_t)ld * P.fa] + na) +
@@ -476,14 +502,15 @@ static double side_cost(const ShPair& b, const ShPair& k) {
   return c ? herm * ((k.ncomp + c - 1) / c) + 12.2 * terms : herm + 18.0 * terms + 1500.0;
 }
 
-// bra slices of a shell quartet in the shared kernel: a CTA's bra primitives so that it has about
-// 1e6 multiply-adds at a hundred kept kets each (16 where it only has the FP64 tier), at most
-// SH_MAXSLICE of them; never from what else is in the list, so that the order of summation is the
-// quartet's own
+// bra slices of a shell quartet in the shared kernel: two to eight bra primitives per CTA (about 1e6
+// multiply-adds at a hundred kept kets each), 16 where it only has the FP64 tier; never from what
+// else is in the list, so that the order of summation is the quartet's own.  On a small system the
+// longest CTA is the stage, on a large one a CTA's start-up counts: at most 4, 8, 16 primitives took
+// 2.37, 2.43, 2.50 ms for the oxygen atom and 45.0, 44.3, 44.0 ms for the 26-function water.
 static int slices(const ShPair& b, const ShPair& k, bool lane) {
   const int L = b.d + k.d;
   const double cost = 30.0 + 4.0 * L + SH_REC[L] + (double)sh_nherm(b.d) * k.nterm;
-  const int per = lane ? SH_MAXSLICE : (int)std::min((double)SH_MAXSLICE, std::max(2.0, 1e4 / cost));
+  const int per = lane ? SH_MAXSLICE : (int)std::min(8.0, std::max(2.0, 1e4 / cost));
   return std::max(1, (b.cap + per - 1) / per);
 }
 
@@ -540,6 +567,7 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
     A.E2 = E2;
     A.scale = (const double*)c->pool["shell_scale"].ptr;
     A.boys = (const ShBoys*)c->pool["shell_boys"].ptr;
+    A.col = (const uint8_t*)c->pool["shell_col"].ptr;
     A.partial = (double*)dp;
     A.eps = eps;
     A.eps32 = eps32;
@@ -571,7 +599,7 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
     }
     const int jrc = join_eri_streams(c);
     if (rc || jrc) return rc ? rc : jrc;
-    shell_reduce<<<(unsigned)chunk.size(), 64, 0, c->stream>>>((int)chunk.size(), (const ShWork*)dw, A.pair, diag,
+    shell_reduce<<<dim3((unsigned)chunk.size(), 4), 256, 0, c->stream>>>((int)chunk.size(), (const ShWork*)dw, A.pair, diag,
                                                                (const double*)dp, elem);
     SS_CUDA_TRY(cudaGetLastError());
     c->launches++;
@@ -608,7 +636,7 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
       g.ncta += w.split;
       g.no = std::max(g.no, sh_nherm(b.d) * k.ncomp);
       g.ni = std::max(g.ni, ni);
-      g.col = std::max(g.col, sh_nherm(b.d) * k.nterm);
+      g.col = std::max(g.col, sh_col_size(b.d, k.nterm));
       ncta += w.split;
       nlane += w.nlane;
       part += need;
@@ -624,9 +652,13 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
   const int np = (int)T.pair.size();
   if (!np) return SS_OK;
   void* p;
-  TRY(pool_get(c, "shell_struct", sizeof(ShStruct) * SH_NSTRUCT, &p));
-  TRY(h2d_copy(c, p, structs().s.data(), sizeof(ShStruct) * SH_NSTRUCT));
-  const ShStruct* st = (const ShStruct*)p;
+  if (!c->pool["shell_struct"].ptr) {  // constants, once per context
+    TRY(pool_get(c, "shell_struct", sizeof(ShStruct) * SH_NSTRUCT, &p));
+    TRY(h2d_copy(c, p, structs().s.data(), sizeof(ShStruct) * SH_NSTRUCT));
+    TRY(pool_get(c, "shell_col", structs().col.size(), &p));
+    TRY(h2d_copy(c, p, structs().col.data(), structs().col.size()));
+  }
+  const ShStruct* st = (const ShStruct*)c->pool["shell_struct"].ptr;
   TRY(h2d_async(c, c->pool["shell_pair"], T.pair.data(), sizeof(ShPair) * np));
   const ShPair* dpair = (const ShPair*)c->pool["shell_pair"].ptr;
   ShFill F;
@@ -661,7 +693,7 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
     if (!P.same_system) continue;
     ShWork w{};
     w.bra = w.ket = x;
-    w.split = slices(P, P, false);
+    w.split = std::max(1, (P.cap + 1) / 2);  // two bra primitives: few quartets, in FP64
     w.lane = -1;
     w.elem = (int64_t)x * SH_MAXCOMP;
     w.mask = ~0ull;
@@ -741,7 +773,8 @@ int shell_plan(ss_ctx* c, bool tiers, const std::vector<int64_t>& sel, std::vect
       bool all = b.onec && k.onec;
       for (int ax = 0; ax < 3; ax++) all = all && c->h_center[3 * b.fa + ax] == c->h_center[3 * k.fa + ax];
       w.lane = 8 * k.st + b.d + (all ? SH_LANE_ONEC : 0);
-      w.nkc = (k.cap + SH_LANE_KET - 1) / SH_LANE_KET;
+      const int kets = sh_lane_kets(b.d + k.d);
+      w.nkc = (k.cap + kets - 1) / kets;
       w.lsplit = w.nkc * ((b.cap + SH_LANE_BRA - 1) / SH_LANE_BRA);
       w.nlane = w.lsplit * ((k.ncomp + chunk - 1) / chunk);
     }
