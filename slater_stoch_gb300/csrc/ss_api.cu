@@ -98,10 +98,10 @@ void dev_free(ss_ctx* c, DevBuf& b) {
   b.bytes = 0;
 }
 
-// Copies up to STAGE_MAX go through a pinned ring (a wrap waits for the copies still in it);
+// Copies up to STAGE_MAX (half of it) go through a pinned ring (a wrap waits for the copies still in it);
 // larger ones are rare and wait for the stream instead.
 int h2d_copy(ss_ctx* c, void* dst, const void* src, size_t bytes) {
-  constexpr size_t STAGE_CAP = (size_t)4 << 20, STAGE_MAX = (size_t)1 << 20;
+  constexpr size_t STAGE_CAP = (size_t)1 << 20, STAGE_MAX = STAGE_CAP / 2;
   if (bytes == 0) return SS_OK;
   if (bytes > STAGE_MAX) {
     SS_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
