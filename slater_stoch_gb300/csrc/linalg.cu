@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(256) sym_eig_smem_kernel(int n, const double* 
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t GRID_SPIN_LIMIT = 1u << 22;  // bounded grid barrier (seconds of L2 polling; a round takes microseconds)
 constexpr int JACOBI_MAX_SWEEPS = 40;
-constexpr int JACOBI_THREADS = 512;
+constexpr int JACOBI_THREADS = 256;  // measured on 351 x 351: 256 threads 40.8 ms, 512 46.6 ms, 1024 67.4 ms
 
 struct JacobiCtl {
   unsigned int count;       // grid barrier: arrivals since the start
