@@ -72,121 +72,174 @@ __device__ __forceinline__ double u_gauss(const BasisDev& B, int i, double r) {
   return u;
 }
 
-__device__ __forceinline__ void pair_density(const BasisDev& B, int i, int k, const double (&u)[3],
-                                             double& rS, double& rG) {
-  const double* ci = B.center + 3 * i;
-  const double* ck = B.center + 3 * k;
-  double dx = u[0] - ci[0], dy = u[1] - ci[1], dz = u[2] - ci[2];
-  double poly_i = 1.0;
-  for (int t = 0; t < B.npower[3 * i]; t++) poly_i = poly_i * dx;
-  for (int t = 0; t < B.npower[3 * i + 1]; t++) poly_i = poly_i * dy;
-  for (int t = 0; t < B.npower[3 * i + 2]; t++) poly_i = poly_i * dz;
-  const double r_i = sqrt(dx * dx + dy * dy + dz * dz);
-  dx = u[0] - ck[0]; dy = u[1] - ck[1]; dz = u[2] - ck[2];
-  double poly_k = 1.0;
-  for (int t = 0; t < B.npower[3 * k]; t++) poly_k = poly_k * dx;
-  for (int t = 0; t < B.npower[3 * k + 1]; t++) poly_k = poly_k * dy;
-  for (int t = 0; t < B.npower[3 * k + 2]; t++) poly_k = poly_k * dz;
-  const double r_k = sqrt(dx * dx + dy * dy + dz * dz);
-  const double poly_ik = poly_i * poly_k;
-  rS = poly_ik * u_orb(B.n_sto[i], B.g_slater[i], r_i) * u_orb(B.n_sto[k], B.g_slater[k], r_k);
-  rG = poly_ik * u_gauss(B, i, r_i) * u_gauss(B, k, r_k);
+// distance from the function's centre
+__device__ __forceinline__ double centre_offset(const BasisDev& B, int f, const double (&u)[3], double (&d)[3]) {
+  const double* c = B.center + 3 * f;
+#pragma unroll
+  for (int l = 0; l < 3; l++) d[l] = u[l] - c[l];
+  return sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
 }
 
-// One thread per (walker, used pair): ZV map (src/two_e_slater.F90:406-411), densities,
-// Jacobians (src/compute_jacobian_and_pi0.F90:22-30).  FP64 mode folds the Jacobians and
-// 1/pi_0 into the density columns; REF32 mode keeps them apart for the single-precision
-// weight of src/two_e_slater.F90:442.
+__device__ __forceinline__ double poly(const BasisDev& B, int f, const double (&d)[3]) {
+  double v = 1.0;
+#pragma unroll
+  for (int l = 0; l < 3; l++)
+    for (int t = 0; t < B.npower[3 * f + l]; t++) v = v * d[l];
+  return v;
+}
+
+// One thread per (walker, pair group): ZV map (src/two_e_slater.F90:406-411), densities,
+// Jacobians (src/compute_jacobian_and_pi0.F90:22-30).  The pairs of a group, all components of two
+// shells, share the map and the radial parts (20 exponentials each in FP64, the cost of this
+// kernel, whose FP64 pipe is 85 % busy); with one thread per pair the 26-function water evaluated
+// them 3.9 times as often (16,000 walkers: 5.0 ms).
+// FP64 mode folds the Jacobians and 1/pi_0 into the density columns; REF32 mode keeps them apart
+// for the single-precision weight of src/two_e_slater.F90:442.
 template <int MODE>
 __global__ void zv_pair_kernel(BasisDev B, ZvPairs P, int64_t S, const double* __restrict__ r1,
                                const double* __restrict__ r2, const double* __restrict__ r1m,
                                const double* __restrict__ r2m, const double* __restrict__ pi0,
                                ZvChunk Z) {
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int p = blockIdx.y;
+  const int g = blockIdx.y;
   if (s >= S) return;
-  const int i = P.i[p], k = P.k[p];
-  const double fzv = P.fzv[p], fjac = P.fjac[p];
-  const double a1 = r1m[s], a2 = r2m[s];
-  double u1[3], u2[3];
+  const int i = P.i[g], k = P.k[g];
+  const bool same = P.same[g] != 0;
+  const double fzv = P.fzv[g], fjac = P.fjac[g];
+  const int64_t og = (int64_t)g * Z.ld + s;
 #pragma unroll
-  for (int l = 0; l < 3; l++) {
-    u1[l] = fzv * r1[3 * s + l] * a1 + P.G[3 * p + l];
-    u2[l] = fzv * r2[3 * s + l] * a2 + P.G[3 * p + l];
-  }
-  double rs1, rg1, rs2, rg2;
-  pair_density(B, i, k, u1, rs1, rg1);
-  pair_density(B, i, k, u2, rs2, rg2);
-  const double f1 = fjac * a1, f2 = fjac * a2;
-  const double j1 = 0.25 * fabs(f1 * f1 * f1);
-  const double j2 = 0.25 * fabs(f2 * f2 * f2);
-  const int64_t o = (int64_t)p * Z.ld + s;
-  Z.u1x[o] = u1[0]; Z.u1y[o] = u1[1]; Z.u1z[o] = u1[2];
-  Z.u2x[o] = u2[0]; Z.u2y[o] = u2[1]; Z.u2z[o] = u2[2];
-  if (MODE == SS_PREC_FP64) {
-    const double ip = 1.0 / pi0[s];
-    Z.a_s[o] = j1 * rs1;
-    Z.a_g[o] = j1 * rg1;
-    Z.b_s[o] = j2 * rs2 * ip;
-    Z.b_g[o] = j2 * rg2 * ip;
-  } else {
-    Z.a_s[o] = rs1;
-    Z.a_g[o] = rg1;
-    Z.b_s[o] = rs2;
-    Z.b_g[o] = rg2;
-    Z.j1[o] = j1;
-    Z.j2[o] = j2;
+  for (int e = 0; e < 2; e++) {
+    const double* r = e == 0 ? r1 : r2;
+    const double am = e == 0 ? r1m[s] : r2m[s];
+    double u[3];
+#pragma unroll
+    for (int l = 0; l < 3; l++) u[l] = fzv * r[3 * s + l] * am + P.G[3 * g + l];
+    (e == 0 ? Z.u1x : Z.u2x)[og] = u[0];
+    (e == 0 ? Z.u1y : Z.u2y)[og] = u[1];
+    (e == 0 ? Z.u1z : Z.u2z)[og] = u[2];
+    const double f = fjac * am;
+    const double jac = 0.25 * fabs(f * f * f);
+    double di[3], dk[3];
+    const double ri = centre_offset(B, i, u, di), rk = centre_offset(B, k, u, dk);
+    const double so = u_orb(B.n_sto[i], B.g_slater[i], ri), go = u_gauss(B, i, ri);
+    const double so2 = same ? so : u_orb(B.n_sto[k], B.g_slater[k], rk);
+    const double go2 = same ? go : u_gauss(B, k, rk);
+    if (MODE != SS_PREC_FP64) (e == 0 ? Z.j1 : Z.j2)[og] = jac;
+    const double ip = e == 0 ? 1.0 : 1.0 / pi0[s];
+    for (int x = P.first[g]; x < P.first[g + 1]; x++) {
+      const int p = P.order[x];
+      const double poly_ik = poly(B, P.pi[p], di) * poly(B, P.pk[p], dk);
+      double rs = poly_ik * so * so2, rg = poly_ik * go * go2;
+      if (MODE == SS_PREC_FP64) {
+        rs = jac * rs;
+        rg = jac * rg;
+        if (e == 1) {
+          rs = rs * ip;
+          rg = rg * ip;
+        }
+      }
+      const int64_t o = (int64_t)p * Z.ld + s;
+      (e == 0 ? Z.a_s : Z.b_s)[o] = rs;
+      (e == 0 ? Z.a_g : Z.b_g)[o] = rg;
+    }
   }
 }
 
-// Accumulation (src/two_e_slater.F90:424-453).  One CTA per (bra pair, walker slice); each
-// warp takes the quartets of the bra pair in turn, lanes stride over walkers.  Each
-// quartet is summed by a single warp, so partials are deterministic.
+// Accumulation (src/two_e_slater.F90:424-453).  One warp per (tile of quartets, walker slice); lanes
+// stride over the walkers, so every quartet's partial sums have a fixed order.
+//
+// The FP64 pipe bounds it (two lanes per clock and SM).  A quartet and walker on their own cost it
+// about 20 operations, 16 of them r12 and its inverse root; these are the same for all quartets of a
+// tile, and the products with them for its quartets of one ket (FP64) or bra pair (REF32).  The
+// 26-function water's 61,776 quartets make about 5,800 tiles: 4 operations each.  16,000 walkers:
+// 54 -> 13 ms (a warp per quartet before); the order of every sum is unchanged.
 template <int MODE>
-__global__ void __launch_bounds__(256) zv_accum_kernel(int64_t S, ZvCsr Q, int nsplit, ZvChunk Z,
-                                                       const double* __restrict__ pi0,
-                                                       double* __restrict__ partS,
-                                                       double* __restrict__ partG) {
-  const int b = blockIdx.x / nsplit, sp = blockIdx.x % nsplit;
-  const int p1 = Q.bra[b];
-  const int64_t e0 = Q.off[b], e1 = Q.off[b + 1];
+__global__ void __launch_bounds__(128, 2) zv_accum_kernel(int64_t S, ZvTiles Q, int nsplit, ZvChunk Z,
+                                                          const double* __restrict__ pi0,
+                                                          double* __restrict__ partS,
+                                                          double* __restrict__ partG) {
+  const int64_t item = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, sp = (int)(item % nsplit);
+  if (item / nsplit >= Q.n) return;
+  const ZvTile& T = Q.tile[item / nsplit];
   const int64_t per = (S + nsplit - 1) / nsplit;
   const int64_t w0 = sp * per, w1 = min(S, w0 + per);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-  const int64_t o1 = (int64_t)p1 * Z.ld;
-  for (int64_t e = e0 + warp; e < e1; e += nwarp) {
-    const int64_t q = Q.q[e];
-    const int64_t o2 = (int64_t)Q.ket[e] * Z.ld;
-    double sS = 0.0, sG = 0.0;
-    for (int64_t s = w0 + lane; s < w1; s += 32) {
-      const double dx = Z.u1x[o1 + s] - Z.u2x[o2 + s];
-      const double dy = Z.u1y[o1 + s] - Z.u2y[o2 + s];
-      const double dz = Z.u1z[o1 + s] - Z.u2z[o2 + s];
-      const double r12_2 = dx * dx + dy * dy + dz * dz;
-      if (MODE == SS_PREC_FP64) {
-        const double inv = rsqrt(r12_2);
-        sS = fma(Z.a_s[o1 + s], Z.b_s[o2 + s] * inv, sS);
-        sG = fma(Z.a_g[o1 + s], Z.b_g[o2 + s] * inv, sG);
-      } else {
-        const double rj = Z.j1[o1 + s] * Z.j2[o2 + s];
-        const double factor = (double)(__fdiv_rn((float)rj, (float)pi0[s]));
-        const double inv = (double)(__fdiv_rn(1.0f, __fsqrt_rn((float)r12_2)));
-        const double wS = factor * Z.a_s[o1 + s] * Z.b_s[o2 + s];
-        const double wG = factor * Z.a_g[o1 + s] * Z.b_g[o2 + s];
-        sS = sS + wS * inv;
-        sG = sG + wG * inv;
+  const int64_t g1 = (int64_t)T.g1 * Z.ld, g2 = (int64_t)T.g2 * Z.ld;
+  const uint64_t mask = T.mask;
+  double sS[ZV_TB][ZV_TK], sG[ZV_TB][ZV_TK];
+  int bra[ZV_TB], ket[ZV_TK];
+#pragma unroll
+  for (int t = 0; t < ZV_TB; t++) bra[t] = T.bra[t];
+#pragma unroll
+  for (int u = 0; u < ZV_TK; u++) ket[u] = T.ket[u];
+#pragma unroll
+  for (int t = 0; t < ZV_TB; t++)
+#pragma unroll
+    for (int u = 0; u < ZV_TK; u++) sS[t][u] = sG[t][u] = 0.0;
+  for (int64_t s = w0 + lane; s < w1; s += 32) {
+    const double dx = Z.u1x[g1 + s] - Z.u2x[g2 + s];
+    const double dy = Z.u1y[g1 + s] - Z.u2y[g2 + s];
+    const double dz = Z.u1z[g1 + s] - Z.u2z[g2 + s];
+    const double r12_2 = dx * dx + dy * dy + dz * dz;
+    double inv, factor = 1.0;
+    if (MODE == SS_PREC_FP64) {
+      inv = rsqrt(r12_2);
+    } else {
+      const double rj = Z.j1[g1 + s] * Z.j2[g2 + s];
+      factor = (double)(__fdiv_rn((float)rj, (float)pi0[s]));
+      inv = (double)(__fdiv_rn(1.0f, __fsqrt_rn((float)r12_2)));
+    }
+    double aS[ZV_TB], aG[ZV_TB];
+#pragma unroll
+    for (int t = 0; t < ZV_TB; t++) {
+      aS[t] = aG[t] = 0.0;
+      if (bra[t] >= 0) {
+        aS[t] = Z.a_s[(int64_t)bra[t] * Z.ld + s];
+        aG[t] = Z.a_g[(int64_t)bra[t] * Z.ld + s];
+        if (MODE != SS_PREC_FP64) {
+          aS[t] = factor * aS[t];
+          aG[t] = factor * aG[t];
+        }
       }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sS += __shfl_down_sync(0xffffffffu, sS, o);
-      sG += __shfl_down_sync(0xffffffffu, sG, o);
-    }
-    if (lane == 0) {
-      partS[q * nsplit + sp] = sS;
-      partG[q * nsplit + sp] = sG;
+    for (int u = 0; u < ZV_TK; u++) {
+      if (ket[u] < 0) continue;
+      double bS = Z.b_s[(int64_t)ket[u] * Z.ld + s], bG = Z.b_g[(int64_t)ket[u] * Z.ld + s];
+      if (MODE == SS_PREC_FP64) {
+        bS = bS * inv;
+        bG = bG * inv;
+      }
+#pragma unroll
+      for (int t = 0; t < ZV_TB; t++) {
+        if (!(mask >> (t * ZV_TK + u) & 1)) continue;
+        if (MODE == SS_PREC_FP64) {
+          sS[t][u] = fma(aS[t], bS, sS[t][u]);
+          sG[t][u] = fma(aG[t], bG, sG[t][u]);
+        } else {
+          sS[t][u] = sS[t][u] + aS[t] * bS * inv;
+          sG[t][u] = sG[t][u] + aG[t] * bG * inv;
+        }
+      }
     }
   }
+  const int64_t* q = Q.q + T.q;
+#pragma unroll
+  for (int t = 0; t < ZV_TB; t++)
+#pragma unroll
+    for (int u = 0; u < ZV_TK; u++) {
+      if (!(mask >> (t * ZV_TK + u) & 1)) continue;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        sS[t][u] += __shfl_down_sync(0xffffffffu, sS[t][u], o);
+        sG[t][u] += __shfl_down_sync(0xffffffffu, sG[t][u], o);
+      }
+      if (lane == 0) {
+        partS[*q * nsplit + sp] = sS[t][u];
+        partG[*q * nsplit + sp] = sG[t][u];
+      }
+      q++;
+    }
 }
 
 __global__ void zv_reduce_partials(int64_t nint, int nsplit, const double* __restrict__ partS,
@@ -250,10 +303,10 @@ cudaError_t launch_walker_aux(cudaStream_t st, int64_t S, const double* r1, cons
   return cudaGetLastError();
 }
 
-cudaError_t launch_zv_pairs(cudaStream_t st, int mode, const BasisDev& B, const ZvPairs& P, int npairs,
+cudaError_t launch_zv_pairs(cudaStream_t st, int mode, const BasisDev& B, const ZvPairs& P,
                             int64_t S, const double* r1, const double* r2, const double* r1m,
                             const double* r2m, const double* pi0, const ZvChunk& Z) {
-  dim3 grid((unsigned)((S + 127) / 128), (unsigned)npairs);
+  dim3 grid((unsigned)((S + 127) / 128), (unsigned)P.ngroups);
   if (mode == SS_PREC_FP64)
     zv_pair_kernel<SS_PREC_FP64><<<grid, 128, 0, st>>>(B, P, S, r1, r2, r1m, r2m, pi0, Z);
   else
@@ -261,13 +314,14 @@ cudaError_t launch_zv_pairs(cudaStream_t st, int mode, const BasisDev& B, const 
   return cudaGetLastError();
 }
 
-cudaError_t launch_zv_accum(cudaStream_t st, int mode, int nbra, int nsplit, int64_t S, const ZvCsr& Q,
+cudaError_t launch_zv_accum(cudaStream_t st, int mode, int nsplit, int64_t S, const ZvTiles& Q,
                             const ZvChunk& Z, const double* pi0, double* partS, double* partG) {
-  dim3 grid((unsigned)(nbra * nsplit));
+  if (Q.n <= 0) return cudaSuccess;
+  dim3 grid((unsigned)(((int64_t)Q.n * nsplit + 3) / 4));
   if (mode == SS_PREC_FP64)
-    zv_accum_kernel<SS_PREC_FP64><<<grid, 256, 0, st>>>(S, Q, nsplit, Z, pi0, partS, partG);
+    zv_accum_kernel<SS_PREC_FP64><<<grid, 128, 0, st>>>(S, Q, nsplit, Z, pi0, partS, partG);
   else
-    zv_accum_kernel<SS_PREC_REF32><<<grid, 256, 0, st>>>(S, Q, nsplit, Z, pi0, partS, partG);
+    zv_accum_kernel<SS_PREC_REF32><<<grid, 128, 0, st>>>(S, Q, nsplit, Z, pi0, partS, partG);
   return cudaGetLastError();
 }
 

@@ -3,6 +3,10 @@
 #include <string.h>
 
 #include <algorithm>
+#include <array>
+#include <map>
+#include <numeric>
+#include <utility>
 #include <vector>
 
 #include "mc.cuh"
@@ -13,6 +17,7 @@
 namespace ss {
 
 int ensure_mono(ss_ctx* c);
+bool same_radial(const ss_ctx* c, int a, int b);  // shared.cu: centre, exponents and fit of two functions
 int launch_combine_mono(ss_ctx* c, double* out);
 
 __global__ void combine_kernel(int64_t nint, const double* __restrict__ g, const double* __restrict__ m,
@@ -88,6 +93,63 @@ static int upload(ss_ctx* c, const char* name, const std::vector<T>& v, T** out)
   return SS_OK;
 }
 
+// Tiles of the quartets, those with the most quartets first (the last CTAs are then short ones).
+// Bra and ket blocks: ZV_TB (ZV_TK) consecutive pairs of a group in the order of `order`.
+static void build_tiles(const PairPlan& P, const std::vector<int>& group, const std::vector<int>& first,
+                        const std::vector<int>& order, std::vector<ZvTile>& tiles, std::vector<int64_t>& tile_q) {
+  const int np = P.npairs, ng = (int)first.size() - 1;
+  std::vector<int> pos(np), row(np, -1), kblk(ng + 1, 0);
+  for (int g = 0; g < ng; g++) {
+    for (int x = first[g]; x < first[g + 1]; x++) pos[order[x]] = x - first[g];
+    kblk[g + 1] = kblk[g] + (first[g + 1] - first[g] + ZV_TK - 1) / ZV_TK;
+  }
+  for (int b = 0; b < P.nbra; b++) row[P.bra[b]] = b;
+  std::vector<int> open(kblk[ng], -1);  // tile that takes the quartets of the current bra block and a ket block
+  std::vector<std::array<int64_t, ZV_TB * ZV_TK>> q;
+  for (int g = 0; g < ng; g++)
+    for (int x0 = first[g]; x0 < first[g + 1]; x0 += ZV_TB) {
+      const size_t begin = tiles.size();
+      for (int x = x0; x < std::min(x0 + ZV_TB, first[g + 1]); x++) {
+        const int p1 = order[x];
+        if (row[p1] < 0) continue;
+        for (int64_t e = P.off[row[p1]]; e < P.off[row[p1] + 1]; e++) {
+          const int p2 = P.ket[e], g2 = group[p2], t = x - x0, u = pos[p2] % ZV_TK;
+          const uint64_t bit = (uint64_t)1 << (t * ZV_TK + u);
+          int& o = open[kblk[g2] + pos[p2] / ZV_TK];
+          if (o < (int)begin || (tiles[o].mask & bit)) {  // none yet, or a quartet listed twice
+            ZvTile T{};
+            T.g1 = g;
+            T.g2 = g2;
+            std::fill(T.bra, T.bra + ZV_TB, -1);
+            std::fill(T.ket, T.ket + ZV_TK, -1);
+            o = (int)tiles.size();
+            tiles.push_back(T);
+            q.emplace_back();
+          }
+          tiles[o].mask |= bit;
+          tiles[o].bra[t] = p1;
+          tiles[o].ket[u] = p2;
+          q[o][t * ZV_TK + u] = P.q[e];
+        }
+      }
+    }
+  std::vector<int> by(tiles.size());
+  std::iota(by.begin(), by.end(), 0);
+  std::stable_sort(by.begin(), by.end(), [&](int a, int b) {
+    return __builtin_popcountll(tiles[a].mask) > __builtin_popcountll(tiles[b].mask);
+  });
+  std::vector<ZvTile> sorted;
+  sorted.reserve(tiles.size());
+  tile_q.reserve(P.q.size());
+  for (int o : by) {
+    sorted.push_back(tiles[o]);
+    sorted.back().q = (int64_t)tile_q.size();
+    for (int s = 0; s < ZV_TB * ZV_TK; s++)
+      if (tiles[o].mask >> s & 1) tile_q.push_back(q[o][s]);
+  }
+  tiles.swap(sorted);
+}
+
 // Faithful estimator over blocks; walkers from Philox(seed) or from host arrays hr1/hr2.
 static int run_faithful(ss_ctx* c, double a_zv, uint64_t seed, const double* hr1, const double* hr2,
                         int64_t npts, int nblocks, int prec, double sigma_target) {
@@ -98,32 +160,70 @@ static int run_faithful(ss_ctx* c, double a_zv, uint64_t seed, const double* hr1
   PairPlan P;
   build_pair_plan(c, P);
   const int np = P.npairs;
-  std::vector<double> G(3 * (size_t)np), fzv(np), fjac(np);
-  for (int p = 0; p < np; p++) {
-    int i = P.pi[p], k = P.pk[p];
-    double gi = c->h_gs[i], gk = c->h_gs[k];
-    for (int l = 0; l < 3; l++)  // src/two_e_slater.F90:344
-      G[3 * p + l] = (gi * c->h_center[l + 3 * i] + gk * c->h_center[l + 3 * k]) / (gi + gk);
-    fzv[p] = 0.5 * a_zv / (gi + gk);  // :406
-    fjac[p] = a_zv / (gi + gk);       // src/compute_jacobian_and_pi0.F90:22
+  // radial id of every function (centre, exponents and fit), and the groups of pairs that share the
+  // radial ids of both functions
+  std::vector<int> rad(c->n, -1), rep;
+  for (int f = 0; f < c->n; f++) {
+    for (size_t r = 0; r < rep.size() && rad[f] < 0; r++)
+      if (same_radial(c, f, rep[r])) rad[f] = (int)r;
+    if (rad[f] < 0) {
+      rad[f] = (int)rep.size();
+      rep.push_back(f);
+    }
   }
-  ZvPairs dP;
-  ZvCsr dQ;
+  std::map<std::pair<int, int>, int> where;
+  std::vector<int> gi, gk, same, group(np), first, order(np);
+  for (int p = 0; p < np; p++) {
+    const auto key = std::make_pair(rad[P.pi[p]], rad[P.pk[p]]);
+    const auto it = where.emplace(key, (int)gi.size());
+    if (it.second) {
+      gi.push_back(P.pi[p]);
+      gk.push_back(P.pk[p]);
+      same.push_back(key.first == key.second);
+    }
+    group[p] = it.first->second;
+  }
+  const int ng = (int)gi.size();
+  first.assign(ng + 1, 0);
+  for (int p = 0; p < np; p++) first[group[p] + 1]++;
+  for (int g = 0; g < ng; g++) first[g + 1] += first[g];
   {
-    int *pi, *pk, *bra, *ket;
+    std::vector<int> at(first.begin(), first.end() - 1);
+    for (int p = 0; p < np; p++) order[at[group[p]]++] = p;
+  }
+  std::vector<double> G(3 * (size_t)ng), fzv(ng), fjac(ng);
+  for (int p = 0; p < ng; p++) {
+    int i = gi[p], k = gk[p];
+    const double zi = c->h_gs[i], zk = c->h_gs[k];
+    for (int l = 0; l < 3; l++)  // src/two_e_slater.F90:344
+      G[3 * p + l] = (zi * c->h_center[l + 3 * i] + zk * c->h_center[l + 3 * k]) / (zi + zk);
+    fzv[p] = 0.5 * a_zv / (zi + zk);  // :406
+    fjac[p] = a_zv / (zi + zk);       // src/compute_jacobian_and_pi0.F90:22
+  }
+  std::vector<ZvTile> tiles;
+  std::vector<int64_t> tile_q;
+  build_tiles(P, group, first, order, tiles, tile_q);
+  ZvPairs dP;
+  ZvTiles dQ;
+  {
+    int *di, *dk, *dsame, *dfirst, *dorder, *pi, *pk;
     double *dG, *dfzv, *dfjac;
-    int64_t *off, *q;
+    int64_t* q;
+    ZvTile* tile;
+    TRY(upload(c, "zv_gi", gi, &di));
+    TRY(upload(c, "zv_gk", gk, &dk));
+    TRY(upload(c, "zv_same", same, &dsame));
+    TRY(upload(c, "zv_first", first, &dfirst));
+    TRY(upload(c, "zv_order", order, &dorder));
     TRY(upload(c, "zv_pi", P.pi, &pi));
     TRY(upload(c, "zv_pk", P.pk, &pk));
     TRY(upload(c, "zv_G", G, &dG));
     TRY(upload(c, "zv_fzv", fzv, &dfzv));
     TRY(upload(c, "zv_fjac", fjac, &dfjac));
-    TRY(upload(c, "zv_bra", P.bra, &bra));
-    TRY(upload(c, "zv_off", P.off, &off));
-    TRY(upload(c, "zv_q", P.q, &q));
-    TRY(upload(c, "zv_ket", P.ket, &ket));
-    dP = ZvPairs{pi, pk, dG, dfzv, dfjac};
-    dQ = ZvCsr{bra, off, q, ket};
+    TRY(upload(c, "zv_tile", tiles, &tile));
+    TRY(upload(c, "zv_q", tile_q, &q));
+    dP = ZvPairs{ng, di, dk, dsame, dfirst, dorder, pi, pk, dG, dfzv, dfjac};
+    dQ = ZvTiles{(int)tiles.size(), tile, q};
   }
   // chunk size: ~1 GiB of pair columns
   const int ncols = (prec == SS_PREC_FP64) ? 10 : 12;
@@ -136,6 +236,7 @@ static int run_faithful(ss_ctx* c, double a_zv, uint64_t seed, const double* hr1
   ZvChunk Z{};
   Z.ld = Sc;
   double** fields[12] = {&Z.u1x, &Z.u1y, &Z.u1z, &Z.u2x, &Z.u2y, &Z.u2z, &Z.a_s, &Z.a_g, &Z.b_s, &Z.b_g, &Z.j1, &Z.j2};
+  // coordinates and Jacobians per group, densities per pair (at most as many groups as pairs)
   for (int f = 0; f < ncols; f++) *fields[f] = cols + (size_t)f * np * Sc;
   double *r1, *r2, *r1m, *r2m, *pi0;
   TRY(pool_get(c, "zv_r1", sizeof(double) * 3 * Sc, &buf)); r1 = (double*)buf;
@@ -175,8 +276,8 @@ static int run_faithful(ss_ctx* c, double a_zv, uint64_t seed, const double* hr1
         c->launches++;
       }
       CUTRY(launch_walker_aux(c->stream, ns, r1, r2, r1m, r2m, pi0));
-      CUTRY(launch_zv_pairs(c->stream, prec, c->basis, dP, np, ns, r1, r2, r1m, r2m, pi0, Z));
-      CUTRY(launch_zv_accum(c->stream, prec, P.nbra, nsplit, ns, dQ, Z, pi0, partS, partG));
+      CUTRY(launch_zv_pairs(c->stream, prec, c->basis, dP, ns, r1, r2, r1m, r2m, pi0, Z));
+      CUTRY(launch_zv_accum(c->stream, prec, nsplit, ns, dQ, Z, pi0, partS, partG));
       CUTRY(launch_zv_reduce(c->stream, nint, nsplit, partS, partG, eS, eG));
       c->launches += 4;
     }

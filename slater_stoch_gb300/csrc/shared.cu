@@ -359,7 +359,7 @@ struct SharedPlan {
   ResidDev resid{};
 };
 
-static bool same_radial(const ss_ctx* c, int a, int b) {
+bool same_radial(const ss_ctx* c, int a, int b) {
   if (c->h_nsto[a] != c->h_nsto[b] || c->h_itype[a] != c->h_itype[b] || c->h_ng[a] != c->h_ng[b] ||
       c->h_gs[a] != c->h_gs[b])
     return false;
