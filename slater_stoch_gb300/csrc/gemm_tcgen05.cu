@@ -185,10 +185,12 @@ __global__ void __launch_bounds__(128, 1)
         mma_bf16(tmem, ahi, blo, 1u);
         mma_bf16(tmem, alo, bhi, 1u);
       }
-      mma_commit(&empty_bar[s]);  // frees the stage once these MMAs have read it
+      // frees the stage once these MMAs have read it.  Not for the last stages, which the producer
+      // does not fill again: nobody would wait for the arrival, and none may be under way when the
+      // CTA exits and hands its shared memory to the next one (waiting for them at the end took 1 us)
+      if (t + STAGES < nkt) mma_commit(&empty_bar[s]);
     }
-    // arrives once every issued MMA has completed; an empty K slice commits nothing, so that no
-    // arrival can be under way when its CTA exits and hands its shared memory to the next one
+    // arrives once every issued MMA has completed; an empty K slice commits nothing
     if (nkt > 0) mma_commit(acc_bar);
   }
   __syncwarp();
@@ -223,14 +225,6 @@ __global__ void __launch_bounds__(128, 1)
       }
     }
   }
-  // nor may one of the stage commits that the producer had no reason to wait for
-  if (warp == 1 && lane == 0 && !*(volatile int*)&s_abort) {
-    for (int s = 0; s < STAGES && s < nkt; s++) {
-      const int t = nkt - 1 - ((nkt - 1 - s) % STAGES);
-      if (!mbar_wait(&empty_bar[s], (uint32_t)((t / STAGES) & 1))) atomicExch(err, ERR_EMPTY_WAIT);
-    }
-  }
-  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   // After an abort, TMA loads the MMA warp never consumed may still be writing into shared
