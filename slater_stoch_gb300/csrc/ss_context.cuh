@@ -65,10 +65,16 @@ struct ss_ctx {
   void* pin = nullptr;
   size_t pin_cap = 0;
   cudaEvent_t pin_evt = nullptr;
-  // pinned staging ring of h2d_copy, and the last copy out of it on each stream
+  // pinned staging ring of h2d_copy (two halves), the half in use and its fill, and per stream that
+  // copied from it the work queued when each half was left last
+  struct StageStream {
+    cudaStream_t stream;
+    cudaEvent_t left[2];
+  };
   char* stage = nullptr;
   size_t stage_off = 0;
-  std::vector<std::pair<cudaStream_t, cudaEvent_t>> stage_evt;
+  int stage_half = 0;
+  std::vector<StageStream> stage_evt;
   int64_t launches = 0;
   int num_sms = 0;
 
