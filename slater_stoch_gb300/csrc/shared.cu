@@ -241,62 +241,74 @@ __device__ __forceinline__ void store_bf16(__nv_bfloat16* dst, const __nv_bfloat
   }
 }
 
-template <int V>
-__global__ void shared_operand_kernel(int64_t S, int64_t Kh, int64_t ld, int n, const int* __restrict__ pi,
-                                      const int* __restrict__ pk, const float* __restrict__ F,
-                                      const float* __restrict__ w, __nv_bfloat16* __restrict__ Ahi,
-                                      __nv_bfloat16* __restrict__ Alo, __nv_bfloat16* __restrict__ Bhi,
-                                      __nv_bfloat16* __restrict__ Blo) {
+// A CTA forms `np` consecutive pairs of one block of samples: consecutive pairs share the function i,
+// whose values stay in registers.  With one pair per CTA the kernel read 44 bytes of orbital values
+// from L2 for every 16 bytes that it wrote, and its writes ran at 4.8 TB/s.
+template <int V, bool ONE>
+__global__ void shared_operand_kernel(int64_t S, int64_t Kh, int64_t ld, int n, int P, int np,
+                                      const int* __restrict__ pi, const int* __restrict__ pk,
+                                      const float* __restrict__ F, const float* __restrict__ w,
+                                      __nv_bfloat16* __restrict__ Ahi, __nv_bfloat16* __restrict__ Alo,
+                                      __nv_bfloat16* __restrict__ Bhi, __nv_bfloat16* __restrict__ Blo) {
   // pairs along x: consecutive CTAs read the orbital values of the same samples, which stay in
   // L2 while all pairs use them (with samples along x the whole sub-chunk's values, 24 n bytes
   // per sample, streamed through L2 once per pair)
   const int64_t s0 = (blockIdx.y * (int64_t)blockDim.x + threadIdx.x) * V;
-  const int p = blockIdx.x;
   if (s0 >= Kh) return;
-  float d1[V], g1[V], s2w[V], d2w[V];
+  const int64_t plane = (int64_t)n * ld, K = 2 * Kh;
+  const bool in = s0 < S;
+  float ww[V], a1S[V], a1G[V], a1D[V], a2S[V], a2D[V];
+  if (in) VecF<V>::load(w + s0, ww);
+  int i = -1;
+  const int p1 = ONE ? blockIdx.x + 1 : min(P, ((int)blockIdx.x + 1) * np);
+#pragma unroll 2
+  for (int p = ONE ? blockIdx.x : blockIdx.x * np; p < p1; p++) {
+    float d1[V], g1[V], s2w[V], d2w[V];
 #pragma unroll
-  for (int e = 0; e < V; e++) d1[e] = g1[e] = s2w[e] = d2w[e] = 0.f;
-  if (s0 < S) {
-    const int i = pi[p], k = pk[p];
-    const int64_t plane = (int64_t)n * ld;
-    const int64_t oi = (int64_t)i * ld + s0, ok = (int64_t)k * ld + s0;
-    float a1S[V], a1G[V], a1D[V], b1G[V], b1D[V], a2S[V], a2D[V], b2S[V], b2G[V], b2D[V], ww[V];
-    VecF<V>::load(F + oi, a1S);
-    VecF<V>::load(F + plane + oi, a1G);
-    VecF<V>::load(F + 2 * plane + oi, a1D);
-    VecF<V>::load(F + plane + ok, b1G);
-    VecF<V>::load(F + 2 * plane + ok, b1D);
-    VecF<V>::load(F + 3 * plane + oi, a2S);
-    VecF<V>::load(F + 5 * plane + oi, a2D);
-    VecF<V>::load(F + 3 * plane + ok, b2S);
-    VecF<V>::load(F + 4 * plane + ok, b2G);
-    VecF<V>::load(F + 5 * plane + ok, b2D);
-    VecF<V>::load(w + s0, ww);
+    for (int e = 0; e < V; e++) d1[e] = g1[e] = s2w[e] = d2w[e] = 0.f;
+    if (in) {
+      const int k = pk[p];
+      if (ONE || pi[p] != i) {
+        i = pi[p];
+        const int64_t oi = (int64_t)i * ld + s0;
+        VecF<V>::load(F + oi, a1S);
+        VecF<V>::load(F + plane + oi, a1G);
+        VecF<V>::load(F + 2 * plane + oi, a1D);
+        VecF<V>::load(F + 3 * plane + oi, a2S);
+        VecF<V>::load(F + 5 * plane + oi, a2D);
+      }
+      float b1G[V], b1D[V], b2S[V], b2G[V], b2D[V];
+      const int64_t ok = (int64_t)k * ld + s0;
+      VecF<V>::load(F + plane + ok, b1G);
+      VecF<V>::load(F + 2 * plane + ok, b1D);
+      VecF<V>::load(F + 3 * plane + ok, b2S);
+      VecF<V>::load(F + 4 * plane + ok, b2G);
+      VecF<V>::load(F + 5 * plane + ok, b2D);
 #pragma unroll
-    for (int e = 0; e < V; e++) {
-      if (s0 + e >= S) break;  // samples past the sub-chunk's end stay zero
-      // rhoS - rhoG = phiS_i delta_k + delta_i phiG_k (exact identity, no cancellation)
-      d1[e] = fmaf(a1S[e], b1D[e], a1D[e] * b1G[e]);
-      g1[e] = a1G[e] * b1G[e];
-      s2w[e] = (a2S[e] * b2S[e]) * ww[e];
-      d2w[e] = fmaf(a2S[e], b2D[e], a2D[e] * b2G[e]) * ww[e];
+      for (int e = 0; e < V; e++) {
+        if (s0 + e >= S) break;  // samples past the sub-chunk's end stay zero
+        // rhoS - rhoG = phiS_i delta_k + delta_i phiG_k (exact identity, no cancellation)
+        d1[e] = fmaf(a1S[e], b1D[e], a1D[e] * b1G[e]);
+        g1[e] = a1G[e] * b1G[e];
+        s2w[e] = (a2S[e] * b2S[e]) * ww[e];
+        d2w[e] = fmaf(a2S[e], b2D[e], a2D[e] * b2G[e]) * ww[e];
+      }
     }
+    const int64_t r = (int64_t)p * K + s0;
+    __nv_bfloat16 h[V], l[V];
+#pragma unroll
+    for (int e = 0; e < V; e++) split_bf16(d1[e], h[e], l[e]);
+    store_bf16<V>(Ahi + r, h); store_bf16<V>(Alo + r, l);
+#pragma unroll
+    for (int e = 0; e < V; e++) split_bf16(g1[e], h[e], l[e]);
+    store_bf16<V>(Ahi + r + Kh, h); store_bf16<V>(Alo + r + Kh, l);
+#pragma unroll
+    for (int e = 0; e < V; e++) split_bf16(s2w[e], h[e], l[e]);
+    store_bf16<V>(Bhi + r, h); store_bf16<V>(Blo + r, l);
+#pragma unroll
+    for (int e = 0; e < V; e++) split_bf16(d2w[e], h[e], l[e]);
+    store_bf16<V>(Bhi + r + Kh, h); store_bf16<V>(Blo + r + Kh, l);
   }
-  const int64_t K = 2 * Kh;
-  const int64_t r = (int64_t)p * K + s0;
-  __nv_bfloat16 h[V], l[V];
-#pragma unroll
-  for (int e = 0; e < V; e++) split_bf16(d1[e], h[e], l[e]);
-  store_bf16<V>(Ahi + r, h); store_bf16<V>(Alo + r, l);
-#pragma unroll
-  for (int e = 0; e < V; e++) split_bf16(g1[e], h[e], l[e]);
-  store_bf16<V>(Ahi + r + Kh, h); store_bf16<V>(Alo + r + Kh, l);
-#pragma unroll
-  for (int e = 0; e < V; e++) split_bf16(s2w[e], h[e], l[e]);
-  store_bf16<V>(Bhi + r, h); store_bf16<V>(Blo + r, l);
-#pragma unroll
-  for (int e = 0; e < V; e++) split_bf16(d2w[e], h[e], l[e]);
-  store_bf16<V>(Bhi + r + Kh, h); store_bf16<V>(Blo + r + Kh, l);
 }
 
 // Cblk[P][P] (double) += sum over K slices of the fp32 partial products.  The slices are summed
@@ -670,6 +682,12 @@ int run_shared(ss_ctx* c, double a_zv, uint64_t seed, int64_t npts, int nblocks,
   TRY(dev_alloc(c, c->d_mean, sizeof(double) * nint));
   TRY(dev_alloc(c, c->d_sigma, sizeof(double) * nint));
   const int64_t PP = (int64_t)P * P;
+  // pairs per CTA of the operand kernel: up to 8, fewer where the grid would fall below 24 CTAs
+  // per SM (26 functions, 2^22 walker pairs: 15.4, 14.4, 13.9, 13.5, 13.6, 13.9 ms of MC with 1, 2, 4, 8,
+  // 16, 27; 14.5 with the kernel of one pair)
+  constexpr int64_t SH_OP_PAIRS = 8;
+  const int64_t op_blocks = (Kh / 4 + 255) / 256;
+  const int np = (int)std::min<int64_t>(SH_OP_PAIRS, std::max<int64_t>(1, P * op_blocks / (24 * c->num_sms)));
   int done = 0;
   for (int b = 0; b < nblocks; b++) {
     SS_CUDA_TRY(cudaMemsetAsync(Cblk, 0, sizeof(double) * PP, c->stream));
@@ -681,10 +699,15 @@ int run_shared(ss_ctx* c, double a_zv, uint64_t seed, int64_t npts, int nblocks,
       shared_fn_density_kernel<<<dim3((unsigned)((ns + 127) / 128), (unsigned)(SP.shell_start.size() - 1)), 128, 0,
                                  c->stream>>>(c->basis, ns, ldF, SP.d_shell, SP.resid, SP.d_Ahl, smp, F);
       SS_CUDA_TRY(cudaGetLastError());
-      // four samples per thread (8-byte stores): per job 0.263 s of MC with one, 0.245 s with
-      // two, 0.226 s with four, 0.262 s with eight
-      shared_operand_kernel<4><<<dim3((unsigned)P, (unsigned)((Kh / 4 + 255) / 256)), 256, 0, c->stream>>>(
-          ns, Kh, ldF, n, SP.d_pi, SP.d_pk, F, w, Ahi, Alo, Bhi, Blo);
+      // four samples per thread (8-byte stores): with one pair per CTA, 0.263 s of MC per job with
+      // one, 0.245 s with two, 0.226 s with four, 0.262 s with eight
+      const dim3 op_grid((unsigned)((P + np - 1) / np), (unsigned)op_blocks);
+      if (np == 1)
+        shared_operand_kernel<4, true><<<op_grid, 256, 0, c->stream>>>(ns, Kh, ldF, n, P, 1, SP.d_pi, SP.d_pk, F, w,
+                                                                        Ahi, Alo, Bhi, Blo);
+      else
+        shared_operand_kernel<4, false><<<op_grid, 256, 0, c->stream>>>(ns, Kh, ldF, n, P, np, SP.d_pi, SP.d_pk, F, w,
+                                                                         Ahi, Alo, Bhi, Blo);
       SS_CUDA_TRY(cudaGetLastError());
       TRY(launch_split_bf16_gemm(c->stream, Ahi, Alo, Bhi, Blo, P, K, ksplit, Cp, err));
       shared_accumulate_block<<<(unsigned)((PP + 255) / 256), 256, 0, c->stream>>>(P, ksplit, Cp, Cblk);
