@@ -88,7 +88,7 @@ __device__ __forceinline__ double poly(const BasisDev& B, int f, const double (&
   return v;
 }
 
-// One thread per (walker, pair group): ZV map (src/two_e_slater.F90:406-411), densities,
+// One thread per (walker, pair group, electron): ZV map (src/two_e_slater.F90:406-411), densities,
 // Jacobians (src/compute_jacobian_and_pi0.F90:22-30).  The pairs of a group, all components of two
 // shells, share the map and the radial parts (20 exponentials each in FP64, the cost of this
 // kernel, whose FP64 pipe is 85 % busy); with one thread per pair the 26-function water evaluated
@@ -107,41 +107,39 @@ __global__ void zv_pair_kernel(BasisDev B, ZvPairs P, int64_t S, const double* _
   const bool same = P.same[g] != 0;
   const double fzv = P.fzv[g], fjac = P.fjac[g];
   const int64_t og = (int64_t)g * Z.ld + s;
+  const int e = blockIdx.z;
+  const double* r = e == 0 ? r1 : r2;
+  const double am = e == 0 ? r1m[s] : r2m[s];
+  double u[3];
 #pragma unroll
-  for (int e = 0; e < 2; e++) {
-    const double* r = e == 0 ? r1 : r2;
-    const double am = e == 0 ? r1m[s] : r2m[s];
-    double u[3];
-#pragma unroll
-    for (int l = 0; l < 3; l++) u[l] = fzv * r[3 * s + l] * am + P.G[3 * g + l];
-    (e == 0 ? Z.u1x : Z.u2x)[og] = u[0];
-    (e == 0 ? Z.u1y : Z.u2y)[og] = u[1];
-    (e == 0 ? Z.u1z : Z.u2z)[og] = u[2];
-    const double f = fjac * am;
-    const double jac = 0.25 * fabs(f * f * f);
-    double di[3], dk[3];
-    const double ri = centre_offset(B, i, u, di), rk = centre_offset(B, k, u, dk);
-    const double so = u_orb(B.n_sto[i], B.g_slater[i], ri), go = u_gauss(B, i, ri);
-    const double so2 = same ? so : u_orb(B.n_sto[k], B.g_slater[k], rk);
-    const double go2 = same ? go : u_gauss(B, k, rk);
-    if (MODE != SS_PREC_FP64) (e == 0 ? Z.j1 : Z.j2)[og] = jac;
-    const double ip = e == 0 ? 1.0 : 1.0 / pi0[s];
-    for (int x = P.first[g]; x < P.first[g + 1]; x++) {
-      const int p = P.order[x];
-      const double poly_ik = poly(B, P.pi[p], di) * poly(B, P.pk[p], dk);
-      double rs = poly_ik * so * so2, rg = poly_ik * go * go2;
-      if (MODE == SS_PREC_FP64) {
-        rs = jac * rs;
-        rg = jac * rg;
-        if (e == 1) {
-          rs = rs * ip;
-          rg = rg * ip;
-        }
+  for (int l = 0; l < 3; l++) u[l] = fzv * r[3 * s + l] * am + P.G[3 * g + l];
+  (e == 0 ? Z.u1x : Z.u2x)[og] = u[0];
+  (e == 0 ? Z.u1y : Z.u2y)[og] = u[1];
+  (e == 0 ? Z.u1z : Z.u2z)[og] = u[2];
+  const double f = fjac * am;
+  const double jac = 0.25 * fabs(f * f * f);
+  double di[3], dk[3];
+  const double ri = centre_offset(B, i, u, di), rk = centre_offset(B, k, u, dk);
+  const double so = u_orb(B.n_sto[i], B.g_slater[i], ri), go = u_gauss(B, i, ri);
+  const double so2 = same ? so : u_orb(B.n_sto[k], B.g_slater[k], rk);
+  const double go2 = same ? go : u_gauss(B, k, rk);
+  if (MODE != SS_PREC_FP64) (e == 0 ? Z.j1 : Z.j2)[og] = jac;
+  const double ip = e == 0 ? 1.0 : 1.0 / pi0[s];
+  for (int x = P.first[g]; x < P.first[g + 1]; x++) {
+    const int p = P.order[x];
+    const double poly_ik = poly(B, P.pi[p], di) * poly(B, P.pk[p], dk);
+    double rs = poly_ik * so * so2, rg = poly_ik * go * go2;
+    if (MODE == SS_PREC_FP64) {
+      rs = jac * rs;
+      rg = jac * rg;
+      if (e == 1) {
+        rs = rs * ip;
+        rg = rg * ip;
       }
-      const int64_t o = (int64_t)p * Z.ld + s;
-      (e == 0 ? Z.a_s : Z.b_s)[o] = rs;
-      (e == 0 ? Z.a_g : Z.b_g)[o] = rg;
     }
+    const int64_t o = (int64_t)p * Z.ld + s;
+    (e == 0 ? Z.a_s : Z.b_s)[o] = rs;
+    (e == 0 ? Z.a_g : Z.b_g)[o] = rg;
   }
 }
 
@@ -151,7 +149,7 @@ __global__ void zv_pair_kernel(BasisDev B, ZvPairs P, int64_t S, const double* _
 // The FP64 pipe bounds it (two lanes per clock and SM).  A quartet and walker on their own cost it
 // about 20 operations, 16 of them r12 and its inverse root; these are the same for all quartets of a
 // tile, and the products with them for its quartets of one ket (FP64) or bra pair (REF32).  The
-// 26-function water's 61,776 quartets make about 5,800 tiles: 4 operations each.  16,000 walkers:
+// 26-function water's 61,776 quartets make 6,250 tiles: 4 operations each.  16,000 walkers:
 // 54 -> 13 ms (a warp per quartet before); the order of every sum is unchanged.
 template <int MODE>
 __global__ void __launch_bounds__(128, 2) zv_accum_kernel(int64_t S, ZvTiles Q, int nsplit, ZvChunk Z,
@@ -306,7 +304,7 @@ cudaError_t launch_walker_aux(cudaStream_t st, int64_t S, const double* r1, cons
 cudaError_t launch_zv_pairs(cudaStream_t st, int mode, const BasisDev& B, const ZvPairs& P,
                             int64_t S, const double* r1, const double* r2, const double* r1m,
                             const double* r2m, const double* pi0, const ZvChunk& Z) {
-  dim3 grid((unsigned)((S + 127) / 128), (unsigned)P.ngroups);
+  dim3 grid((unsigned)((S + 127) / 128), (unsigned)P.ngroups, 2);
   if (mode == SS_PREC_FP64)
     zv_pair_kernel<SS_PREC_FP64><<<grid, 128, 0, st>>>(B, P, S, r1, r2, r1m, r2m, pi0, Z);
   else

@@ -3,9 +3,6 @@
 #include <string.h>
 
 #include <algorithm>
-#include <array>
-#include <map>
-#include <numeric>
 #include <utility>
 #include <vector>
 
@@ -94,28 +91,28 @@ static int upload(ss_ctx* c, const char* name, const std::vector<T>& v, T** out)
 }
 
 // Tiles of the quartets, those with the most quartets first (the last CTAs are then short ones).
-// Bra and ket blocks: ZV_TB (ZV_TK) consecutive pairs of a group in the order of `order`.
-static void build_tiles(const PairPlan& P, const std::vector<int>& group, const std::vector<int>& first,
+// Bra and ket blocks: tb <= ZV_TB (tk <= ZV_TK) consecutive pairs of a group in the order of `order`.
+static void build_tiles(const PairPlan& P, int tb, int tk, const std::vector<int>& group, const std::vector<int>& first,
                         const std::vector<int>& order, std::vector<ZvTile>& tiles, std::vector<int64_t>& tile_q) {
   const int np = P.npairs, ng = (int)first.size() - 1;
   std::vector<int> pos(np), row(np, -1), kblk(ng + 1, 0);
   for (int g = 0; g < ng; g++) {
     for (int x = first[g]; x < first[g + 1]; x++) pos[order[x]] = x - first[g];
-    kblk[g + 1] = kblk[g] + (first[g + 1] - first[g] + ZV_TK - 1) / ZV_TK;
+    kblk[g + 1] = kblk[g] + (first[g + 1] - first[g] + tk - 1) / tk;
   }
   for (int b = 0; b < P.nbra; b++) row[P.bra[b]] = b;
   std::vector<int> open(kblk[ng], -1);  // tile that takes the quartets of the current bra block and a ket block
-  std::vector<std::array<int64_t, ZV_TB * ZV_TK>> q;
+  std::vector<std::pair<int, int>> at(P.q.size());  // tile and bit of every entry of P.q
   for (int g = 0; g < ng; g++)
-    for (int x0 = first[g]; x0 < first[g + 1]; x0 += ZV_TB) {
+    for (int x0 = first[g]; x0 < first[g + 1]; x0 += tb) {
       const size_t begin = tiles.size();
-      for (int x = x0; x < std::min(x0 + ZV_TB, first[g + 1]); x++) {
+      for (int x = x0; x < std::min(x0 + tb, first[g + 1]); x++) {
         const int p1 = order[x];
         if (row[p1] < 0) continue;
         for (int64_t e = P.off[row[p1]]; e < P.off[row[p1] + 1]; e++) {
-          const int p2 = P.ket[e], g2 = group[p2], t = x - x0, u = pos[p2] % ZV_TK;
+          const int p2 = P.ket[e], g2 = group[p2], t = x - x0, u = pos[p2] % tk;
           const uint64_t bit = (uint64_t)1 << (t * ZV_TK + u);
-          int& o = open[kblk[g2] + pos[p2] / ZV_TK];
+          int& o = open[kblk[g2] + pos[p2] / tk];
           if (o < (int)begin || (tiles[o].mask & bit)) {  // none yet, or a quartet listed twice
             ZvTile T{};
             T.g1 = g;
@@ -124,28 +121,43 @@ static void build_tiles(const PairPlan& P, const std::vector<int>& group, const 
             std::fill(T.ket, T.ket + ZV_TK, -1);
             o = (int)tiles.size();
             tiles.push_back(T);
-            q.emplace_back();
           }
           tiles[o].mask |= bit;
           tiles[o].bra[t] = p1;
           tiles[o].ket[u] = p2;
-          q[o][t * ZV_TK + u] = P.q[e];
+          at[e] = {o, t * ZV_TK + u};
         }
       }
     }
-  std::vector<int> by(tiles.size());
-  std::iota(by.begin(), by.end(), 0);
-  std::stable_sort(by.begin(), by.end(), [&](int a, int b) {
-    return __builtin_popcountll(tiles[a].mask) > __builtin_popcountll(tiles[b].mask);
-  });
-  std::vector<ZvTile> sorted;
-  sorted.reserve(tiles.size());
-  tile_q.reserve(P.q.size());
-  for (int o : by) {
-    sorted.push_back(tiles[o]);
-    sorted.back().q = (int64_t)tile_q.size();
-    for (int s = 0; s < ZV_TB * ZV_TK; s++)
-      if (tiles[o].mask >> s & 1) tile_q.push_back(q[o][s]);
+  // counting sort by the number of quartets
+  constexpr int MOST = ZV_TB * ZV_TK;
+  size_t at_count[MOST + 1] = {};  // where the tiles of each number of quartets begin
+  for (const ZvTile& T : tiles) at_count[__builtin_popcountll(T.mask) - 1]++;
+  size_t sum = 0;
+  for (int n = MOST; n >= 0; n--) {
+    const size_t have = at_count[n];
+    at_count[n] = sum;
+    sum += have;
+  }
+  std::vector<ZvTile> sorted(tiles.size());
+  std::vector<int64_t> first_q(tiles.size());
+  {
+    std::vector<int> to(tiles.size());
+    for (size_t x = 0; x < tiles.size(); x++) {
+      to[x] = (int)at_count[__builtin_popcountll(tiles[x].mask) - 1]++;
+      sorted[to[x]] = tiles[x];
+    }
+    int64_t nq = 0;
+    for (ZvTile& T : sorted) {
+      T.q = nq;
+      nq += __builtin_popcountll(T.mask);
+    }
+    for (size_t x = 0; x < tiles.size(); x++) first_q[x] = sorted[to[x]].q;
+  }
+  tile_q.resize(P.q.size());
+  for (size_t e = 0; e < at.size(); e++) {
+    const uint64_t before = tiles[at[e].first].mask & (((uint64_t)1 << at[e].second) - 1);
+    tile_q[first_q[at[e].first] + __builtin_popcountll(before)] = P.q[e];
   }
   tiles.swap(sorted);
 }
@@ -171,17 +183,18 @@ static int run_faithful(ss_ctx* c, double a_zv, uint64_t seed, const double* hr1
       rep.push_back(f);
     }
   }
-  std::map<std::pair<int, int>, int> where;
+  std::vector<int> where(rep.size() * rep.size(), -1);
   std::vector<int> gi, gk, same, group(np), first, order(np);
   for (int p = 0; p < np; p++) {
-    const auto key = std::make_pair(rad[P.pi[p]], rad[P.pk[p]]);
-    const auto it = where.emplace(key, (int)gi.size());
-    if (it.second) {
+    const int ri = rad[P.pi[p]], rk = rad[P.pk[p]];
+    int& g = where[ri * rep.size() + rk];
+    if (g < 0) {
+      g = (int)gi.size();
       gi.push_back(P.pi[p]);
       gk.push_back(P.pk[p]);
-      same.push_back(key.first == key.second);
+      same.push_back(ri == rk);
     }
-    group[p] = it.first->second;
+    group[p] = g;
   }
   const int ng = (int)gi.size();
   first.assign(ng + 1, 0);
@@ -200,36 +213,40 @@ static int run_faithful(ss_ctx* c, double a_zv, uint64_t seed, const double* hr1
     fzv[p] = 0.5 * a_zv / (zi + zk);  // :406
     fjac[p] = a_zv / (zi + zk);       // src/compute_jacobian_and_pi0.F90:22
   }
-  std::vector<ZvTile> tiles;
-  std::vector<int64_t> tile_q;
-  build_tiles(P, group, first, order, tiles, tile_q);
-  ZvPairs dP;
-  ZvTiles dQ;
-  {
-    int *di, *dk, *dsame, *dfirst, *dorder, *pi, *pk;
-    double *dG, *dfzv, *dfjac;
-    int64_t* q;
-    ZvTile* tile;
-    TRY(upload(c, "zv_gi", gi, &di));
-    TRY(upload(c, "zv_gk", gk, &dk));
-    TRY(upload(c, "zv_same", same, &dsame));
-    TRY(upload(c, "zv_first", first, &dfirst));
-    TRY(upload(c, "zv_order", order, &dorder));
-    TRY(upload(c, "zv_pi", P.pi, &pi));
-    TRY(upload(c, "zv_pk", P.pk, &pk));
-    TRY(upload(c, "zv_G", G, &dG));
-    TRY(upload(c, "zv_fzv", fzv, &dfzv));
-    TRY(upload(c, "zv_fjac", fjac, &dfjac));
-    TRY(upload(c, "zv_tile", tiles, &tile));
-    TRY(upload(c, "zv_q", tile_q, &q));
-    dP = ZvPairs{ng, di, dk, dsame, dfirst, dorder, pi, pk, dG, dfzv, dfjac};
-    dQ = ZvTiles{(int)tiles.size(), tile, q};
-  }
   // chunk size: ~1 GiB of pair columns
   const int ncols = (prec == SS_PREC_FP64) ? 10 : 12;
   int64_t Sc = (int64_t)(1.0e9 / (8.0 * ncols * std::max(np, 1)));
   Sc = std::max<int64_t>(1024, std::min<int64_t>(Sc, 1 << 18));
   Sc = std::min<int64_t>(Sc, npts);
+  int nsplit = (int)std::max<int64_t>(1, std::min<int64_t>((4 * c->num_sms + P.nbra - 1) / std::max(P.nbra, 1),
+                                                          std::max<int64_t>(1, Sc / 256)));
+  // Tiles of 6 x 6 quartets where full ones would give every SM three warps, smaller ones on small
+  // systems, where the longest tile is the kernel: carbon, 16,000 walkers: 1.32 ms with 6 x 6 (the
+  // rule's), 1.53 with 3 x 3; H2, 1,920 walkers: 0.42 with 6 x 6, 0.32 with 2 x 2 (the rule's).
+  // A quartet's sums do not depend on its tile.
+  int t = ZV_TB;
+  while (t > 1 && c->nint * nsplit < (int64_t)3 * c->num_sms * t * t) t = t == ZV_TB ? 3 : t - 1;
+  std::vector<ZvTile> tiles;
+  std::vector<int64_t> tile_q;
+  build_tiles(P, t, t, group, first, order, tiles, tile_q);
+  ZvPairs dP;
+  ZvTiles dQ;
+  {  // one upload for all tables
+    std::vector<char> blob;
+    auto put = [&](const auto& v) {
+      const size_t at = (blob.size() + 15) / 16 * 16, bytes = v.size() * sizeof(v[0]);
+      blob.resize(at + bytes);
+      if (bytes) memcpy(blob.data() + at, v.data(), bytes);
+      return at;
+    };
+    const size_t oi = put(gi), ok = put(gk), osame = put(same), ofirst = put(first), oorder = put(order), opi = put(P.pi),
+                 opk = put(P.pk), oG = put(G), ofzv = put(fzv), ofjac = put(fjac), otile = put(tiles), oq = put(tile_q);
+    char* tab;
+    TRY(upload(c, "zv_tables", blob, &tab));
+    dP = ZvPairs{ng, (int*)(tab + oi), (int*)(tab + ok), (int*)(tab + osame), (int*)(tab + ofirst), (int*)(tab + oorder),
+                 (int*)(tab + opi), (int*)(tab + opk), (double*)(tab + oG), (double*)(tab + ofzv), (double*)(tab + ofjac)};
+    dQ = ZvTiles{(int)tiles.size(), (const ZvTile*)(tab + otile), (const int64_t*)(tab + oq)};
+  }
   void* buf;
   TRY(pool_get(c, "zv_cols", sizeof(double) * (size_t)ncols * np * Sc, &buf));
   double* cols = (double*)buf;
@@ -245,8 +262,6 @@ static int run_faithful(ss_ctx* c, double a_zv, uint64_t seed, const double* hr1
   TRY(pool_get(c, "zv_r2m", sizeof(double) * Sc, &buf)); r2m = (double*)buf;
   TRY(pool_get(c, "zv_pi0", sizeof(double) * Sc, &buf)); pi0 = (double*)buf;
   const int64_t nint = c->nint;
-  int nsplit = (int)std::max<int64_t>(1, std::min<int64_t>((4 * c->num_sms + P.nbra - 1) / std::max(P.nbra, 1),
-                                                          std::max<int64_t>(1, Sc / 256)));
   double *partS, *partG, *eS, *eG, *acc, *acc2;
   TRY(pool_get(c, "zv_partS", sizeof(double) * nint * nsplit, &buf)); partS = (double*)buf;
   TRY(pool_get(c, "zv_partG", sizeof(double) * nint * nsplit, &buf)); partG = (double*)buf;
@@ -425,8 +440,8 @@ int ss_two_e_job(ss_ctx* c, double a_zv, uint64_t seed, int64_t samples_per_bloc
   // The analytic stage and the MC meet only in ss_combine.  The analytic stage is queued on its
   // own lowest-priority stream (ensure_gauss returns once its launches are queued) and the MC
   // runs on the context stream (greatest priority) meanwhile: the MC kernels take SM slots as
-  // ERI CTAs retire instead of waiting for the whole stage (measured on the 26-function H2O job:
-  // 1.771 s -> 1.740 s; without the priorities the two streams gave no gain).  Results are
+  // ERI CTAs retire instead of waiting for the whole stage (26-function H2O job: the stages alone
+  // take 44 + 214 ms, the job 250 ms; the GEMM's CTAs leave an SM little room).  Results are
   // bitwise the same.  The context stream waits for the analytic stage before the combine.
   if (!c->ana_stream) {
     int lo = 0, hi = 0;

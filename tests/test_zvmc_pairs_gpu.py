@@ -33,7 +33,7 @@ def _mixed_basis():
 
 
 @pytest.mark.parametrize("precision,rtol", [("fp64", 1e-10), ("ref32", 1e-9)])
-@pytest.mark.parametrize("npts,count", [(80, 40), (40, 1500), (280, 1500)])
+@pytest.mark.parametrize("npts,count", [(80, 40), (40, 1500), (280, 1500), (40, 11000)])
 def test_pair_groups_and_tiles(npts, count, precision, rtol):
     from oracle import binding as O
     b = _mixed_basis()
