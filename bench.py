@@ -475,18 +475,17 @@ def main():
     roofline = {"bound": "fp64", "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                 "frac": achieved / peak64 if (peak64 and achieved) else None,
                 "traffic": EXEC_DRAM_BYTES.get(wl),
-                "traffic_note": "DRAM bytes of all eri_kernel launches of one job (ncu, one pass per metric)",
-                "kernel": "eri_kernel (analytic Gaussian-fit ERIs, all launches of one job)",
+                "traffic_note": "DRAM bytes of the stage's shell_* launches (ncu, one pass per metric)",
+                "kernel": "shell_eri_kernel and shell_lane_kernel (analytic Gaussian-fit ERIs, all launches of one job)",
                 "peak_source": "measured in this run: torch float64 matmul 4096^3 (FP64 peak is not "
                                "in MEASURED_PEAKS.json)",
-                "fp64_pipe_issue_pct": 82.7,
-                "fp64_pipe_note": ("ncu sm__inst_executed_pipe_fp64 of the largest instance, eri_kernel<2,0,1> "
-                                   "(--set full, small case): the stage is FP64-issue bound; the flop "
-                                   "fraction is lower because its FP64 instructions mix DMUL/DADD (1 flop) "
-                                   "with DFMA (2) while the DGEMM peak issues only DFMAs"),
-                "units": (f"executed FP64 flops of the job's eri_kernel launches (ncu instruction "
-                          f"counters, DFMA = 2): {flops:.4g}; plus {EXEC_FLOPS[wl][1]:.4g} FP32 FFMA flops "
-                          f"of the FP32 tier; {nprim:.4g} primitive quartets before screening")
+                "fp64_pipe_issue_pct": 26.9,
+                "fp64_pipe_note": ("ncu sm__inst_executed_pipe_fp64, time-weighted over the stage's launches (60-75 % "
+                                   "in the FP64 tier of the light classes, 14-43 % in the heavy classes, 1-13 % in "
+                                   "the two-float and FP32 tiers, which run on the FP32 pipe)"),
+                "units": (f"executed FP64 flops of the stage's shell_* launches (ncu instruction "
+                          f"counters, DFMA = 2): {flops:.4g}; plus {EXEC_FLOPS[wl][1]:.4g} FP32 flops "
+                          f"of the two-float and FP32 tiers; {nprim:.4g} primitive quartets before screening")
                 if wl in EXEC_FLOPS else f"{nprim:.4g} primitive quartets x FP64 flops per primitive quartet"}
 
     # the MC stage: HBM-bound.  Algorithmic bytes 32 P S per job (the BF16 hi/lo operands of both

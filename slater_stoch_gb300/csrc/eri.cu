@@ -1,4 +1,5 @@
-// eri.cu -- analytic FP64 ERIs of the STO Gaussian fits on sm_103a.
+// eri.cu -- analytic FP64 ERIs of the STO Gaussian fits on sm_103a, per function quartet: the
+// quartets with a function in no shell (degree 3 and more).  shell_tables.cu has all others.
 //
 // Replaces gauss_ijkl (src/gauss_ijkl.F90:51-154) and its callees
 // bielec_integral / give_explicit_poly_and_gaussian / general_primitive_integral /

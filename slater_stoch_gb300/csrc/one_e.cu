@@ -18,7 +18,7 @@
 // The exponentials and the Boys function of an item serve all cartesian components of the r^2-type
 // fits, and every table has compile-time bounds (powers <= 2 per function and axis, which
 // ss_basis_set guarantees), so it stays in registers.  With the tables indexed at run time they
-// lived in local memory: 26.1 ms for the 26-function water (20 Gaussians).
+// lived in local memory: 26.1 ms for the 26-function water (20 Gaussians), 0.64 ms now.
 #include <math.h>
 
 #include <algorithm>

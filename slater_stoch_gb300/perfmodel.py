@@ -5,9 +5,9 @@
   r^2-type fits (i_type 2) and 1 otherwise.  The GPU skips the primitive quartets below its
   Schwarz screen and evaluates those below the FP32 bound in FP32, so the executed work is
   measured rather than modelled:
-* EXEC_FLOPS: executed flops of all eri_kernel launches of one job (Schwarz factors, Schwarz
+* EXEC_FLOPS: executed flops of all shell_* launches of one analytic stage (primitive tables, Schwarz
   diagonal and screened quartets), from ncu instruction counters on the full workload
-  (smsp__sass_thread_inst_executed_op_{dfma,dmul,dadd,ffma}_pred_on.sum, one pass each; DFMA
+  (smsp__sass_thread_inst_executed_op_{dfma,dmul,dadd,ffma,fmul,fadd}_pred_on.sum, one pass each; DFMA
   and FFMA counted as 2 flops), and EXEC_DRAM_BYTES their DRAM traffic (the per-class table and
   the command are kept with the profiles).
 * EXEC_FLOPS_PER_PRIM: the earlier all-FP64 kernel's executed FP64 flops per primitive quartet
@@ -20,22 +20,21 @@ import numpy as np
 # executed FP64 flops per primitive quartet of the all-FP64 kernel (fallback model)
 EXEC_FLOPS_PER_PRIM = 241.5
 
-# workload -> (executed FP64 flops, executed FP32 FFMA flops) of the analytic stage of one job, at
-# the default tiers (primitive screen 1e-18, FP32 tier below 1e-11 of the Schwarz bound)
+# workload -> (executed FP64 flops, executed FP32 flops) of the analytic stage of one job, at the
+# default tiers (primitive screen 1e-18, FP32 below 1e-11 of the Schwarz bound, two floats below 1e-5)
 EXEC_FLOPS = {
-    "h2o_26_ng20": (5.518e11, 4.700e11),
+    "h2o_26_ng20": (7.542e9, 2.902e11),
 }
-# workload -> DRAM bytes (read + write) of all eri_kernel launches of one job (ncu
-# dram__bytes_read.sum + dram__bytes_write.sum, one pass each; mostly the local-memory spill
-# traffic of the L = 4 classes with several r^2-type fits)
+# workload -> DRAM bytes (read + write) of the same launches (EXEC_DRAM_BYTES; ncu
+# dram__bytes_read.sum + dram__bytes_write.sum, one pass each)
 # workload -> DRAM bytes per walker pair of the shared-walker MC kernels (sampler, orbital values,
-# operands, tcgen05 GEMM, accumulation): ncu --set full of one 262,144-sample sub-chunk (reads
-# 2.0146e9 B + writes 1.5291e9 B) / 262,144
+# operands, tcgen05 GEMM, accumulation): ncu of one 262,144-sample sub-chunk (reads 1.9909e9 B +
+# writes 1.5202e9 B) / 262,144
 MC_DRAM_BYTES_PER_SAMPLE = {
-    "h2o_26_ng20": 3.5437e9 / 262144,
+    "h2o_26_ng20": 3.5111e9 / 262144,
 }
 EXEC_DRAM_BYTES = {
-    "h2o_26_ng20": 1.2443e10,
+    "h2o_26_ng20": 1.349e8,
 }
 
 
