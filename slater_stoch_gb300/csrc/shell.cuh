@@ -101,7 +101,6 @@ struct ShPair {
   int fa, fb;                        // one function of each shell (exponents, coefficients, centre)
   int onec, fold, same_system;
   int64_t prim_off, e_off;           // first primitive; first Hermite coefficient
-  double pmax;                       // largest exponent sum of its primitives
   int col[5];                        // where ShArgs::col has this pair type's columns as the ket, by bra degree
 };
 
@@ -110,9 +109,11 @@ struct ShPair {
 struct ShPrim {
   double p, P[3], w, S;
 };
-// Two-float view (high and low parts); w is divided by the pair's power of two (ShArgs::scale)
+// Two-float view (high and low parts); w is divided by the pair's power of two (ShArgs::scale).  s is
+// the power of two next below sqrt(2 p), is = 1 / s: the primitive's unit of length in the FP32
+// evaluations (shell_eri.cuh).
 struct ShPrimF {
-  float p[2], ph[3], pl[3], w[2], pad[2];
+  float p[2], ph[3], pl[3], w[2], s, is;
 };
 static_assert(sizeof(ShPrim) == 48 && sizeof(ShPrimF) == 48, "primitive records are 48 bytes");
 
@@ -143,7 +144,7 @@ struct ShArgs {
   const ShPrim* prim;
   const ShPrimF* primf;
   const double* E;
-  const float2* E2;      // the same as two floats
+  const float2* E2;      // E_t s^|t| as two floats, s of the primitive
   const double* scale;   // power of two of each pair's w in primf
   const ShBoys* boys;    // [SH_MAXL + 1]
   const uint8_t* col;    // columns of t + tau of every bra degree and pair type (ShPair::col)

@@ -19,6 +19,13 @@
 //   >= eps_df   FP64
 //   >= eps32    two floats (df32.cuh, 48 bits): FP64 issues 2 lanes per clock and SM, FP32 128
 //   >= eps      FP32
+// Range of the FP32 exponent: over the primitives of a fit (2 alpha)^n spans more decades at n = 8
+// than FP32 has.  An item's integrals are therefore formed in its own unit of length, R_n k^-n with
+// k = min(s_P, s_Q) (about sqrt(2 alpha); powers of two, so scaling is exact), and the coefficients
+// are E_t s^|t|.  What remains of a term is (k / s_P)^|t| (k / s_Q)^|tau|, at most one: where it
+// underflows the term is negligible.  One unit for the whole shell quartet let the integrals of its
+// diffuse primitives underflow: two centres and 30-Gaussian fits were wrong by 4e-7 of the Schwarz
+// bound (now 5e-14 at most); the factors cost 2 to 6 % (26-function water 44.3 -> 46.1 ms).
 // The decomposition (slices, batches, groups) depends on the shell quartet alone, so a value does
 // not depend on which other quartets were asked for.
 #pragma once
@@ -261,6 +268,16 @@ __constant__ uint32_t sh_hermite[SH_MAXH] = {
 };
 __device__ __forceinline__ int sh_degree(uint32_t h) { return (int)((h & 255) + ((h >> 8) & 255) + (h >> 16)); }
 
+// (k / s_Q)^dtau (k / s_P)^dt of an item, k = min(s_P, s_Q), from the exponents of s_Q / k and s_P / k as
+// float bits (one of them is zero; both below 32, so the factor is a normal number)
+__device__ __forceinline__ int2 sh_shift(const ShPrimF& a, const ShPrimF& b) {
+  const int d = __float_as_int(b.s) - __float_as_int(a.s);
+  return make_int2(min(max(d, 0), 31 << 23), min(max(-d, 0), 31 << 23));
+}
+__device__ __forceinline__ float sh_factor(int2 sh, int dtau, int dt) {
+  return __int_as_float(0x3f800000 - sh.x * dtau - sh.y * dt);
+}
+
 // Threads of a CTA and items of a batch: rows of 8 bytes x Hermite integrals bound the batch from
 // degree 5 on, where the sums of step 2 are most of the work.
 template <int L>
@@ -287,6 +304,7 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
   double* s_acc = reinterpret_cast<double*>(s_col + max_col);  // [group][bra Hermite][ket component]: double or df
   double* s_out = s_acc + (max_no > NT ? max_no : NT);
   __shared__ int s_scan[3][SH_MAXSLICE + 1], s_first[3][SH_MAXSLICE], s_p[SH_MAXSLICE];
+  __shared__ int2 s_sh[NB];  // exponents (as float bits) of s_Q / k and s_P / k of an item
   const int tid = threadIdx.x;
   {  // the launch's dynamic shared memory must hold this carve-up: checked, not assumed
     uint32_t dyn;
@@ -369,11 +387,6 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
   const int my_o = NO < NT ? tid - my_g * NO : tid;
   for (int o = tid; o < (NO > NT ? NO : NT); o += NT) s_acc[o] = 0.0;
   const double scale = diag ? 1.0 : A.scale[W.bra] * A.scale[W.ket];
-  // FP32 evaluations: degree n carries a factor kx^-n, a power of two that holds (2 alpha / kx^2)^L
-  // below 2^100 for the tightest primitives (1 unless 2 alpha exceeds 2^(100/L))
-  float kx = 1.f;
-  if (L > 0) kx = exp2f(fmaxf(0.f, ceilf(0.5f * (log2f((float)(2.0 * fmin(B.pmax, K.pmax))) - 100.f / (L > 0 ? L : 1)))));
-  const float k2 = kx * kx, ik2 = 1.f / k2;
   __syncthreads();
 
   for (int tier = 0; tier < tiers; tier++) {
@@ -423,6 +436,8 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
           continue;
         }
         const ShPrimF a = A.primf[B.prim_off + p], b = A.primf[K.prim_off + q];
+        const float kx = fminf(a.s, b.s), ik = fmaxf(a.is, b.is), ik2 = ik * ik;
+        s_sh[item - base] = sh_shift(a, b);
         if (tier == 1) {
           df* row = reinterpret_cast<df*>(s_R) + (item - base) * ROW;
           const df pa{a.p[0], a.p[1]}, pb{b.p[0], b.p[1]};
@@ -535,24 +550,24 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
                 if (onec && ((ht + tau) & 0x010101u)) continue;
                 const float2* Ek = A.E2 + K.e_off + (size_t)q0 * nterm + x;
                 const int col = s_col[x * H + t];
-                const int dt = sh_degree(tau);
-                // the ket's share of the degree scaling and its sign: exact
-                const float sc = ((dt & 1) ? -kx : 1.f) * ((dt & 2) ? k2 : 1.f) * ((dt & 4) ? k2 * k2 : 1.f);
+                const int dtau = sh_degree(tau), dt = sh_degree(ht);
+                const float sign = (dtau & 1) ? -1.f : 1.f;
                 if (tier == 1) {
                   const df* Rc = reinterpret_cast<const df*>(s_R) + col;
                   df s{0.f, 0.f};
 #pragma unroll 4
                   for (int i = i0; i < i1; i += G, Ek += (size_t)G * nterm) {
                     const float2 e = *Ek;
-                    s = df_fma(Rc[i * ROW], df{e.x, e.y}, s);
+                    s = df_fma(Rc[i * ROW], df_scale(df{e.x, e.y}, sh_factor(s_sh[i], dtau, dt)), s);
                   }
-                  acc = df_add(acc, df_scale(s, sc));
+                  acc = df_add(acc, df_scale(s, sign));
                 } else {
                   const float* Rc = reinterpret_cast<const float*>(s_R) + col;
                   float s = 0.f;
 #pragma unroll 4
-                  for (int i = i0; i < i1; i += G, Ek += (size_t)G * nterm) s = fmaf(Rc[i * ROW], Ek->x, s);
-                  acc = df_add(acc, df{s * sc, 0.f});
+                  for (int i = i0; i < i1; i += G, Ek += (size_t)G * nterm)
+                    s = fmaf(Rc[i * ROW], Ek->x * sh_factor(s_sh[i], dtau, dt), s);
+                  acc = df_add(acc, df{s * sign, 0.f});
                 }
               }
               reinterpret_cast<df*>(s_acc)[o + my_g * NO] = df_renorm(acc);
@@ -573,8 +588,9 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
               df sum = acc[o];
               for (int g = 1; g < G; g++) sum = df_add(sum, acc[o + g * NO]);
               v = df_to(sum) * scale;
-              // the bra's share of the degree scaling
-              for (int d = sh_degree(sh_hermite[o / nf]); d > 0; d--) v *= (double)kx;
+              // the sums are in the bra primitive's unit (degree 0 where they hold several primitives')
+              if (H > 1)
+                for (int d = sh_degree(sh_hermite[o / nf]); d > 0; d--) v *= (double)A.primf[B.prim_off + s_p[j]].s;
             }
             for (int g = 1; g < G; g++) s_acc[o + g * NO] = 0.0;
             s_acc[o] = v;

@@ -34,14 +34,29 @@ __device__ __forceinline__ df lane_zero<df>() { return df{0.f, 0.f}; }
 template <>
 __device__ __forceinline__ float lane_zero<float>() { return 0.f; }
 
-// G[f][t] += R[t + tau] e for all bra Hermite functions t (ONE4: only where t + tau is even on every axis)
+// powers of k / s_P and k / s_Q (shell_eri.cuh) of an item
+struct LaneUnit {
+  float a[5], b[5];
+};
+__device__ __forceinline__ df r_scale(df x, float k) { return df_scale(x, k); }
+__device__ __forceinline__ float r_scale(float x, float k) { return x * k; }
+
+// G[f][t] += R[t + tau] e (k / s_P)^|t| (k / s_Q)^|tau| for all bra Hermite functions t (ONE4: only where
+// t + tau is even on every axis)
 template <uint32_t TAU, bool ONE4, typename Real, int NR, int H, int... T>
-__device__ __forceinline__ void lane_term(const Real (&R)[NR], Real e, Real (&G)[H], std::integer_sequence<int, T...>) {
+__device__ __forceinline__ void lane_term(const Real (&R)[NR], Real e, const LaneUnit& u, Real (&G)[H],
+                                          std::integer_sequence<int, T...>) {
+  constexpr int dtau = (int)((TAU & 255) + ((TAU >> 8) & 255) + (TAU >> 16));
+  Real ed[5];  // by the degree of t
+  ed[0] = dtau ? r_scale(e, u.b[dtau]) : e;
+#pragma unroll
+  for (int d = 1; d < 5; d++)
+    if (H >= sh_nherm(d)) ed[d] = r_scale(ed[0], u.a[d]);
   auto one = [&](auto tc) {
     constexpr int t = decltype(tc)::value;
     constexpr ShDeg h = sh_degs(t);
     constexpr int x = h.t + (int)(TAU & 255), y = h.u + (int)((TAU >> 8) & 255), z = h.v + (int)(TAU >> 16);
-    if constexpr (!ONE4 || !((x | y | z) & 1)) G[t] = r_fma(R[sh_hidx(x, y, z)], e, G[t]);
+    if constexpr (!ONE4 || !((x | y | z) & 1)) G[t] = r_fma(R[sh_hidx(x, y, z)], ed[h.t + h.u + h.v], G[t]);
   };
   (one(std::integral_constant<int, T>()), ...);
 }
@@ -52,17 +67,17 @@ __device__ __forceinline__ df lane_load(const float2* e, df) {
 __device__ __forceinline__ float lane_load(const float2* e, float) { return e->x; }
 
 template <class KET, int X, int X1, bool ONE4, typename Real, int NR, int H>
-__device__ __forceinline__ void lane_comp(const Real (&R)[NR], const float2* e, Real (&G)[H]) {
+__device__ __forceinline__ void lane_comp(const Real (&R)[NR], const float2* e, const LaneUnit& u, Real (&G)[H]) {
   if constexpr (X < X1) {
-    lane_term<KET::S.term[X], ONE4>(R, lane_load(e + X, Real()), G, std::make_integer_sequence<int, H>());
-    lane_comp<KET, X + 1, X1, ONE4>(R, e, G);
+    lane_term<KET::S.term[X], ONE4>(R, lane_load(e + X, Real()), u, G, std::make_integer_sequence<int, H>());
+    lane_comp<KET, X + 1, X1, ONE4>(R, e, u, G);
   }
 }
 template <class KET, int F0, int F, int NF, bool ONE4, typename Real, int NR, int H>
-__device__ __forceinline__ void lane_comps(const Real (&R)[NR], const float2* e, Real (&G)[NF][H]) {
+__device__ __forceinline__ void lane_comps(const Real (&R)[NR], const float2* e, const LaneUnit& u, Real (&G)[NF][H]) {
   if constexpr (F < NF) {
-    lane_comp<KET, KET::S.fs[F0 + F], KET::S.fs[F0 + F + 1], ONE4>(R, e, G[F]);
-    lane_comps<KET, F0, F + 1, NF, ONE4>(R, e, G);
+    lane_comp<KET, KET::S.fs[F0 + F], KET::S.fs[F0 + F + 1], ONE4>(R, e, u, G[F]);
+    lane_comps<KET, F0, F + 1, NF, ONE4>(R, e, u, G);
   }
 }
 
@@ -149,12 +164,22 @@ __device__ __forceinline__ void lane_range(int lo, int hi, int& qa, int& qb) {
 
 // one ket summed into G
 template <typename Real, class KET, int DB, int F0, int NF, bool ONE4>
-__device__ __forceinline__ void lane_ket(const ShPrimF& P, int q, const ShPrimF* s_ket, const float2* s_E, float kx,
-                                         float ik2, const float* boys, Real (&G)[NF][sh_nherm(DB)]) {
+__device__ __forceinline__ void lane_ket(const ShPrimF& P, int q, const ShPrimF* s_ket, const float2* s_E,
+                                         const float* boys, Real (&G)[NF][sh_nherm(DB)]) {
   constexpr int L = DB + KET::S.d;
+  const ShPrimF& Q = s_ket[q];
+  const float kx = fminf(P.s, Q.s), ik = fmaxf(P.is, Q.is);
   Real R[sh_nherm(L)];
-  lane_hermite<L, ONE4>(P, s_ket[q], kx, ik2, boys, R);
-  lane_comps<KET, F0, 0, NF, ONE4>(R, s_E + q * KET::S.nterm, G);
+  lane_hermite<L, ONE4>(P, Q, kx, ik * ik, boys, R);
+  LaneUnit u;
+  u.a[1] = kx * P.is;
+  u.b[1] = kx * Q.is;
+#pragma unroll
+  for (int d = 2; d < 5; d++) {
+    u.a[d] = u.a[d - 1] * u.a[1];
+    u.b[d] = u.b[d - 1] * u.b[1];
+  }
+  lane_comps<KET, F0, 0, NF, ONE4>(R, s_E + q * KET::S.nterm, u, G);
 }
 
 template <class KET, int DB>
@@ -205,11 +230,7 @@ __device__ __forceinline__ void lane_body(const ShArgs& A, const ShWork& W, int 
 #pragma unroll
     for (int t = 0; t < H; t++) G[f][t] = lane_zero<df>();
   const bool any = __syncthreads_or(c > cd);
-  float kx = 1.f;
   if (any) {
-    // as in shell_eri.cuh: degree n carries kx^-n
-    if (L > 0) kx = exp2f(fmaxf(0.f, ceilf(0.5f * (log2f((float)(2.0 * fmin(B.pmax, K.pmax))) - 100.f / (L > 0 ? L : 1)))));
-    const float k2 = kx * kx, ik2 = 1.f / k2;
     const float4* src = reinterpret_cast<const float4*>(A.boys[L].f);
     float4* dst = reinterpret_cast<float4*>(s_boys);
     for (int i = tid; i < SH_BOYS_K * SH_BOYS_ROW / 4; i += SH_LANE_BRA) dst[i] = src[i];
@@ -220,11 +241,9 @@ __device__ __forceinline__ void lane_body(const ShArgs& A, const ShWork& W, int 
     const float2* esrc = A.E2 + K.e_off + (size_t)k0 * NT;
     const ShStruct& SK = A.st[K.st];
     for (int i = tid; i < n * NT; i += SH_LANE_BRA) {
-      // the ket's sign (-1)^|tau| and its share of the degree scaling: exact
-      const int dt = sh_degree(SK.term[i % NT]);
-      const float sc = ((dt & 1) ? -kx : 1.f) * ((dt & 2) ? k2 : 1.f) * ((dt & 4) ? k2 * k2 : 1.f);
+      const float sign = (sh_degree(SK.term[i % NT]) & 1) ? -1.f : 1.f;  // (-1)^|tau|
       const float2 e = esrc[i];
-      s_E[i] = make_float2(e.x * sc, e.y * sc);
+      s_E[i] = make_float2(e.x * sign, e.y * sign);
     }
     __syncthreads();
     ShPrimF P{};
@@ -233,7 +252,7 @@ __device__ __forceinline__ void lane_body(const ShArgs& A, const ShWork& W, int 
     int qa, qb;
     lane_range(cd - k0, cf - k0, qa, qb);
     for (int q = qa; q < qb; q++)
-      if (q >= cd - k0 && q < cf - k0) lane_ket<df, KET, DB, F0, NF, ONE4>(P, q, s_ket, s_E, kx, ik2, s_boys, G);
+      if (q >= cd - k0 && q < cf - k0) lane_ket<df, KET, DB, F0, NF, ONE4>(P, q, s_ket, s_E, s_boys, G);
     // FP32 sums of at most eight kets, then into the two-float sums
     lane_range(cf - k0, c - k0, qa, qb);
     for (int q8 = qa; q8 < qb; q8 += 8) {
@@ -243,7 +262,7 @@ __device__ __forceinline__ void lane_body(const ShArgs& A, const ShWork& W, int 
 #pragma unroll
         for (int t = 0; t < H; t++) Gf[f][t] = 0.f;
       for (int q = q8; q < min(q8 + 8, qb); q++)
-        if (q >= cf - k0 && q < c - k0) lane_ket<float, KET, DB, F0, NF, ONE4>(P, q, s_ket, s_E, kx, ik2, s_boys, Gf);
+        if (q >= cf - k0 && q < c - k0) lane_ket<float, KET, DB, F0, NF, ONE4>(P, q, s_ket, s_E, s_boys, Gf);
 #pragma unroll
       for (int f = 0; f < NF; f++)
 #pragma unroll
@@ -273,7 +292,6 @@ __device__ __forceinline__ void lane_body(const ShArgs& A, const ShWork& W, int 
           const float2 e = *eb;
           v = df_fma(df{e.x, e.y}, g[i], v);
         }
-        for (int d = sh_degree(ht); d > 0; d--) v = df_scale(v, kx);
         s = df_renorm(df_add(s, v));
       }
     }

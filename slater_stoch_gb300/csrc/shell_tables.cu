@@ -198,6 +198,9 @@ __global__ void shell_expand(const ShWork* __restrict__ work, int* __restrict__ 
   for (int s = threadIdx.x; s < W.nlane; s += blockDim.x) lcta[W.lcta0 + s] = blockIdx.x;
 }
 
+// exponent of the largest power of two whose square is at most 2 p
+__device__ __forceinline__ int unit_exp(double p) { return ilogb(p + p) >> 1; }
+
 // Schwarz factors of a pair's primitives and their sorted tables.  A primitive's factor is the
 // largest over the components of sqrt((P_f|P_f) / (f|f)), (f|f) the contracted diagonal: then
 // |(P_f|Q_g)| <= S_P S_Q sqrt((f|f)(g|g)) for every pair of components.  A component without a
@@ -292,15 +295,19 @@ __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pai
     two(a.p, &g.p[0], &g.p[1]);
     two(ldexp(a.w, -ex), &g.w[0], &g.w[1]);
     for (int ax = 0; ax < 3; ax++) two(a.P[ax], &g.ph[ax], &g.pl[ax]);
-    g.pad[0] = g.pad[1] = 0.f;
+    g.s = ldexpf(1.f, unit_exp(a.p));
+    g.is = ldexpf(1.f, -unit_exp(a.p));
     oprimf[P.prim_off + t] = g;
   }
   for (int t = threadIdx.x; t < m * P.nterm; t += blockDim.x) {
     const int r = t / P.nterm, x = t - r * P.nterm;
     const double v = E[P.e_off + (size_t)s_idx[r] * P.nterm + x];
     oE[P.e_off + t] = v;
-    const float hi = (float)v;
-    oE2[P.e_off + t] = make_float2(hi, (float)(v - (double)hi));
+    const uint32_t tm = S.term[x];
+    const int deg = (int)((tm & 255) + ((tm >> 8) & 255) + (tm >> 16));
+    const double u = ldexp(v, deg * unit_exp(prim[P.prim_off + s_idx[r]].p));
+    const float hi = (float)u;
+    oE2[P.e_off + t] = make_float2(hi, (float)(u - (double)hi));
   }
 }
 
@@ -440,8 +447,6 @@ void build_shells(ss_ctx* c) {
       for (int d = 0; d < 5; d++) P.col[d] = structs().off[P.st][d];
       const int na = c->h_ng[P.fa], nb = c->h_ng[P.fb];
       P.cap = P.fold ? na * (na + 1) / 2 : na * nb;
-      P.pmax = *std::max_element(&c->h_gg[(size_t)ld * P.fa], &c->h_gg[(size_t)ld * P.fa] + na) +
-               *std::max_element(&c->h_gg[(size_t)ld * P.fb], &c->h_gg[(size_t)ld * P.fb] + nb);
       P.prim_off = po;
       P.e_off = eo;
       po += P.cap;
