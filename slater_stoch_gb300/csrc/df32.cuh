@@ -55,6 +55,11 @@ SS_DF df df_add(df a, df b) {
   return df{s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l))};
 }
 SS_DF df df_sub(df a, df b) { return df_add(a, df_neg(b)); }
+// a - b of three floats each, to two-float accuracy however much of the leading parts cancels
+SS_DF df df_sub3(float a0, float a1, float a2, float b0, float b1, float b2) {
+  const df s = df_two_sum(a0, -b0), t = df_two_sum(a1, -b1), u = df_two_sum(s.h, t.h);
+  return df{u.h, __fadd_rn(u.l, __fadd_rn(s.l, __fadd_rn(t.l, __fsub_rn(a2, b2))))};
+}
 SS_DF df df_mul(df a, df b) {
   const float p = __fmul_rn(a.h, b.h);
   float e = __fmaf_rn(a.h, b.h, -p);

@@ -109,13 +109,14 @@ struct ShPair {
 struct ShPrim {
   double p, P[3], w, S;
 };
-// Two-float view (high and low parts); w is divided by the pair's power of two (ShArgs::scale).  s is
-// the power of two next below sqrt(2 p), is = 1 / s: the primitive's unit of length in the FP32
-// evaluations (shell_eri.cuh).
+// Two-float view (high and low parts); w is divided by the pair's power of two (ShArgs::scale).  The
+// centre has a third part, so that the distance of two centres keeps two-float accuracy wherever the
+// molecule lies.  s is the power of two next below sqrt(2 p), is = 1 / s: the primitive's unit of
+// length in the FP32 evaluations (shell_eri.cuh).
 struct ShPrimF {
-  float p[2], ph[3], pl[3], w[2], s, is;
+  float p[2], ph[3], pl[3], pm[3], w[2], s, is, pad;
 };
-static_assert(sizeof(ShPrim) == 48 && sizeof(ShPrimF) == 48, "primitive records are 48 bytes");
+static_assert(sizeof(ShPrimF) % sizeof(float4) == 0, "the records are copied as float4");
 
 // One shell quartet of a launch.
 struct ShWork {

@@ -25,7 +25,11 @@
 // are E_t s^|t|.  What remains of a term is (k / s_P)^|t| (k / s_Q)^|tau|, at most one: where it
 // underflows the term is negligible.  One unit for the whole shell quartet let the integrals of its
 // diffuse primitives underflow: two centres and 30-Gaussian fits were wrong by 4e-7 of the Schwarz
-// bound (now 5e-14 at most); the factors cost 2 to 6 % (26-function water 44.3 -> 46.1 ms).
+// bound; the factors cost 2 to 6 % (26-function water 44.3 -> 46.1 ms).
+// Centres are three floats: with two, the distance of two centres that nearly coincide kept 48 bits
+// of their coordinates, and a molecule 120 bohr from the origin was wrong by up to 1e-10 of the bound;
+// the third costs 0 to 3 % (46.1 -> 47.3 ms).  With both, the tiers differ from the all-FP64 evaluation
+// by at most 2.3e-15 of the bound over the bases of tests/test_shell_range_gpu.py.
 // The decomposition (slices, batches, groups) depends on the shell quartet alone, so a value does
 // not depend on which other quartets were asked for.
 #pragma once
@@ -268,6 +272,10 @@ __constant__ uint32_t sh_hermite[SH_MAXH] = {
 };
 __device__ __forceinline__ int sh_degree(uint32_t h) { return (int)((h & 255) + ((h >> 8) & 255) + (h >> 16)); }
 
+__device__ __forceinline__ df sh_distance(const ShPrimF& a, const ShPrimF& b, int ax) {
+  return df_sub3(a.ph[ax], a.pl[ax], a.pm[ax], b.ph[ax], b.pl[ax], b.pm[ax]);
+}
+
 // (k / s_Q)^dtau (k / s_P)^dt of an item, k = min(s_P, s_Q), from the exponents of s_Q / k and s_P / k as
 // float bits (one of them is zero; both below 32, so the factor is a normal number)
 __device__ __forceinline__ int2 sh_shift(const ShPrimF& a, const ShPrimF& b) {
@@ -457,9 +465,7 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
             }
             store_row_1c<L, df>(bs, row);
           } else {
-            df X = df_sub(df{a.ph[0], a.pl[0]}, df{b.ph[0], b.pl[0]});
-            df Y = df_sub(df{a.ph[1], a.pl[1]}, df{b.ph[1], b.pl[1]});
-            df Z = df_sub(df{a.ph[2], a.pl[2]}, df{b.ph[2], b.pl[2]});
+            const df X = sh_distance(a, b, 0), Y = sh_distance(a, b, 1), Z = sh_distance(a, b, 2);
             df F[L + 1];
             boys_shell<L>(df_renorm(df_mul(alpha, df_fma(X, X, df_fma(Y, Y, df_mul(Z, Z))))), F, s_boys);
             df pw = pre;

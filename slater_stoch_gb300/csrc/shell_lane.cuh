@@ -102,9 +102,7 @@ __device__ __forceinline__ void lane_hermite(const ShPrimF& a, const ShPrimF& b,
     }
     store_row_1c<L, df>(bs, R);
   } else {
-    const df X = df_sub(df{a.ph[0], a.pl[0]}, df{b.ph[0], b.pl[0]});
-    const df Y = df_sub(df{a.ph[1], a.pl[1]}, df{b.ph[1], b.pl[1]});
-    const df Z = df_sub(df{a.ph[2], a.pl[2]}, df{b.ph[2], b.pl[2]});
+    const df X = sh_distance(a, b, 0), Y = sh_distance(a, b, 1), Z = sh_distance(a, b, 2);
     df F[L + 1];
     boys_shell<L>(df_renorm(df_mul(alpha, df_fma(X, X, df_fma(Y, Y, df_mul(Z, Z))))), F, boys);
     df pw = pre;
@@ -237,7 +235,7 @@ __device__ __forceinline__ void lane_body(const ShArgs& A, const ShWork& W, int 
     const int n = k1 - k0;
     const float4* ksrc = reinterpret_cast<const float4*>(A.primf + K.prim_off + k0);
     float4* kdst = reinterpret_cast<float4*>(s_ket);
-    for (int i = tid; i < n * 3; i += SH_LANE_BRA) kdst[i] = ksrc[i];
+    for (int i = tid; i < n * (int)(sizeof(ShPrimF) / sizeof(float4)); i += SH_LANE_BRA) kdst[i] = ksrc[i];
     const float2* esrc = A.E2 + K.e_off + (size_t)k0 * NT;
     const ShStruct& SK = A.st[K.st];
     for (int i = tid; i < n * NT; i += SH_LANE_BRA) {

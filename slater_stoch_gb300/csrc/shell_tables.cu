@@ -294,7 +294,11 @@ __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pai
     ShPrimF g;
     two(a.p, &g.p[0], &g.p[1]);
     two(ldexp(a.w, -ex), &g.w[0], &g.w[1]);
-    for (int ax = 0; ax < 3; ax++) two(a.P[ax], &g.ph[ax], &g.pl[ax]);
+    for (int ax = 0; ax < 3; ax++) {
+      two(a.P[ax], &g.ph[ax], &g.pl[ax]);
+      g.pm[ax] = (float)((a.P[ax] - (double)g.ph[ax]) - (double)g.pl[ax]);
+    }
+    g.pad = 0.f;
     g.s = ldexpf(1.f, unit_exp(a.p));
     g.is = ldexpf(1.f, -unit_exp(a.p));
     oprimf[P.prim_off + t] = g;

@@ -1,6 +1,6 @@
-"""The two-float and FP32 tiers of the shell-quartet ERIs where FP32's range could be left: fits of
-30 Gaussians (exponents over 8 decades and more), exponents that differ between the shells, one
-and two centres.  Every value against the same kernels with the tiers off (all FP64), and a sample
+"""The two-float and FP32 tiers of the shell-quartet ERIs where FP32's range or digits could be left:
+fits of 30 Gaussians (exponents over 8 decades and more), exponents that differ between the shells,
+one and two centres, a molecule far from the origin.  Every value against the same kernels with the tiers off (all FP64), and a sample
 against the oracle.
 
 Gate per quartet, as for the other analytic ERIs: 1e-12 |ERI| + 1e-12 sqrt((ik|ik)(jl|jl)).
@@ -63,3 +63,11 @@ def test_long_fits_against_the_oracle(orbs):
     ref, _ = O.gauss_eri(ob, q, O.precond(ob))
     g, _, pre = _default_and_fp64(b, q)
     _gate(g, ref, pre, q)
+
+
+@pytest.mark.parametrize("orbs", list(ORBS))
+def test_far_from_the_origin(orbs):
+    b = _basis(ORBS[orbs], 20, [[100.1, -60.2, 33.3], [101.3, -59.1, 32.2]])
+    q = basis.build_mapping(b.n)
+    g, f, pre = _default_and_fp64(b, q)
+    _gate(g, f, pre, q)
