@@ -94,12 +94,12 @@ constexpr ShStruct sh_struct(int ta, int tb, bool same, bool onec) {
   return S;
 }
 
-// One shell pair.  Its primitives occupy prim[prim_off .. prim_off + cap), cnt[pair] of them used.
+// One shell pair of a system.  Its primitives occupy prim[prim_off .. prim_off + cap), cnt[pair] of them used.
 struct ShPair {
   int st, d, ncomp, nterm;
-  int cap;                           // most primitives it can have (before the K_AB screen)
+  int cap;                           // most primitives it can have after the K_AB screen
   int fa, fb;                        // one function of each shell (exponents, coefficients, centre)
-  int onec, fold, same_system;
+  int onec, fold;
   int64_t prim_off, e_off;           // first primitive; first Hermite coefficient
   int col[5];                        // where ShArgs::col has this pair type's columns as the ket, by bra degree
 };

@@ -12,7 +12,6 @@ struct ShellPlan {
   std::vector<ShWork> work[SH_MAXL + 1];
 };
 
-void build_shells(ss_ctx* c);
 int shell_precond(ss_ctx* c, std::vector<double>& pre);
 int shell_plan(ss_ctx* c, bool tiers, const std::vector<int64_t>& sel, std::vector<int64_t>& slot, std::vector<int64_t>& rest,
                ShellPlan& plan, int64_t* nelem);

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "boys_grid.cuh"
+#include "shell_basis.h"
 #include "shell_host.h"
 #include "ss_context.cuh"
 
@@ -27,49 +28,6 @@ constexpr double SH_DF_EPS = 1e-5;
     int rc_ = (x);       \
     if (rc_) return rc_; \
   } while (0)
-
-// ---- pair types ------------------------------------------------------------------------------
-
-// pair type of canonical shell types ta >= tb; same: one shell with itself (components ca >= cb)
-static int struct_index(int ta, int tb, bool same, bool onec) {
-  int base = ta * (ta + 1) / 2 + tb;
-  if (same && ta == SH_P) base = SH_NBASE;
-  if (same && ta == SH_D) base = SH_NBASE + 1;
-  return 2 * base + (onec ? 1 : 0);
-}
-
-struct StructTable {
-  std::vector<ShStruct> s;
-  std::vector<uint8_t> col;         // ShArgs::col
-  int off[SH_NSTRUCT][5] = {};
-  StructTable() : s(SH_NSTRUCT) {
-    for (int ta = 0; ta < 4; ta++)
-      for (int tb = 0; tb <= ta; tb++)
-        for (int oc = 0; oc < 2; oc++) s[struct_index(ta, tb, false, oc)] = sh_struct(ta, tb, false, oc);
-    for (int oc = 0; oc < 2; oc++) {
-      s[struct_index(SH_P, SH_P, true, oc)] = sh_struct(SH_P, SH_P, true, oc);
-      s[struct_index(SH_D, SH_D, true, oc)] = sh_struct(SH_D, SH_D, true, oc);
-    }
-    for (int st = 0; st < SH_NSTRUCT; st++)
-      for (int d = 0; d < 5; d++) {
-        const ShStruct& S = s[st];
-        off[st][d] = (int)col.size();
-        col.resize(col.size() + sh_col_size(d, S.nterm));
-        for (int x = 0; x < S.nterm; x++)
-          for (int n = 0, t = 0; n <= d; n++)  // bra Hermite functions in the order of sh_hidx
-            for (int w = 0; w <= n; w++)
-              for (int v = 0; v <= w; v++, t++) {
-                const uint32_t tm = S.term[x];
-                col[off[st][d] + x * sh_nherm(d) + t] = (uint8_t)sh_hidx(
-                    n - w + (int)(tm & 255), w - v + (int)((tm >> 8) & 255), v + (int)(tm >> 16));
-              }
-      }
-  }
-};
-static const StructTable& structs() {
-  static const StructTable t;
-  return t;
-}
 
 // ---- device tables ---------------------------------------------------------------------------
 
@@ -97,7 +55,7 @@ __global__ void __launch_bounds__(256) shell_fill(BasisDev B, const ShPair* __re
   const double x0 = A[0] - C[0], x1 = A[1] - C[1], x2 = A[2] - C[2];
   const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int n = P.same_system ? na * nb : 0;
+  const int n = na * nb;
   for (int t0 = 0; t0 < n; t0 += 256) {
     const int t = t0 + threadIdx.x;
     const int m1 = t / nb, m2 = t - m1 * nb;
@@ -380,112 +338,6 @@ cudaError_t launch_shell_lane(int instance, int ncta, cudaStream_t st, const ShA
 
 // ---- host ------------------------------------------------------------------------------------
 
-// Shells of the basis and their pairs (host only; rebuilt by ss_basis_set / ss_basis_systems).
-// A function beyond d, or an r^2-type fit with angular factors, belongs to no shell: its quartets
-// take the per-function kernel (eri_kernel.cuh).
-void build_shells(ss_ctx* c) {
-  ShellBasis& T = c->shells;
-  T = ShellBasis();
-  const int n = c->n, ld = c->ld;
-  T.fsh.assign(n, -1);
-  T.fcomp.assign(n, 0);
-  std::vector<int> first, type, deg_nsys;
-  auto same_fit = [&](int a, int b) {
-    if (c->h_ng[a] != c->h_ng[b] || c->h_itype[a] != c->h_itype[b]) return false;
-    const size_t t = c->h_itype[a] == 2 ? 1 : 0;
-    for (int m = 0; m < c->h_ng[a]; m++)
-      if (c->h_gg[m + (size_t)ld * a] != c->h_gg[m + (size_t)ld * b] ||
-          c->h_cg[m + (size_t)ld * (a + n * t)] != c->h_cg[m + (size_t)ld * (b + n * t)])
-        return false;
-    return true;
-  };
-  auto same_centre = [&](int a, int b) {
-    for (int ax = 0; ax < 3; ax++)
-      if (c->h_center[3 * a + ax] != c->h_center[3 * b + ax]) return false;
-    return true;
-  };
-  auto sys = [&](int f) { return c->h_sys.empty() ? 0 : c->h_sys[f]; };
-  for (int f = 0; f < n; f++) {
-    const int* np = &c->h_npower[3 * f];
-    const int l = np[0] + np[1] + np[2];
-    if (c->h_itype[f] == 2 ? l > 0 : l > 2) {
-      T.all = false;
-      continue;
-    }
-    const int ty = c->h_itype[f] == 2 ? SH_R : (l == 0 ? SH_S : l == 1 ? SH_P : SH_D);
-    int comp = 0;
-    for (int x = 0; x < SH_NC[ty]; x++)
-      if (ty != SH_R && SH_POW[ty][x][0] == np[0] && SH_POW[ty][x][1] == np[1] && SH_POW[ty][x][2] == np[2]) comp = x;
-    T.fcomp[f] = comp;
-    // a shell with this fit whose component is still free (components are mostly consecutive: the
-    // latest shells first)
-    for (int s = (int)first.size() - 1; s >= 0 && T.fsh[f] < 0; s--)
-      if (type[s] == ty && sys(first[s]) == sys(f) && same_centre(first[s], f) && same_fit(first[s], f)) T.fsh[f] = s;
-    if (T.fsh[f] < 0) {
-      T.fsh[f] = (int)first.size();
-      first.push_back(f);
-      type.push_back(ty);
-    }
-  }
-  const int nsh = (int)first.size();
-  T.nsh = nsh;
-  T.pair.clear();
-  T.spair.assign((size_t)nsh * nsh, -1);
-  T.flip.assign((size_t)nsh * nsh, 0);
-  int64_t po = 0, eo = 0;
-  for (int x = 0; x < nsh; x++)
-    for (int y = 0; y <= x; y++) {
-      int a = x, b = y;
-      if (type[a] < type[b]) std::swap(a, b);
-      ShPair P{};
-      P.fa = first[a];
-      P.fb = first[b];
-      P.onec = same_centre(P.fa, P.fb);
-      P.fold = P.onec && same_fit(P.fa, P.fb);
-      P.same_system = sys(P.fa) == sys(P.fb);
-      P.st = struct_index(type[a], type[b], a == b, P.onec);
-      const ShStruct& S = structs().s[P.st];
-      P.d = S.d;
-      P.ncomp = S.ncomp;
-      P.nterm = S.nterm;
-      for (int d = 0; d < 5; d++) P.col[d] = structs().off[P.st][d];
-      const int na = c->h_ng[P.fa], nb = c->h_ng[P.fb];
-      P.cap = P.fold ? na * (na + 1) / 2 : na * nb;
-      P.prim_off = po;
-      P.e_off = eo;
-      po += P.cap;
-      eo += (int64_t)P.cap * P.nterm;
-      T.spair[(size_t)x * nsh + y] = T.spair[(size_t)y * nsh + x] = (int)T.pair.size();
-      // (x, y) as given is (b, a) of the pair
-      T.flip[(size_t)a * nsh + b] = 0;
-      T.flip[(size_t)b * nsh + a] = a != b;
-      T.pair.push_back(P);
-    }
-  T.nb.resize(nsh);
-  for (int s = 0; s < nsh; s++) T.nb[s] = SH_NC[type[s]];
-  T.nprim = po;
-  T.nE = eo;
-}
-
-// shell pair and component of functions i and k; false if one of them is in no shell
-static bool shell_component(const ShellBasis& T, int i, int k, int* pair, int* comp) {
-  int a = T.fsh[i], b = T.fsh[k];
-  if (a < 0 || b < 0) return false;
-  int ca = T.fcomp[i], cb = T.fcomp[k];
-  if (T.flip[(size_t)a * T.nsh + b]) {
-    std::swap(a, b);
-    std::swap(ca, cb);
-  }
-  *pair = T.spair[(size_t)a * T.nsh + b];
-  if (a == b) {
-    if (ca < cb) std::swap(ca, cb);
-    *comp = ca * (ca + 1) / 2 + cb;
-  } else {
-    *comp = ca * T.nb[b] + cb;
-  }
-  return true;
-}
-
 // multiply-adds of the Hermite integrals of total degree L
 static const double SH_REC[SH_MAXL + 1] = {2, 8, 24, 60, 120, 200, 330, 520, 790};
 
@@ -699,7 +551,7 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
   ShellPlan Lw;
   for (int x = 0; x < np; x++) {
     const ShPair& P = T.pair[x];
-    if (!P.same_system) continue;
+    if (P.cap == 0) continue;  // (ik|ik) = 0
     ShWork w{};
     w.bra = w.ket = x;
     w.split = std::max(1, (P.cap + 1) / 2);  // two bra primitives: few quartets, in FP64
@@ -716,12 +568,14 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
   SS_CUDA_TRY(cudaMemcpyAsync(h.data(), diag, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
   SS_CUDA_TRY(cudaStreamSynchronize(c->stream));
   const int n = c->n;
-  for (int i = 0; i < n; i++)
-    for (int k = 0; k <= i; k++) {
+  for (int i = 0, f0 = 0; i < n; i++) {
+    if (!c->h_sys.empty() && c->h_sys[i] != c->h_sys[f0]) f0 = i;  // first function of the system
+    for (int k = f0; k <= i; k++) {
       int pr, f;
-      if (!shell_component(T, i, k, &pr, &f)) continue;
+      if (!T.component(i, k, &pr, &f)) continue;
       pre[i + (size_t)n * k] = pre[k + (size_t)n * i] = h[(size_t)pr * SH_MAXCOMP + f];
     }
+  }
   return SS_OK;
 }
 
@@ -732,32 +586,54 @@ int shell_plan(ss_ctx* c, bool tiers, const std::vector<int64_t>& sel, std::vect
                ShellPlan& plan, int64_t* nelem) {
   const ShellBasis& T = c->shells;
   const int n = c->n;
-  std::vector<int32_t> fpair((size_t)n * n, -1);
-  std::vector<int16_t> fcomp((size_t)n * n, 0);
-  for (int i = 0; i < n; i++)
-    for (int k = 0; k <= i; k++) {
-      int pr, f;
-      if (!shell_component(T, i, k, &pr, &f)) continue;
-      fpair[i + (size_t)n * k] = pr;
-      fcomp[i + (size_t)n * k] = (int16_t)f;
+  auto sys = [&](int f) { return c->h_sys.empty() ? 0 : c->h_sys[f]; };
+  // shell pair and component of every two functions of a system
+  std::vector<int> f0(n);
+  std::vector<int64_t> row(n);
+  std::vector<int32_t> fpair;
+  std::vector<int16_t> fcomp;
+  for (int i = 0; i < n; i++) {
+    f0[i] = i > 0 && sys(i) == sys(i - 1) ? f0[i - 1] : i;
+    row[i] = (int64_t)fpair.size() - f0[i];
+    for (int k = f0[i]; k <= i; k++) {
+      int pr = -1, f = 0;
+      T.component(i, k, &pr, &f);
+      fpair.push_back(pr);
+      fcomp.push_back((int16_t)f);
     }
-  const int64_t np = (int64_t)T.pair.size(), nkey = np * (np + 1) / 2;
-  const bool dense = nkey <= (int64_t)64 << 20;
-  std::vector<int32_t> where(dense ? nkey : 0, -1);
+  }
+  // entry of Q of every two pairs of a system, and of those across systems that the list has
+  const int nsys = (int)T.first.size() - 1;
+  std::vector<int64_t> block(nsys + 1, 0);
+  std::vector<int> psys(T.pair.size());
+  for (int s = 0; s < nsys; s++) {
+    const int64_t np = T.pfirst[s + 1] - T.pfirst[s];
+    block[s + 1] = block[s] + np * (np + 1) / 2;
+    std::fill(psys.begin() + T.pfirst[s], psys.begin() + T.pfirst[s + 1], s);
+  }
+  const bool dense = block[nsys] <= (int64_t)64 << 20;
+  std::vector<int32_t> where(dense ? block[nsys] : 0, -1);
   std::unordered_map<int64_t, int32_t> sparse;
   struct Quartet { int bra, ket; uint64_t mask; int64_t elem; };
   std::vector<Quartet> Q;
   int64_t elem = 0;
   for (int64_t t : sel) {
     const int i = c->h_is[t] - 1, k = c->h_ks[t] - 1, j = c->h_js[t] - 1, l = c->h_ls[t] - 1;
-    const size_t a = i + (size_t)n * k, b = j + (size_t)n * l;
+    if (k < f0[i] || l < f0[j]) continue;  // a product of functions of two systems is none: 0
+    const int64_t a = row[i] + k, b = row[j] + l;
     const int pa = fpair[a], pb = fpair[b];
     if (pa < 0 || pb < 0) {
       rest.push_back(t);
       continue;
     }
-    const int64_t hi = std::max(pa, pb), lo = std::min(pa, pb), key = hi * (hi + 1) / 2 + lo;
-    int32_t* w = dense ? &where[key] : &sparse.emplace(key, -1).first->second;
+    const int64_t hi = std::max(pa, pb), lo = std::min(pa, pb);
+    int32_t* w;
+    if (dense && psys[hi] == psys[lo]) {
+      const int64_t h = hi - T.pfirst[psys[hi]];
+      w = &where[block[psys[hi]] + h * (h + 1) / 2 + (lo - T.pfirst[psys[hi]])];
+    } else {
+      w = &sparse.emplace(hi * (hi + 1) / 2 + lo, -1).first->second;
+    }
     if (*w < 0) {
       *w = (int32_t)Q.size();
       const ShPair &x = T.pair[hi], &y = T.pair[lo];
@@ -776,7 +652,7 @@ int shell_plan(ss_ctx* c, bool tiers, const std::vector<int64_t>& sel, std::vect
     w.bra = s.bra;
     w.ket = s.ket;
     const ShPair &b = T.pair[s.bra], &k = T.pair[s.ket];
-    const int chunk = tiers ? lane_chunk(b, k) : 0;
+    const int chunk = tiers && b.cap && k.cap ? lane_chunk(b, k) : 0;
     w.lane = -1;
     if (chunk) {
       bool all = b.onec && k.onec;

@@ -188,17 +188,16 @@ int join_eri_streams(ss_ctx* c) {
   return SS_OK;
 }
 
+// nothing that was made from the basis holds any more
+static void reset_tables(ss_ctx* c) {
+  c->have_shells = c->have_precond = c->have_gauss = c->have_mc = false;
+  c->have_resid = c->have_mono = false;
+}
+
 // Run the per-function ERI kernels for the quartets listed in (qis..qls) restricted to `sel`
 // (indices into them); partial sums are written to d_scratch_b from entry `first` on and slot[q]
 // gives the partial row of q.  These kernels serve the quartets that have a function in no shell
 // (shell_tables.cu); the others take the shell-quartet kernel.
-static int reset_tables(ss_ctx* c) {
-  build_shells(c);
-  c->have_precond = c->have_gauss = c->have_mc = false;
-  c->have_resid = c->have_mono = false;
-  return SS_OK;
-}
-
 static int run_eri(ss_ctx* c, const int32_t* d_qis, const int32_t* d_qjs, const int32_t* d_qks,
                    const int32_t* d_qls, const std::vector<int32_t>& qis, const std::vector<int32_t>& qjs,
                    const std::vector<int32_t>& qks, const std::vector<int32_t>& qls,
@@ -400,6 +399,12 @@ int ensure_precond(ss_ctx* c) {
     return SS_ERR_STATE;
   }
   const int n = c->n;
+  if (!c->have_shells) {
+    c->shells = build_shell_basis(BasisHost{n, c->ld, c->h_center.data(), c->h_npower.data(), c->h_itype.data(),
+                                            c->h_ng.data(), c->h_cg.data(), c->h_gg.data(),
+                                            c->h_sys.empty() ? nullptr : c->h_sys.data()});
+    c->have_shells = true;
+  }
   c->h_precond.assign((size_t)n * n, 0.0);
   TRY(shell_precond(c, c->h_precond));
   if (!c->shells.all) TRY(function_precond(c, c->h_precond));
@@ -603,6 +608,8 @@ int ss_basis_set(ss_ctx* c, int nbasis, const double* center, const int* npower,
       return SS_ERR_ARG;
     }
   }
+  reset_tables(c);
+  c->h_sys.clear();
   c->n = nbasis;
   c->ld = ld;
   c->h_center.assign(center, center + 3 * nbasis);
@@ -630,13 +637,15 @@ int ss_basis_set(ss_ctx* c, int nbasis, const double* center, const int* npower,
   rc |= h2d(c, c->d_cg, c_gauss, sizeof(double) * ld * nbasis * 2);
   rc |= h2d(c, c->d_gg, g_gauss, sizeof(double) * ld * nbasis);
   rc |= h2d(c, c->d_gs, g_slater, sizeof(double) * nbasis);
-  if (rc) return SS_ERR_NOMEM;
+  if (rc) {
+    c->n = 0;  // the device has not all of it
+    return SS_ERR_NOMEM;
+  }
   c->basis = BasisDev{nbasis, ld, (const double*)c->d_center.ptr, (const int*)c->d_npower.ptr,
                       (const int*)c->d_nsto.ptr, (const int*)c->d_itype.ptr, (const int*)c->d_ng.ptr,
                       (const double*)c->d_cg.ptr, (const double*)c->d_gg.ptr, (const double*)c->d_gs.ptr,
                       nullptr};
-  c->h_sys.clear();
-  return reset_tables(c);
+  return SS_OK;
 }
 
 int ss_basis_systems(ss_ctx* c, int nsys, const int* first) {
@@ -661,7 +670,8 @@ int ss_basis_systems(ss_ctx* c, int nsys, const int* first) {
   if (rc) return rc;
   c->h_sys = sys;
   c->basis.sys = (const int*)c->d_sys.ptr;
-  return reset_tables(c);
+  reset_tables(c);
+  return SS_OK;
 }
 
 }  // extern "C"

@@ -9,7 +9,7 @@
 #include <vector>
 
 #include "admission.h"
-#include "shell.cuh"
+#include "shell_basis.h"
 #include "ss_common.cuh"
 
 namespace ss {
@@ -18,17 +18,6 @@ namespace ss {
 struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
-};
-
-// Shells of the basis (shell_tables.cu): shell and component of every function (-1: in no shell),
-// the pair of every two shells, and whether a pair holds them in the other order.
-struct ShellBasis {
-  bool all = true;  // every function is in a shell
-  int nsh = 0;
-  std::vector<int> fsh, fcomp, nb, spair;
-  std::vector<char> flip;
-  std::vector<ShPair> pair;
-  int64_t nprim = 0, nE = 0;
 };
 
 // Parameters of the shared-walker proposal: a mixture of ZV-map densities
@@ -90,7 +79,8 @@ struct ss_ctx {
   // nuclei for the one-electron nuclear attraction (ss_nuclei_set)
   std::vector<double> h_nuc_xyz, h_nuc_charge;
 
-  ss::ShellBasis shells;
+  bool have_shells = false;
+  ss::ShellBasis shells;  // of the current basis, built when first used (ensure_precond)
 
   // primitive pairs of the per-function kernels (built when a function is in no shell)
   ss::DevBuf d_pp, d_pp_off, d_pp_cnt;
