@@ -513,11 +513,16 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
   const int np = (int)T.pair.size();
   if (!np) return SS_OK;
   void* p;
-  if (!c->pool["shell_struct"].ptr) {  // constants, once per context
+  if (!c->have_shell_consts) {  // once per context; a call that failed half-way left the flag unset
     TRY(pool_get(c, "shell_struct", sizeof(ShStruct) * SH_NSTRUCT, &p));
     TRY(h2d_copy(c, p, structs().s.data(), sizeof(ShStruct) * SH_NSTRUCT));
     TRY(pool_get(c, "shell_col", structs().col.size(), &p));
     TRY(h2d_copy(c, p, structs().col.data(), structs().col.size()));
+    TRY(pool_get(c, "shell_boys", sizeof(ShBoys) * (SH_MAXL + 1), &p));
+    shell_boys<<<dim3((SH_BOYS_K + 63) / 64, SH_MAXL + 1), 64, 0, c->stream>>>((ShBoys*)p);
+    SS_CUDA_TRY(cudaGetLastError());
+    c->launches++;
+    c->have_shell_consts = true;
   }
   const ShStruct* st = (const ShStruct*)c->pool["shell_struct"].ptr;
   TRY(h2d_async(c, c->pool["shell_pair"], T.pair.data(), sizeof(ShPair) * np));
@@ -537,12 +542,6 @@ int shell_precond(ss_ctx* c, std::vector<double>& pre) {
   TRY(pool_get(c, "shell_E", sizeof(double) * T.nE, &p)); E2 = (double*)p;
   TRY(pool_get(c, "shell_E2", sizeof(float2) * T.nE, &p)); E2f = (float2*)p;
   TRY(pool_get(c, "shell_scale", sizeof(double) * np, &p)); scale = (double*)p;
-  if (!c->pool["shell_boys"].ptr) {  // constants, once per context
-    TRY(pool_get(c, "shell_boys", sizeof(ShBoys) * (SH_MAXL + 1), &p));
-    shell_boys<<<dim3((SH_BOYS_K + 63) / 64, SH_MAXL + 1), 64, 0, c->stream>>>((ShBoys*)p);
-    SS_CUDA_TRY(cudaGetLastError());
-    c->launches++;
-  }
   TRY(pool_get(c, "shell_diag", sizeof(double) * np * SH_MAXCOMP, &p)); diag = (double*)p;
   SS_CUDA_TRY(cudaMemsetAsync(diag, 0, sizeof(double) * np * SH_MAXCOMP, c->stream));
   shell_fill<<<np, 256, 0, c->stream>>>(c->basis, dpair, st, F);

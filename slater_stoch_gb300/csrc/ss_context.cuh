@@ -79,6 +79,7 @@ struct ss_ctx {
   // nuclei for the one-electron nuclear attraction (ss_nuclei_set)
   std::vector<double> h_nuc_xyz, h_nuc_charge;
 
+  bool have_shell_consts = false;  // pair-type tables and Boys tables (pool "shell_struct", "_col", "_boys")
   bool have_shells = false;
   ss::ShellBasis shells;  // of the current basis, built when first used (ensure_precond)
 
