@@ -376,7 +376,8 @@ static int slices(const ShPair& b, const ShPair& k, bool lane) {
 }
 
 // Launch the work entries (grouped by total degree), in chunks whose partial sums fit the buffer,
-// and reduce each chunk's partial sums to elements.
+// and reduce each chunk's partial sums to elements.  All chunks' entries go up in one copy before the
+// first launch, so that the host waits for no chunk's kernels.
 static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF* primf, const double* E, const float2* E2,
                     bool diag, double eps, double eps32, double* elem) {
   const ShellBasis& T = c->shells;
@@ -384,73 +385,114 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
   size_t cap = (size_t)64 << 20;
   if (c->budget) cap = std::min(cap, std::max<size_t>((c->budget - std::min(c->budget, c->used)) / 4, 1 << 20));
   const int64_t cap_d = (int64_t)(cap / sizeof(double));
-  // heaviest degrees first: their CTAs are the longest
-  std::vector<ShWork> chunk;
-  struct Seg { int L, first, n, ncta, no, ni, col; };
-  std::vector<Seg> segs;
+  struct Seg { int L, cta0, ncta, no, ni, col; };
   struct LaneSeg { int instance, cta0, ncta; };
-  std::vector<LaneSeg> lanes;
-  int64_t part = 0, most = 0;
-  int ncta = 0, nlane = 0;
-  auto flush = [&]() -> int {
-    if (chunk.empty()) return SS_OK;
-    // the lane kernels' CTAs, an instance's together
-    std::vector<int> order;
-    for (size_t t = 0; t < chunk.size(); t++)
-      if (chunk[t].lane >= 0) order.push_back((int)t);
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return chunk[x].lane > chunk[y].lane; });
-    lanes.clear();
-    nlane = 0;
-    for (int t : order) {
-      if (lanes.empty() || lanes.back().instance != chunk[t].lane) lanes.push_back(LaneSeg{chunk[t].lane, nlane, 0});
-      chunk[t].lcta0 = nlane;
-      lanes.back().ncta += chunk[t].nlane;
-      nlane += chunk[t].nlane;
+  struct Chunk {
+    size_t first, n = 0;
+    int64_t part = 0;
+    int ncta = 0, nlane = 0;
+    std::vector<Seg> segs;
+    std::vector<LaneSeg> lanes;
+    explicit Chunk(size_t f) : first(f) {}
+  };
+  std::vector<ShWork> work;
+  std::vector<Chunk> chunks;
+  // heaviest degrees first: their CTAs are the longest
+  for (int L = SH_MAXL; L >= 0; L--) {
+    std::vector<ShWork>& v = Lw.work[L];
+    auto cost = [&](const ShWork& w) { return side_cost(T.pair[w.bra], T.pair[w.ket]); };
+    std::stable_sort(v.begin(), v.end(), [&](const ShWork& a, const ShWork& b) { return cost(a) > cost(b); });
+    bool open = false;
+    for (ShWork w : v) {
+      const ShPair &b = T.pair[w.bra], &k = T.pair[w.ket];
+      const int ni = b.ncomp * k.ncomp;
+      const int64_t need = (int64_t)(w.split + w.lsplit) * (diag ? b.ncomp : ni);
+      if (chunks.empty() || (chunks.back().n && (chunks.back().part + need > cap_d ||
+                                                 chunks.back().ncta + chunks.back().nlane > (1 << 28)))) {
+        chunks.emplace_back(work.size());
+        open = false;
+      }
+      Chunk& C = chunks.back();
+      if (!open) {
+        C.segs.push_back(Seg{L, C.ncta, 0, 0, 0, 0});
+        open = true;
+      }
+      Seg& g = C.segs.back();
+      w.cta0 = C.ncta;
+      w.part = C.part;
+      work.push_back(w);
+      g.ncta += w.split;
+      g.no = std::max(g.no, sh_nherm(b.d) * k.ncomp);
+      g.ni = std::max(g.ni, ni);
+      g.col = std::max(g.col, sh_col_size(b.d, k.nterm));
+      C.n++;
+      C.ncta += w.split;
+      C.nlane += w.nlane;
+      C.part += need;
     }
-    void *dw, *dc, *dp;
-    TRY(pool_get(c, "shell_part", sizeof(double) * (size_t)std::max(part, std::min(most, cap_d)), &dp));
-    DevBuf& wb = c->pool["shell_work"];
-    TRY(h2d_async(c, wb, chunk.data(), sizeof(ShWork) * chunk.size()));
-    dw = wb.ptr;
-    TRY(pool_get(c, "shell_cta", sizeof(int) * ((size_t)ncta + nlane), &dc));
-    int* lcta = (int*)dc + ncta;
-    shell_expand<<<(unsigned)chunk.size(), 32, 0, c->stream>>>((const ShWork*)dw, (int*)dc, lcta);
+  }
+  if (chunks.empty()) return SS_OK;
+  int64_t part = 0, ctas = 0;
+  for (Chunk& C : chunks) {
+    // the lane kernels' CTAs, an instance's together
+    std::vector<size_t> order;
+    for (size_t t = C.first; t < C.first + C.n; t++)
+      if (work[t].lane >= 0) order.push_back(t);
+    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return work[x].lane > work[y].lane; });
+    int nlane = 0;
+    for (size_t t : order) {
+      if (C.lanes.empty() || C.lanes.back().instance != work[t].lane) C.lanes.push_back(LaneSeg{work[t].lane, nlane, 0});
+      work[t].lcta0 = nlane;
+      C.lanes.back().ncta += work[t].nlane;
+      nlane += work[t].nlane;
+    }
+    part = std::max(part, C.part);
+    ctas = std::max(ctas, (int64_t)C.ncta + C.nlane);
+  }
+  void *dc, *dp;
+  TRY(pool_get(c, "shell_part", sizeof(double) * (size_t)part, &dp));
+  TRY(pool_get(c, "shell_cta", sizeof(int) * (size_t)ctas, &dc));
+  TRY(h2d_async(c, c->pool["shell_work"], work.data(), sizeof(ShWork) * work.size()));
+  const ShWork* dwork = (const ShWork*)c->pool["shell_work"].ptr;
+  ShArgs A{};
+  A.pair = (const ShPair*)c->pool["shell_pair"].ptr;
+  A.cnt = (const int*)c->pool["shell_cnt"].ptr;
+  A.st = (const ShStruct*)c->pool["shell_struct"].ptr;
+  A.prim = prim;
+  A.primf = primf;
+  A.E = E;
+  A.E2 = E2;
+  A.scale = (const double*)c->pool["shell_scale"].ptr;
+  A.boys = (const ShBoys*)c->pool["shell_boys"].ptr;
+  A.col = (const uint8_t*)c->pool["shell_col"].ptr;
+  A.partial = (double*)dp;
+  A.eps = eps;
+  A.eps32 = eps32;
+  A.eps_df = SH_DF_EPS;
+  A.diag = diag;
+  A.cta = (const int*)dc;
+  for (const Chunk& C : chunks) {
+    A.work = dwork + C.first;
+    int* lcta = (int*)dc + C.ncta;
+    A.lcta = lcta;
+    shell_expand<<<(unsigned)C.n, 32, 0, c->stream>>>(A.work, (int*)dc, lcta);
     SS_CUDA_TRY(cudaGetLastError());
     c->launches++;
     TRY(fork_eri_streams(c));
-    ShArgs A{};
-    A.pair = (const ShPair*)c->pool["shell_pair"].ptr;
-    A.cnt = (const int*)c->pool["shell_cnt"].ptr;
-    A.st = (const ShStruct*)c->pool["shell_struct"].ptr;
-    A.prim = prim;
-    A.primf = primf;
-    A.E = E;
-    A.E2 = E2;
-    A.scale = (const double*)c->pool["shell_scale"].ptr;
-    A.boys = (const ShBoys*)c->pool["shell_boys"].ptr;
-    A.col = (const uint8_t*)c->pool["shell_col"].ptr;
-    A.partial = (double*)dp;
-    A.eps = eps;
-    A.eps32 = eps32;
-    A.eps_df = SH_DF_EPS;
-    A.diag = diag;
-    A.work = (const ShWork*)dw;
-    A.cta = (const int*)dc;
-    A.lcta = lcta;
     int rc = SS_OK;
     size_t launch = 0;
-    for (size_t s = 0; s < lanes.size() && !rc; s++) {
-      A.cta0 = lanes[s].cta0;
-      const cudaError_t e = launch_shell_lane(lanes[s].instance, lanes[s].ncta, c->eri_stream[launch++ % ss_ctx::ERI_STREAMS], A);
+    for (size_t s = 0; s < C.lanes.size() && !rc; s++) {
+      A.cta0 = C.lanes[s].cta0;
+      const cudaError_t e = launch_shell_lane(C.lanes[s].instance, C.lanes[s].ncta, c->eri_stream[launch++ % ss_ctx::ERI_STREAMS], A);
       if (e != cudaSuccess) {
         ss_set_cuda_error(e, "shell_lane_kernel launch", __FILE__, __LINE__);
         rc = SS_ERR_CUDA;
       }
       c->launches++;
     }
-    for (size_t s = 0; s < segs.size() && !rc; s++) {
-      const Seg& g = segs[s];
-      A.cta0 = chunk[g.first].cta0;
+    for (size_t s = 0; s < C.segs.size() && !rc; s++) {
+      const Seg& g = C.segs[s];
+      A.cta0 = g.cta0;
       const cudaError_t e = launch_shell_eri(g.L, g.ncta, g.no, g.ni, g.col, c->eri_stream[launch++ % ss_ctx::ERI_STREAMS], A);
       if (e != cudaSuccess) {
         ss_set_cuda_error(e, "shell_eri_kernel launch", __FILE__, __LINE__);
@@ -460,50 +502,11 @@ static int run_work(ss_ctx* c, ShellPlan& Lw, const ShPrim* prim, const ShPrimF*
     }
     const int jrc = join_eri_streams(c);
     if (rc || jrc) return rc ? rc : jrc;
-    shell_reduce<<<dim3((unsigned)chunk.size(), 4), 256, 0, c->stream>>>((int)chunk.size(), (const ShWork*)dw, A.pair, diag,
-                                                               (const double*)dp, elem);
+    shell_reduce<<<dim3((unsigned)C.n, 4), 256, 0, c->stream>>>((int)C.n, A.work, A.pair, diag, (const double*)dp, elem);
     SS_CUDA_TRY(cudaGetLastError());
     c->launches++;
-    chunk.clear();
-    segs.clear();
-    part = 0;
-    ncta = nlane = 0;
-    return SS_OK;
-  };
-  for (int L = 0; L <= SH_MAXL; L++)
-    for (const ShWork& w : Lw.work[L]) most += (int64_t)(w.split + w.lsplit) * (diag ? T.pair[w.bra].ncomp : T.pair[w.bra].ncomp * T.pair[w.ket].ncomp);
-  for (int L = SH_MAXL; L >= 0; L--) {
-    std::vector<ShWork>& v = Lw.work[L];
-    auto cost = [&](const ShWork& w) { return side_cost(T.pair[w.bra], T.pair[w.ket]); };
-    std::stable_sort(v.begin(), v.end(), [&](const ShWork& a, const ShWork& b) { return cost(a) > cost(b); });
-    bool open = false;
-    for (ShWork& w : v) {
-      const ShPair &b = T.pair[w.bra], &k = T.pair[w.ket];
-      const int ni = b.ncomp * k.ncomp;
-      const int64_t need = (int64_t)(w.split + w.lsplit) * (diag ? b.ncomp : ni);
-      if (!chunk.empty() && (part + need > cap_d || ncta + nlane > (1 << 28))) {
-        TRY(flush());
-        open = false;
-      }
-      if (!open) {
-        segs.push_back(Seg{L, (int)chunk.size(), 0, 0, 0, 0, 0});
-        open = true;
-      }
-      Seg& g = segs.back();
-      w.cta0 = ncta;
-      w.part = part;
-      chunk.push_back(w);
-      g.n++;
-      g.ncta += w.split;
-      g.no = std::max(g.no, sh_nherm(b.d) * k.ncomp);
-      g.ni = std::max(g.ni, ni);
-      g.col = std::max(g.col, sh_col_size(b.d, k.nterm));
-      ncta += w.split;
-      nlane += w.nlane;
-      part += need;
-    }
   }
-  return flush();
+  return SS_OK;
 }
 
 // Primitive tables of the shell pairs and the Schwarz diagonal (ik|ik) of every function pair in

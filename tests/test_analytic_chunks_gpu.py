@@ -1,0 +1,56 @@
+"""The analytic stage in several chunks of partial sums (a tight device-memory budget): the values are
+those of one chunk, bit for bit, and a job queues its MC while the chunks run, not after them."""
+import threading
+import time
+
+import numpy as np
+import pytest
+
+from slater_stoch_gb300 import api, basis, configs
+from slater_stoch_gb300._lib import SSError
+
+pytestmark = pytest.mark.gpu
+
+
+def _smallest_budget(b, q, job):
+    """The first budget, in steps of 4 MB, under which the job runs (a small part of it is then left
+    for the partial sums)."""
+    for mb in range(16, 256, 4):
+        try:
+            with api.Context(0, mb << 20) as ctx:
+                ctx.set_basis(b)
+                ctx.set_quartets(*q)
+                job(ctx)
+            return mb << 20
+        except SSError as e:
+            assert "budget" in str(e)
+    raise AssertionError("no budget below 256 MB is enough")
+
+
+def test_chunks_give_the_same_values_and_do_not_hold_up_the_mc():
+    b = configs.h2o_26(ng0=20)
+    q = basis.build_mapping(b.n)
+    job = lambda ctx: ctx.two_e_job(1.8, 3, 40, 2, "faithful", "fp64")  # noqa: E731
+    with api.Context(0) as ctx:
+        ctx.set_basis(b)
+        ctx.set_quartets(*q)
+        ref, _ = ctx.gauss_eri()
+        one = ctx.launches
+    with api.Context(0, _smallest_budget(b, q, job)) as ctx:
+        ctx.set_basis(b)
+        ctx.set_quartets(*q)
+        job(ctx)
+        ctx.invalidate()
+        n0, t0 = ctx.launches, time.perf_counter()
+        g, _ = ctx.gauss_eri()
+        stage, launches = time.perf_counter() - t0, ctx.launches - n0
+        assert launches >= one + 20  # several chunks
+        np.testing.assert_array_equal(g, ref)
+        n0, t0 = ctx.launches, time.perf_counter()
+        worker = threading.Thread(target=job, args=(ctx,))
+        worker.start()
+        while ctx.launches - n0 <= launches and worker.is_alive():
+            time.sleep(0.0002)
+        queued = time.perf_counter() - t0
+        worker.join()
+        assert queued <= 0.5 * stage, (queued, stage)
