@@ -99,8 +99,21 @@ void dev_free(ss_ctx* c, DevBuf& b) {
 }
 
 // Copies up to STAGE_HALF go through a pinned ring of two halves: on leaving a half an event is
-// recorded on every stream that copied from it, and it is used again after these events (an event
-// per copy cost the short calls 6 to 15 us).  Larger copies are rare and wait for the stream instead.
+// recorded on every stream that copied from it since its last event, and it is used again after these
+// events (an event per copy cost the short calls 6 to 15 us).  Larger copies are rare and wait for
+// their stream instead.
+//
+// stage_mark records the context stream's event now: before long work is queued on it, so that a later
+// change of half waits for the copies and not for that work.
+static int stage_mark(ss_ctx* c) {
+  for (auto& e : c->stage_evt) {
+    if (e.stream != c->stream || !e.pending) continue;
+    SS_CUDA_TRY(cudaEventRecord(e.left[c->stage_half], e.stream));
+    e.pending = false;
+  }
+  return SS_OK;
+}
+
 int h2d_copy(ss_ctx* c, void* dst, const void* src, size_t bytes) {
   constexpr size_t STAGE_HALF = (size_t)512 << 10;
   if (bytes == 0) return SS_OK;
@@ -111,21 +124,25 @@ int h2d_copy(ss_ctx* c, void* dst, const void* src, size_t bytes) {
   }
   if (!c->stage) SS_CUDA_TRY(cudaHostAlloc((void**)&c->stage, 2 * STAGE_HALF, cudaHostAllocDefault));
   if (c->stage_off + bytes > STAGE_HALF) {
-    for (auto& e : c->stage_evt) SS_CUDA_TRY(cudaEventRecord(e.left[c->stage_half], e.stream));
+    for (auto& e : c->stage_evt) {
+      if (e.pending) SS_CUDA_TRY(cudaEventRecord(e.left[c->stage_half], e.stream));
+      e.pending = false;
+    }
     c->stage_half ^= 1;
     for (auto& e : c->stage_evt) SS_CUDA_TRY(cudaEventSynchronize(e.left[c->stage_half]));
     c->stage_off = 0;
   }
-  bool known = false;
-  for (auto& e : c->stage_evt) known = known || e.stream == c->stream;
-  if (!known) {
-    ss_ctx::StageStream e{c->stream, {nullptr, nullptr}};
+  size_t at_evt = 0;
+  while (at_evt < c->stage_evt.size() && c->stage_evt[at_evt].stream != c->stream) at_evt++;
+  if (at_evt == c->stage_evt.size()) {
+    ss_ctx::StageStream e{c->stream, {nullptr, nullptr}, false};
     for (auto& v : e.left) SS_CUDA_TRY(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
     c->stage_evt.push_back(e);
   }
   char* at = c->stage + c->stage_half * STAGE_HALF + c->stage_off;
   memcpy(at, src, bytes);
   SS_CUDA_TRY(cudaMemcpyAsync(dst, at, bytes, cudaMemcpyHostToDevice, c->stream));
+  c->stage_evt[at_evt].pending = true;
   c->stage_off += (bytes + 255) / 256 * 256;
   return SS_OK;
 }
@@ -166,6 +183,8 @@ static int pair_L(const ss_ctx* c, int f1, int f2) {
 }
 
 int fork_eri_streams(ss_ctx* c) {
+  const int mrc = stage_mark(c);
+  if (mrc) return mrc;
   if (!c->eri_fork) {
     int lo = 0, hi = 0;  // lowest priority: the MC of a job runs beside the analytic stage
     SS_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));

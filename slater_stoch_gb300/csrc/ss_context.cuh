@@ -55,10 +55,11 @@ struct ss_ctx {
   size_t pin_cap = 0;
   cudaEvent_t pin_evt = nullptr;
   // pinned staging ring of h2d_copy (two halves), the half in use and its fill, and per stream that
-  // copied from it the work queued when each half was left last
+  // copied from it an event after its last copies from each half, and whether it copied since
   struct StageStream {
     cudaStream_t stream;
     cudaEvent_t left[2];
+    bool pending;
   };
   char* stage = nullptr;
   size_t stage_off = 0;
