@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(ShDim<L>::NT, ShDim<L>::MINB) shell_eri_kernel
     int c = 0, cd = 0, cf = 0;  // ranges [0, cd) FP64, [cd, cf) two floats, [cf, c) FP32
     if (tid < ns) {
       c = cd = cf = diag ? p + 1 : nk;
-      if (!diag && A.eps > 0.0) {
+      if (!diag) {
         const double sb = bra[p].S;
         auto first_below = [&](double thr) {  // first ket with sb * S < thr
           int lo = 0, hi = nk;

@@ -458,7 +458,7 @@ int ensure_gauss(ss_ctx* c) {
   std::vector<int64_t> slot(c->nint, -1), rest;
   ShellPlan plan;
   int64_t nelem = 0, npartial = 0;
-  TRY(shell_plan(c, c->eri_eps_screen > 0.0 && c->eri_eps32 > c->eri_eps_screen, sel, slot, rest, plan, &nelem));
+  TRY(shell_plan(c, c->eri_eps32 > c->eri_eps_screen, sel, slot, rest, plan, &nelem));
   // results: one element per component of the shell quartets, then the per-function partial sums
   if (rest.empty()) {
     TRY(dev_alloc(c, c->d_scratch_b, sizeof(double) * std::max<int64_t>(nelem, 1)));

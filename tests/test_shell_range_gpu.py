@@ -71,3 +71,21 @@ def test_far_from_the_origin(orbs):
     q = basis.build_mapping(b.n)
     g, f, pre = _default_and_fp64(b, q)
     _gate(g, f, pre, q)
+
+
+def test_tiers_without_a_screen():
+    """screen_eps = 0 skips nothing and leaves the other thresholds as they are: the same values as with a
+    screen below every primitive quartet's bound, and not those of the all-FP64 evaluation."""
+    b = _basis(ORBS["mixed"], 12, TWO)
+    q = basis.build_mapping(b.n)
+    out = {}
+    with api.Context(0) as ctx:
+        ctx.set_basis(b)
+        ctx.set_quartets(*q)
+        pre = ctx.precond()
+        for screen, fp32 in ((0.0, 1e-11), (1e-300, 1e-11), (0.0, 0.0)):
+            ctx.set_eri_tiers(screen, fp32)
+            out[screen, fp32], _ = ctx.gauss_eri()
+    np.testing.assert_array_equal(out[0.0, 1e-11], out[1e-300, 1e-11])
+    assert not np.array_equal(out[0.0, 1e-11], out[0.0, 0.0])
+    _gate(out[0.0, 1e-11], out[0.0, 0.0], pre, q)
