@@ -42,12 +42,13 @@
 #include "df32.cuh"
 #include "shell.cuh"
 
-#ifndef __CUDACC__
+namespace ss {
+
+#ifndef __CUDACC__  // the host build of the tests
 using std::fma;
 using std::min;
+inline double rsqrt(double x) { return 1.0 / std::sqrt(x); }
 #endif
-
-namespace ss {
 
 constexpr double SH_PI_5_2 = 34.9868366552;  // src/general_primitive_integral.F90:25
 
