@@ -517,8 +517,8 @@ def main():
             "metric": METRIC,
             "value": value, "unit": "ERIs/s", "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3),
             "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": ("f64 analytic (f32 for primitive quartets below 1e-11 of their Schwarz bound) + "
-                      "bf16x3 (fp32 accumulate) MC"), "data": "synthetic",
+            "dtype": ("f64 analytic (two floats, 48 bits, for primitive quartets below 1e-5 of the Schwarz bound, "
+                      "f32 below 1e-11) + bf16x3 (fp32 accumulate) MC"), "data": "synthetic",
             "config": {"workload": WORKLOAD,
                        "walkers": args.walkers, "blocks": NBLOCKS, "estimator": "shared-walker, split-BF16",
                        "max_sigma_Ha": max_sigma, "sigma_target_Ha": SIGMA_TARGET,

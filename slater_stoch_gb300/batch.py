@@ -4,16 +4,17 @@ The reference runs one system per process (src/two_e_slater.F90:219-564).  Here 
 fitted bases are concatenated into one basis, ``ss_basis_systems`` marks the system boundaries
 (primitive pairs of functions of two systems are never formed), and the systems' own unique
 quartet lists, concatenated with their function indices shifted, go to one ``ss_gauss_eri``:
-the analytic stage of every system then runs as one launch per kernel instance (L, LK, tc),
-quartets of all systems mixed, which fills the GPU where a small system alone would leave most
-SMs idle.  The ZV-MC correction of each system runs as its own job on the pooled worker
-contexts (``SS_JOB_MC_ONLY``: its proposal mixture is the system's own), all of them
-concurrently; each system's ERIs are its analytic values plus its correction.
+the analytic stage of every system then runs as one launch per kernel class, shell quartets of all
+systems mixed, which fills the GPU where a small system alone would leave most SMs idle.  The
+shell-pair tables are those of the systems' own pairs, so memory grows with the number of systems.
+The ZV-MC correction of each system runs as its own job on the pooled worker contexts
+(``SS_JOB_MC_ONLY``: its proposal mixture is the system's own), all of them concurrently; each
+system's ERIs are its analytic values plus its correction.
 
-A system's result does not depend on the batch it ran in beyond summation order: the analytic
-values agree with a run of the system alone to rounding (the bra-slice split of a quartet
-depends on how many quartets share its kernel class), and the MC correction is bitwise the
-same (same seed, same walkers, same reductions).
+A system's result does not depend on the batch it ran in: the analytic values are bitwise those of
+a run of the system alone (the decomposition follows from the shell quartet; only quartets with a
+function in no shell, degree 3 and more, agree to rounding), and so is the MC correction (same
+seed, same walkers, same reductions).
 """
 from __future__ import annotations
 

@@ -11,9 +11,9 @@
 //    trailing columns and the explicit Q are updated by three dgemm calls per panel;
 //  * sym_eig, n > 128: cyclic two-sided Jacobi with the round-robin ("circle") pair order.  The
 //    n/2 rotations of a round act on disjoint index pairs, so A' = J^T A J splits into
-//    independent 2 x 2 blocks J_P^T A_PR J_R, written into a second buffer (no read-after-write
-//    hazard inside a round), and V' = V J into independent row pairs.  One cooperative grid
-//    does all rounds and sweeps with a bounded grid barrier per round;
+//    independent 2 x 2 blocks J_P^T A_PR J_R, each updated in place by one thread, and V' = V J
+//    into independent row pairs.  One cooperative grid does all rounds and sweeps with a bounded
+//    grid barrier per round;
 //  * sym_eig, n <= 128: one CTA with the matrix in shared memory: Householder reduction to
 //    tridiagonal form with accumulated transformations and implicit QL with Wilkinson shifts
 //    (the classical tred2 / tql2 procedure), used for Davidson's small projected problems.
@@ -592,7 +592,11 @@ __global__ void __launch_bounds__(256) sym_eig_smem_kernel(int n, const double* 
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t GRID_SPIN_LIMIT = 1u << 22;  // bounded grid barrier (seconds of L2 polling; a round takes microseconds)
 constexpr int JACOBI_MAX_SWEEPS = 40;
-constexpr int JACOBI_THREADS = 256;  // measured on 351 x 351: 256 threads 40.8 ms, 512 46.6 ms, 1024 67.4 ms
+// Measured on 351 x 351: 256 threads 40.8 ms, 512 46.6 ms, 1024 67.4 ms.  At the other sizes that the
+// cleanup reaches, against the form before it (all CTAs that fit, a second matrix; whole calls of the
+// projection at 210 and 990, of the SVD cleanup at 496, 1,400, 2,016): 29.7 -> 20.9, 643 -> 447,
+// 193 -> 107, 2,144 -> 1,599, 3,544 -> 2,815 ms.
+constexpr int JACOBI_THREADS = 256;
 
 struct JacobiCtl {
   unsigned int count;       // grid barrier: arrivals since the start

@@ -20,6 +20,9 @@ namespace ss {
 // functions; O; O-H; H2O of 19 functions): all FP64 1.4e-15, 4.3e-15, 4.5e-15, 2.8e-15 with the
 // per-function kernels; here 1e-5: 1.2e-15, 2.4e-15, 1.9e-15, 2.8e-15; 1e-4: 1.9e-15, 2.2e-15,
 // 9.4e-15, 2.8e-15; 1e-3: 1.4e-14, 9.6e-15, 4.0e-14, 9.9e-15; all two-float: 2.5e-14 to 1.5e-13.
+// Against 80-bit sums (water 7 functions at 20, 13, 9 Gaussians; H2; O; N; O-H), per-function kernels ->
+// here: largest error 1.3e-15 -> 9.4e-16, 1.2e-15 -> 4.1e-16, 9.9e-16 -> 4.2e-16, 1.5e-15 -> 5.6e-16,
+// 9.6e-16 -> 6.8e-16, 4.3e-15 -> 1.9e-15, 2.8e-15 -> 6.9e-16 of the Schwarz bound.
 // About a tenth of the FP64 work is left above 1e-5.
 constexpr double SH_DF_EPS = 1e-5;
 

@@ -3,8 +3,8 @@
 * primitive quartets: the reference loops over n_gauss(i)*nc(i) x ... x n_gauss(l)*nc(l)
   primitive Gaussian products per (ik|jl) (src/gauss_ijkl.F90:127-150), nc = 3 for the
   r^2-type fits (i_type 2) and 1 otherwise.  The GPU skips the primitive quartets below its
-  Schwarz screen and evaluates those below the FP32 bound in FP32, so the executed work is
-  measured rather than modelled:
+  Schwarz screen and evaluates the small ones in two floats or FP32, and it forms the integrals of a
+  shell quartet once for all its components, so the executed work is measured rather than modelled:
 * EXEC_FLOPS: executed flops of all shell_* launches of one analytic stage (primitive tables, Schwarz
   diagonal and screened quartets), from ncu instruction counters on the full workload
   (smsp__sass_thread_inst_executed_op_{dfma,dmul,dadd,ffma,fmul,fadd}_pred_on.sum, one pass each; DFMA
@@ -25,14 +25,14 @@ EXEC_FLOPS_PER_PRIM = 241.5
 EXEC_FLOPS = {
     "h2o_26_ng20": (7.542e9, 2.902e11),
 }
-# workload -> DRAM bytes (read + write) of the same launches (EXEC_DRAM_BYTES; ncu
-# dram__bytes_read.sum + dram__bytes_write.sum, one pass each)
 # workload -> DRAM bytes per walker pair of the shared-walker MC kernels (sampler, orbital values,
 # operands, tcgen05 GEMM, accumulation): ncu of one 262,144-sample sub-chunk (reads 1.9909e9 B +
 # writes 1.5202e9 B) / 262,144
 MC_DRAM_BYTES_PER_SAMPLE = {
     "h2o_26_ng20": 3.5111e9 / 262144,
 }
+# workload -> DRAM bytes of the launches of EXEC_FLOPS (ncu dram__bytes_read.sum + dram__bytes_write.sum,
+# one pass each)
 EXEC_DRAM_BYTES = {
     "h2o_26_ng20": 1.349e8,
 }
