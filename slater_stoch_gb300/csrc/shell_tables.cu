@@ -159,8 +159,13 @@ __global__ void shell_expand(const ShWork* __restrict__ work, int* __restrict__ 
   for (int s = threadIdx.x; s < W.nlane; s += blockDim.x) lcta[W.lcta0 + s] = blockIdx.x;
 }
 
-// exponent of the largest power of two whose square is at most 2 p
-__device__ __forceinline__ int unit_exp(double p) { return ilogb(p + p) >> 1; }
+// exponent of the largest power of two whose square is at most 2 p, and a power of two, from the bits
+// of the double (normal numbers; with ilogb and ldexp the sort took 0.28 ms instead of 0.21 for the
+// 26-function water)
+__device__ __forceinline__ int unit_exp(double p) {
+  return ((int)((uint64_t)__double_as_longlong(p + p) >> 52) - 1023) >> 1;
+}
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((int64_t)(1023 + e) << 52); }
 
 // Schwarz factors of a pair's primitives and their sorted tables.  A primitive's factor is the
 // largest over the components of sqrt((P_f|P_f) / (f|f)), (f|f) the contracted diagonal: then
@@ -260,8 +265,8 @@ __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pai
       g.pm[ax] = (float)((a.P[ax] - (double)g.ph[ax]) - (double)g.pl[ax]);
     }
     g.pad = 0.f;
-    g.s = ldexpf(1.f, unit_exp(a.p));
-    g.is = ldexpf(1.f, -unit_exp(a.p));
+    g.s = (float)pow2(unit_exp(a.p));
+    g.is = (float)pow2(-unit_exp(a.p));
     oprimf[P.prim_off + t] = g;
   }
   for (int t = threadIdx.x; t < m * P.nterm; t += blockDim.x) {
@@ -270,7 +275,7 @@ __global__ void __launch_bounds__(512) shell_sort(const ShPair* __restrict__ pai
     oE[P.e_off + t] = v;
     const uint32_t tm = S.term[x];
     const int deg = (int)((tm & 255) + ((tm >> 8) & 255) + (tm >> 16));
-    const double u = ldexp(v, deg * unit_exp(prim[P.prim_off + s_idx[r]].p));
+    const double u = v * pow2(deg * unit_exp(prim[P.prim_off + s_idx[r]].p));
     const float hi = (float)u;
     oE2[P.e_off + t] = make_float2(hi, (float)(u - (double)hi));
   }
