@@ -479,9 +479,9 @@ def main():
                 "kernel": "shell_eri_kernel and shell_lane_kernel (analytic Gaussian-fit ERIs, all launches of one job)",
                 "peak_source": "measured in this run: torch float64 matmul 4096^3 (FP64 peak is not "
                                "in MEASURED_PEAKS.json)",
-                "fp64_pipe_issue_pct": 26.9,
+                "fp64_pipe_issue_pct": 25.1,
                 "fp64_pipe_note": ("ncu sm__inst_executed_pipe_fp64, time-weighted over the stage's launches (60-75 % "
-                                   "in the FP64 tier of the light classes, 14-43 % in the heavy classes, 1-13 % in "
+                                   "in the FP64 tier of the light classes, 12-41 % in the heavy classes, 1-12 % in "
                                    "the two-float and FP32 tiers, which run on the FP32 pipe)"),
                 "units": (f"executed FP64 flops of the stage's shell_* launches (ncu instruction "
                           f"counters, DFMA = 2): {flops:.4g}; plus {EXEC_FLOPS[wl][1]:.4g} FP32 flops "

@@ -441,7 +441,7 @@ int ss_two_e_job(ss_ctx* c, double a_zv, uint64_t seed, int64_t samples_per_bloc
   // own lowest-priority stream (ensure_gauss returns once its launches are queued) and the MC
   // runs on the context stream (greatest priority) meanwhile: the MC kernels take SM slots as
   // ERI CTAs retire instead of waiting for the whole stage (26-function H2O job: the stages alone
-  // take 44 + 214 ms, the job 250 ms; the GEMM's CTAs leave an SM little room).  Results are
+  // take 47 + 207 ms, the job 251 ms; the GEMM's CTAs leave an SM little room).  Results are
   // bitwise the same.  The context stream waits for the analytic stage before the combine.
   if (!c->ana_stream) {
     int lo = 0, hi = 0;

@@ -23,7 +23,7 @@ EXEC_FLOPS_PER_PRIM = 241.5
 # workload -> (executed FP64 flops, executed FP32 flops) of the analytic stage of one job, at the
 # default tiers (primitive screen 1e-18, FP32 below 1e-11 of the Schwarz bound, two floats below 1e-5)
 EXEC_FLOPS = {
-    "h2o_26_ng20": (7.542e9, 2.902e11),
+    "h2o_26_ng20": (7.508e9, 3.087e11),
 }
 # workload -> DRAM bytes per walker pair of the shared-walker MC kernels (sampler, orbital values,
 # operands, tcgen05 GEMM, accumulation): ncu of one 262,144-sample sub-chunk (reads 1.9909e9 B +
@@ -34,7 +34,7 @@ MC_DRAM_BYTES_PER_SAMPLE = {
 # workload -> DRAM bytes of the launches of EXEC_FLOPS (ncu dram__bytes_read.sum + dram__bytes_write.sum,
 # one pass each)
 EXEC_DRAM_BYTES = {
-    "h2o_26_ng20": 1.349e8,
+    "h2o_26_ng20": 1.332e8,
 }
 
 
